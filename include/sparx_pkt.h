@@ -240,8 +240,8 @@ typedef struct sparx_tuning {
   uint32_t merge_ratio;     /* peel: merge the two rows when the longer is <= this x the shorter (8) */
   uint32_t hub_min_degree;  /* dense neighbour -> edge maps for vertices of at least this degree,
                                >= 256, or 0 for none (1024) */
-  uint32_t sample_min;      /* support: longer out-lists of at least this length are narrowed
-                               through 64 samples before the search (64) */
+  uint32_t sample_min;      /* support: longer out-lists of at least this length (8 at least) are
+                               searched through a rank index, shorter ones by binary search (64) */
   uint32_t support_kernel;  /* 1 balanced edge form, 2 vertex form (1; 2 for keys with no
                                slots in rows of degree >= 256 and a largest degree of 64..255,
                                which is what sparx_tuning_lookup reports for such a key) */
@@ -252,7 +252,7 @@ typedef struct sparx_tuning {
                                Skipped, with the same results, when its workspace (32 B per slot
                                plus 16 B per edge) is over a batch's budget or cannot be allocated */
   uint32_t sup_hash_min;    /* support: oriented out-lists of at least this length (>= 4) get a hash
-                               table probed instead of the sampled search; 0 = none (0) */
+                               table probed instead of the search; 0 = none (0) */
   uint32_t relabel;         /* graphs and batched unions without parallel edges: rebuild the CSR on vertex ids
                                in (floor(log2 degree), id) order (a union's members each within their own
                                id range) before the decomposition, for locality;

@@ -552,7 +552,8 @@ __global__ void __launch_bounds__(256) k_orient_count(const uint32_t* __restrict
 // Kernel B2: fill oriented lists (kept in id order) and, for each vertex's
 // out-slots, the (id | edge id << 32) pair of row0; self-loop slots get edge id
 // 0xFFFFFFFF.  In-slots are left to B3: owner[s] = u marks them (kInvalid for
-// the others).
+// the others).  `oname` (nullptr: not wanted) takes the out-slots' names (the
+// rank index's keys, off[v]).
 __device__ __forceinline__ unsigned long long make_pair(uint32_t id, uint32_t e) {
   return (unsigned long long)id | ((unsigned long long)e << 32);
 }
@@ -565,7 +566,8 @@ __global__ void __launch_bounds__(256) k_orient_fill(const uint32_t* __restrict_
                                                      unsigned long long* __restrict__ row0,
                                                      uint32_t* __restrict__ owner,
                                                      const uint32_t* __restrict__ big_list,
-                                                     const uint32_t* __restrict__ big_count) {
+                                                     const uint32_t* __restrict__ big_count,
+                                                     uint32_t* __restrict__ oname) {
   const uint32_t lane = lane_id();
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -583,6 +585,7 @@ __global__ void __launch_bounds__(256) k_orient_fill(const uint32_t* __restrict_
         } else if (rank_less(e - b, u, deg_of(off, v), v)) {
           ocol[p] = v;
           osrc[p] = u;
+          if (oname) oname[p] = __ldg(off + v);
           row0[s] = make_pair(v, p);
           ++p;
         } else {
@@ -615,6 +618,7 @@ __global__ void __launch_bounds__(256) k_orient_fill(const uint32_t* __restrict_
           const uint32_t p = p0 + __popc(bal & ((1u << lane) - 1));
           ocol[p] = v;
           osrc[p] = bu;
+          if (oname) oname[p] = __ldg(off + v);
           row0[s] = make_pair(v, p);
         }
         p0 += __popc(bal);
@@ -652,6 +656,7 @@ __global__ void __launch_bounds__(256) k_orient_fill(const uint32_t* __restrict_
         if (outm & (1u << i)) {
           ocol[p] = v[i];
           osrc[p] = bu;
+          if (oname) oname[p] = __ldg(off + v[i]);
           row0[s0 + i] = make_pair(v[i], p);
           ++p;
         }
@@ -759,12 +764,6 @@ struct LoadU32 {
 };
 
 // support work of oriented edge e = min(d+(src), d+(dst))
-#ifndef SPARX_SAMPLED_LIST
-#define SPARX_SAMPLED_LIST 64
-#endif
-// longer lists from this length on are searched through 32 samples
-constexpr uint32_t kSampledList = SPARX_SAMPLED_LIST;
-
 struct SupportWork {
   const uint32_t* opos;
   const uint32_t* osrc;
@@ -776,6 +775,156 @@ struct SupportWork {
     return min(da, db);
   }
 };
+
+// ---------------------------------------------------------------------------
+// Rank index of a sorted list (or row) of d entries: 2^lg buckets, lg =
+// ceil(log2 d) + 3, of the entries' names, mapped linearly from the list's own
+// smallest and largest name; 32 buckets share one 8-byte word {occupied
+// buckets, position of the first entry at or past the word's first bucket}.
+// A search costs one word; nine in ten absent names end there (8 to 16 buckets
+// per entry), a present one is at the position plus the occupied buckets below
+// it (later only when two entries share a bucket, found by a binary search of
+// the word's entries, so a badly clustered list costs no more than before).
+// Names are a vertex's offset in the CSR: ascending with the id, and spread as
+// evenly as the slots are, whatever the degrees of neighbouring ids, which is
+// what the linear map needs (ids sorted by degree would fill few buckets).
+// Consecutive elements of an edge ask ascending names, so a warp's 32 searches
+// fall on neighbouring words and neighbouring entries, as a merge's would.
+// Words lie at (start + 1) / 2 of the pool (fewer than d / 2 of them); the
+// header is {smallest name, scale}, scale 0: no index.
+__device__ __forceinline__ uint32_t rank_shift(uint32_t d) { return 30 - hash_log2cap(d); }  // 32 - lg
+__device__ __forceinline__ uint32_t rank_scale(uint32_t mn, uint32_t mx) { return 0xFFFFFFFFu / max(mx - mn, 1u); }
+__device__ __forceinline__ uint32_t list_name(uint32_t x) { return x; }
+__device__ __forceinline__ uint32_t list_name(unsigned long long x) { return (uint32_t)x; }
+
+// The entry at p is below `name`, whose bucket (in a word starting at `words`)
+// is bk: entries that share a bucket precede it.  Mostly it is the next one;
+// else a binary search of the word's entries finds it.
+template <class E>
+__device__ __forceinline__ uint32_t rank_later(const E* __restrict__ arr, uint32_t p, uint32_t le,
+                                               const unsigned long long* __restrict__ words, uint32_t bk, uint32_t sh,
+                                               uint32_t name, E* en) {
+  if (++p >= le) return kInvalid;
+  *en = __ldg(arr + p);
+  if (list_name(*en) < name) {
+    const uint32_t j = (bk >> 5) + 1;
+    const uint32_t end = j == (1u << (27 - sh)) ? le : (uint32_t)(__ldg(words + j) >> 32);
+    uint32_t hi = end;
+    ++p;
+    while (p < hi) {
+      const uint32_t mid = p + ((hi - p) >> 1);
+      if (list_name(__ldg(arr + mid)) < name) p = mid + 1; else hi = mid;
+    }
+    if (p >= end) return kInvalid;
+    *en = __ldg(arr + p);
+  }
+  return list_name(*en) == name ? p : kInvalid;
+}
+
+// Position of `name` in the indexed list arr[lb, le) or kInvalid; *en: the entry.
+// `name` may lie outside the list's range: its bucket is then arbitrary (but
+// within the 2^lg), and the entry's own name decides.
+template <class E>
+__device__ __forceinline__ uint32_t rank_find(const unsigned long long* __restrict__ pool,
+                                              const E* __restrict__ arr, uint32_t lb, uint32_t le, uint32_t mn,
+                                              uint32_t scale, uint32_t name, E* en) {
+  const uint32_t sh = rank_shift(le - lb);
+  const uint32_t bk = ((name - mn) * scale) >> sh;
+  const unsigned long long* words = pool + ((lb + 1) >> 1);
+  const unsigned long long w = __ldg(words + (bk >> 5));
+  const uint32_t bits = (uint32_t)w, bit = 1u << (bk & 31);
+  if (!(bits & bit)) return kInvalid;
+  const uint32_t p = (uint32_t)(w >> 32) + __popc(bits & (bit - 1));
+  *en = __ldg(arr + p);
+  const uint32_t x = list_name(*en);
+  if (x < name) return rank_later(arr, p, le, words, bk, sh, name, en);
+  return x == name ? p : kInvalid;
+}
+
+// Entry p of the list [b, e): the first entry of each word writes it, with the
+// empty words before it; the last entry writes the empty words after it.  Every
+// word is written once, by one thread, so the pool needs no clearing.
+template <class E>
+__device__ __forceinline__ void rank_emit(const E* __restrict__ arr, uint32_t b, uint32_t e, uint32_t p, uint32_t mn,
+                                          uint32_t scale, unsigned long long* __restrict__ pool) {
+  const uint32_t sh = rank_shift(e - b);
+  unsigned long long* wp = pool + ((b + 1) >> 1);
+  uint32_t bk = ((list_name(__ldg(arr + p)) - mn) * scale) >> sh;
+  const uint32_t j = bk >> 5;
+  // words this entry is the first at or past: (word of the entry before, j]
+  uint32_t k = p == b ? 0u : ((((list_name(__ldg(arr + p - 1)) - mn) * scale) >> sh) >> 5) + 1;
+  if (k <= j) {
+    for (; k < j; ++k) wp[k] = (unsigned long long)p << 32;
+    uint32_t bits = 0;
+    for (uint32_t q = p; (bk >> 5) == j;) {
+      bits |= 1u << (bk & 31);
+      if (++q == e) break;
+      bk = ((list_name(__ldg(arr + q)) - mn) * scale) >> sh;
+    }
+    wp[j] = bits | ((unsigned long long)p << 32);
+  }
+  if (p + 1 == e)
+    for (k = j + 1; k < (1u << (27 - sh)); ++k) wp[k] = (unsigned long long)e << 32;
+}
+
+// Headers of all lists and the words of those of at least `min_len` entries
+// (>= 8), 32 lists per warp: each qualifying list is walked by the whole warp,
+// lists longer than kWarpRow are listed for k_rank_index_big (chunks of 1024
+// entries spread over all blocks).
+template <class E>
+__global__ void __launch_bounds__(256) k_rank_index(const uint32_t* __restrict__ off, uint32_t n, uint32_t min_len,
+                                                    const E* __restrict__ arr, unsigned long long* __restrict__ pool,
+                                                    unsigned long long* __restrict__ hdr,
+                                                    uint32_t* __restrict__ big, uint32_t* __restrict__ big_count) {
+  const uint32_t lane = lane_id();
+  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t u0 = warp * 32; u0 < n; u0 += nwarps * 32) {
+    const uint32_t u = u0 + lane;
+    uint32_t b = 0, e = 0, mn = 0, scale = 0;
+    if (u < n) {
+      b = __ldg(off + u);
+      e = __ldg(off + u + 1);
+      if (e - b >= min_len) {
+        mn = list_name(__ldg(arr + b));
+        scale = rank_scale(mn, list_name(__ldg(arr + e - 1)));
+      }
+      hdr[u] = mn | ((unsigned long long)scale << 32);
+    }
+    const bool large = scale && e - b > kWarpRow;
+    if (large) big[atomicAdd(big_count, 1u)] = u;
+    unsigned todo = __ballot_sync(kFull, scale && !large);
+    while (todo) {
+      const int j = __ffs(todo) - 1;
+      todo &= todo - 1;
+      const uint32_t rb = __shfl_sync(kFull, b, j), re = __shfl_sync(kFull, e, j);
+      const uint32_t rm = __shfl_sync(kFull, mn, j), rs = __shfl_sync(kFull, scale, j);
+      for (uint32_t p = rb + lane; p < re; p += 32) rank_emit(arr, rb, re, p, rm, rs, pool);
+    }
+  }
+}
+
+template <class E>
+__global__ void __launch_bounds__(256) k_rank_index_big(const uint32_t* __restrict__ off,
+                                                        const E* __restrict__ arr,
+                                                        unsigned long long* __restrict__ pool,
+                                                        const unsigned long long* __restrict__ hdr,
+                                                        const uint32_t* __restrict__ big,
+                                                        const uint32_t* __restrict__ big_count) {
+  const uint32_t nb = *big_count;
+  uint32_t c0 = 0;  // chunks of the lists before list i
+  for (uint32_t i = 0; i < nb; ++i) {
+    const uint32_t u = big[i];
+    const uint32_t b = __ldg(off + u), e = __ldg(off + u + 1);
+    const uint32_t chunks = (e - b + 1023) / 1024;
+    const unsigned long long h = hdr[u];
+    // chunk x belongs to block (c0 + x) mod gridDim.x
+    for (uint32_t x = (blockIdx.x + gridDim.x - c0 % gridDim.x) % gridDim.x; x < chunks; x += gridDim.x)
+      for (uint32_t p = b + x * 1024 + threadIdx.x; p < min(e, b + (x + 1) * 1024); p += blockDim.x)
+        rank_emit(arr, b, e, p, (uint32_t)h, (uint32_t)(h >> 32), pool);
+    c0 += chunks;
+  }
+}
 
 // ---------------------------------------------------------------------------
 // Kernel C (balanced form): per oriented edge e = (a -> b), each element of the
@@ -792,16 +941,27 @@ template <class StartF>
 __device__ __forceinline__ uint32_t window_find(const StartF& start, uint32_t i, uint32_t count,
                                                 unsigned long long j, bool valid);
 
-// 8 resident blocks per SM (32 registers): the pass is latency-bound and
-// loses more to fewer warps than to the few spilled values.
-//
+// What bounds it: issue slots (61% busy) and the latency of its three dependent
+// loads (element, word, entry); the credits are a tenth of it (R-MAT-20 9.1 ms
+// with them, 8.2 without).  Hence the most warps (8 blocks of 256 threads per
+// SM, 32 registers: 40.3 ms on R-MAT-22, 42.7 / 44.0 / 43.6 at 7 / 6 / 5 blocks
+// with 2 / 2 / 3 groups in flight), and a run of at least kSupRun elements of
+// one edge goes kSupWays groups of 32 at a time with its loads side by side (one
+// group 50.0 ms, two 40.3).  Against binary searches narrowed through 64 samples
+// of the longer list the rank index takes the pass from 80.0 to 40.3 ms on
+// R-MAT-22 (11.8 G elements), 15.0 to 8.5 ms on R-MAT-20; 4 to 8 buckets per entry
+// instead of 8 to 16 cost 5 ms more.
+constexpr int kSupBlocks = 8;
+constexpr int kSupRun = 24;
+constexpr int kSupWays = 2;
+
 // kMulti (multigraphs, `mu` = multiplicity per edge id): a triangle of pairs
 // (e, f, h) stands for mu_e * mu_f * mu_h triangles of copies, so a copy of e
 // is credited mu_f * mu_h (each hit lane adds its own product; the one-atomic
 // run credit of the simple form is for unit weights only).
 //
 // kHash: out-lists of at least hash_min entries have an open-addressed table
-// of (id | position << 32) at 4 * their start in `hpool` (k_table_fill with
+// of (name | position << 32) at 4 * their start in `hpool` (k_table_fill with
 // OutListSource, the same layout as the peel's row tables), probed instead of
 // searched.
 __device__ __forceinline__ uint32_t probe_list(const unsigned long long* __restrict__ hpool, uint32_t lb,
@@ -820,19 +980,27 @@ __device__ __forceinline__ uint32_t probe_list(const unsigned long long* __restr
   return kInvalid;
 }
 
-#ifndef SPARX_SUP_SAMPLES
-#define SPARX_SUP_SAMPLES 2  // samples of a long out-list per lane in the support fast path (2 or 4)
-#endif
-constexpr int kSupSamples = SPARX_SUP_SAMPLES;
-static_assert(kSupSamples == 2 || kSupSamples == 4, "2 or 4 samples per lane");
-constexpr int kSupSampleShift = kSupSamples == 4 ? 7 : 6;  // log2 of the sample count
+// Credit of one hit (f, h: positions of c in the two lists) of edge e.
+__device__ __forceinline__ void credit_multi(int2* __restrict__ es, const uint32_t* __restrict__ mu, uint32_t e,
+                                             uint32_t f, uint32_t h, unsigned long long* found) {
+  const uint32_t me = __ldg(mu + e), mf = __ldg(mu + f), mh = __ldg(mu + h);
+  atomicAdd(&es[f].x, (int)(me * mh));
+  atomicAdd(&es[h].x, (int)(me * mf));
+  atomicAdd(&es[e].x, (int)(mf * mh));
+  *found += (unsigned long long)me * mf * mh;
+}
 
+// `oname`: the lists' keys, ascending in each list (the ids themselves when
+// there is no index); `hdr` / `pool`: rank index of the lists of at least
+// rank_min entries (hdr nullptr: none).
 template <bool kMulti, bool kHash>
-__global__ void __launch_bounds__(256, 8) k_support_balanced(
+__global__ void __launch_bounds__(256, kSupBlocks) k_support_balanced(
     const uint32_t* __restrict__ opos, const uint32_t* __restrict__ ocol,
-    const uint32_t* __restrict__ osrc, const unsigned long long* __restrict__ spref, uint32_t m,
-    int2* __restrict__ es, unsigned long long* __restrict__ tri_total, uint32_t* __restrict__ err,
-    const uint32_t* __restrict__ mu, uint32_t sample_min, const unsigned long long* __restrict__ hpool,
+    const uint32_t* __restrict__ osrc, const uint32_t* __restrict__ oname,
+    const unsigned long long* __restrict__ spref, uint32_t m,
+    int2* __restrict__ es, unsigned long long* __restrict__ tri_total,
+    const uint32_t* __restrict__ mu, uint32_t rank_min, const unsigned long long* __restrict__ hdr,
+    const unsigned long long* __restrict__ pool, const unsigned long long* __restrict__ hpool,
     uint32_t hash_min) {
   const uint32_t lane = lane_id();
   const unsigned long long total = spref[m];
@@ -845,40 +1013,112 @@ __global__ void __launch_bounds__(256, 8) k_support_balanced(
   for (unsigned long long c0 = warp * ch; c0 < total; c0 += nwarps * ch) {
     const unsigned long long kend = min(c0 + ch, total);
     uint32_t i = warp_last_le(PrefKey{spref}, 0, m - 1, c0);
-    for (unsigned long long kb = c0; kb < kend; kb += 32) {
+    for (unsigned long long kb = c0; kb < kend;) {
+      // edge i owns element kb (or has none left: then some later edge does)
+      const unsigned long long e_start = spref[i], e_end = min(kend, spref[i + 1]);
+      if (e_end >= kb + kSupRun) {
+        // the rest of a long edge: its lists are the same for the whole warp
+        const uint32_t a = __ldg(osrc + i), b = __ldg(ocol + i);
+        const uint32_t ab = __ldg(opos + a), ae = __ldg(opos + a + 1);
+        const uint32_t bb = __ldg(opos + b), be = __ldg(opos + b + 1);
+        const bool a_short = ae - ab <= be - bb;
+        const uint32_t flb = a_short ? bb : ab, fle = a_short ? be : ae;
+        const unsigned long long fh = hdr && fle - flb >= rank_min ? __ldg(hdr + (a_short ? b : a)) : 0ull;
+        const uint32_t mn = (uint32_t)fh, scale = (uint32_t)(fh >> 32);
+        const bool hashed = kHash && fle - flb >= hash_min;
+        const uint32_t f0 = (a_short ? ab : bb) + (uint32_t)(kb - e_start);
+        const uint32_t f1 = f0 + (uint32_t)(e_end - kb);
+        int cnt = 0;
+        auto credit = [&](uint32_t f, uint32_t q) {
+          if (kMulti) {
+            credit_multi(es, mu, i, f, q, &found_total);
+          } else {
+            atomicAdd(&es[f].x, 1);
+            atomicAdd(&es[q].x, 1);
+            ++cnt;
+          }
+        };
+        if (scale && !hashed) {
+          // kSupWays groups of 32 at a time: their words, then their entries,
+          // are loaded together
+          const uint32_t sh = rank_shift(fle - flb);
+          const unsigned long long* words = pool + ((flb + 1) >> 1);
+          for (uint32_t f = f0 + lane; f < f1; f += 32 * kSupWays) {
+            uint32_t c[kSupWays], p[kSupWays], x[kSupWays];
+            unsigned long long w[kSupWays];
+#pragma unroll
+            for (int j = 0; j < kSupWays; ++j) c[j] = f + 32 * j < f1 ? __ldg(oname + f + 32 * j) : mn;
+#pragma unroll
+            for (int j = 0; j < kSupWays; ++j) {
+              p[j] = ((c[j] - mn) * scale) >> sh;
+              w[j] = __ldg(words + (p[j] >> 5));
+            }
+#pragma unroll
+            for (int j = 0; j < kSupWays; ++j) {
+              const uint32_t bit = 1u << (p[j] & 31);
+              const bool maybe = ((uint32_t)w[j] & bit) && f + 32 * j < f1;
+              p[j] = maybe ? (uint32_t)(w[j] >> 32) + __popc((uint32_t)w[j] & (bit - 1)) : kInvalid;
+              x[j] = maybe ? __ldg(oname + p[j]) : 0xFFFFFFFFu;
+            }
+#pragma unroll
+            for (int j = 0; j < kSupWays; ++j) {
+              if (x[j] < c[j]) p[j] = rank_later(oname, p[j], fle, words, ((c[j] - mn) * scale) >> sh, sh, c[j], &x[j]);
+              if (x[j] == c[j] && p[j] != kInvalid) credit(f + 32 * j, p[j]);
+            }
+          }
+        } else {
+          for (uint32_t f = f0 + lane; f < f1; f += 32) {
+            const uint32_t c = __ldg(oname + f);
+            if (hashed) {
+              const uint32_t q = probe_list(hpool, flb, fle - flb, c);
+              if (q != kInvalid) credit(f, q);
+            } else {
+              const uint32_t q = lower_bound_u32(oname, flb, fle, c);
+              if (q < fle && __ldg(oname + q) == c) credit(f, q);
+            }
+          }
+        }
+        if (!kMulti) {  // the edge's own credit, once per run
+          found_total += cnt;
+          cnt = __reduce_add_sync(kFull, cnt);
+          if (lane == 0 && cnt) atomicAdd(&es[i].x, cnt);
+        }
+        kb = e_end;
+        i = min(i + 1, m - 1);
+        continue;
+      }
+      // short edges: 32 elements, each lane finds its own edge and lists
       const unsigned long long k = kb + lane;
       const bool valid = k < kend;
       const uint32_t e = window_find(ps, i, m, k, valid);
       const uint32_t last = (uint32_t)min(31ull, kend - 1 - kb);
       const uint32_t e_last = __shfl_sync(kFull, e, last);
-      uint32_t o = 0, sb = 0, lb = 0, le = 0;
+      uint32_t o = 0, sb = 0, lb = 0, le = 0, lv = 0;
       if (valid) {
         o = (uint32_t)(k - spref[e]);
         const uint32_t a = __ldg(osrc + e), b = __ldg(ocol + e);
         const uint32_t ab = __ldg(opos + a), ae = __ldg(opos + a + 1);
         const uint32_t bb = __ldg(opos + b), be = __ldg(opos + b + 1);
-        if (ae - ab <= be - bb) { sb = ab; lb = bb; le = be; }
-        else { sb = bb; lb = ab; le = ae; }
+        if (ae - ab <= be - bb) { sb = ab; lb = bb; le = be; lv = b; }
+        else { sb = bb; lb = ab; le = ae; lv = a; }
       }
       uint32_t p = kInvalid;  // position of c in the longer list
       if (valid) {
-        const uint32_t c = __ldg(ocol + sb + o);
+        const uint32_t c = __ldg(oname + sb + o);
         if (kHash && le - lb >= hash_min) {
           p = probe_list(hpool, lb, le - lb, c);
+        } else if (hdr && le - lb >= rank_min) {
+          const unsigned long long h = __ldg(hdr + lv);
+          uint32_t en;
+          p = rank_find(pool, oname, lb, le, (uint32_t)h, (uint32_t)(h >> 32), c, &en);
         } else {
-          const uint32_t q = lower_bound_u32(ocol, lb, le, c);
-          if (q < le && __ldg(ocol + q) == c) p = q;
+          const uint32_t q = lower_bound_u32(oname, lb, le, c);
+          if (q < le && __ldg(oname + q) == c) p = q;
         }
       }
       const bool hit = valid && p != kInvalid;
       if (kMulti) {
-        if (hit) {
-          const uint32_t me = __ldg(mu + e), mf = __ldg(mu + sb + o), mh = __ldg(mu + p);
-          atomicAdd(&es[sb + o].x, (int)(me * mh));
-          atomicAdd(&es[p].x, (int)(me * mf));
-          atomicAdd(&es[e].x, (int)(mf * mh));
-          found_total += (unsigned long long)me * mf * mh;
-        }
+        if (hit) credit_multi(es, mu, e, sb + o, p, &found_total);
       } else {
         if (hit) {
           atomicAdd(&es[sb + o].x, 1);
@@ -894,95 +1134,7 @@ __global__ void __launch_bounds__(256, 8) k_support_balanced(
         }
       }
       i = e_last;
-      // fast path: while the next 32 elements all lie inside edge i, the
-      // lists and the element offsets are the same for the whole warp
-      const unsigned long long nb = kb + 32;
-      const unsigned long long e_end = i + 1 < m ? spref[i + 1] : total;
-      if (nb + 32 <= min(kend, e_end)) {
-        const unsigned long long e_start = spref[i];
-        const uint32_t a = __ldg(osrc + i), b = __ldg(ocol + i);
-        const uint32_t ab = __ldg(opos + a), ae = __ldg(opos + a + 1);
-        const uint32_t bb = __ldg(opos + b), be = __ldg(opos + b + 1);
-        const bool a_short = ae - ab <= be - bb;
-        const uint32_t fsb = a_short ? ab : bb, flb = a_short ? bb : ab, fle = a_short ? be : ae;
-        const unsigned long long stop = min(kend, e_end);
-        // a long list is narrowed first through 32 * kSupSamples evenly spaced
-        // samples, kSupSamples per lane (gathered once per edge, then
-        // shuffles), leaving that fraction of it to search
-        const uint32_t flen = fle - flb;
-        const bool hashed = kHash && flen >= hash_min;
-        const bool sampled = !hashed && flen >= sample_min;
-        uint32_t smp[kSupSamples];
-#pragma unroll
-        for (int x = 0; x < kSupSamples; ++x)
-          smp[x] = sampled ? __ldg(ocol + flb + (uint32_t)(((unsigned long long)(kSupSamples * lane + x) * flen) >>
-                                                          kSupSampleShift))
-                           : 0u;
-        do {
-          kb += 32;
-          const uint32_t fo = (uint32_t)(kb + lane - e_start);
-          const uint32_t c = __ldg(ocol + fsb + fo);
-          uint32_t lo = flb, hi = fle;
-          if (hashed) {
-            const uint32_t q = probe_list(hpool, flb, flen, c);
-            const bool fh = q != kInvalid;
-            if (kMulti) {
-              if (fh) {
-                const uint32_t me = __ldg(mu + i), mf = __ldg(mu + fsb + fo), mh = __ldg(mu + q);
-                atomicAdd(&es[fsb + fo].x, (int)(me * mh));
-                atomicAdd(&es[q].x, (int)(me * mf));
-                atomicAdd(&es[i].x, (int)(mf * mh));
-                found_total += (unsigned long long)me * mf * mh;
-              }
-            } else {
-              if (fh) {
-                atomicAdd(&es[fsb + fo].x, 1);
-                atomicAdd(&es[q].x, 1);
-                found_total++;
-              }
-              const int cnt = __popc(__ballot_sync(kFull, fh));
-              if (lane == 0 && cnt) atomicAdd(&es[i].x, cnt);
-            }
-            continue;
-          }
-          if (sampled) {
-            uint32_t t = 0;
-#pragma unroll
-            for (int d = 16; d > 0; d >>= 1) {
-              const uint32_t cand = __shfl_sync(kFull, smp[0], t + d);
-              if (cand <= c) t += d;
-            }
-            // lane t's first sample is the last lane-first one <= c; its
-            // other samples (ascending) decide how far past it c lies
-            uint32_t kk = kSupSamples * t;
-#pragma unroll
-            for (int x = 1; x < kSupSamples; ++x) kk += __shfl_sync(kFull, smp[x], t) <= c ? 1u : 0u;
-            lo = flb + (uint32_t)(((unsigned long long)kk * flen) >> kSupSampleShift);
-            hi = kk == 32 * kSupSamples - 1
-                     ? fle
-                     : flb + (uint32_t)(((unsigned long long)(kk + 1) * flen) >> kSupSampleShift);
-          }
-          const uint32_t q = lower_bound_u32(ocol, lo, hi, c);
-          const bool fh = q < hi && __ldg(ocol + q) == c;
-          if (kMulti) {
-            if (fh) {
-              const uint32_t me = __ldg(mu + i), mf = __ldg(mu + fsb + fo), mh = __ldg(mu + q);
-              atomicAdd(&es[fsb + fo].x, (int)(me * mh));
-              atomicAdd(&es[q].x, (int)(me * mf));
-              atomicAdd(&es[i].x, (int)(mf * mh));
-              found_total += (unsigned long long)me * mf * mh;
-            }
-          } else {
-            if (fh) {
-              atomicAdd(&es[fsb + fo].x, 1);
-              atomicAdd(&es[q].x, 1);
-              found_total++;
-            }
-            const int cnt = __popc(__ballot_sync(kFull, fh));
-            if (lane == 0 && cnt) atomicAdd(&es[i].x, cnt);
-          }
-        } while (kb + 64 <= stop);
-      }
+      kb += 32;
     }
   }
 #pragma unroll
@@ -2909,11 +3061,11 @@ struct RowPairSource {
     return (uint32_t)(pr >> 32) == kInvalid ? ~0ull : pr;
   }
 };
-// support: (column id | position << 32) from the oriented out-lists
+// support: (name | position << 32) from the oriented out-lists
 struct OutListSource {
-  const uint32_t* ocol;
+  const uint32_t* oname;
   __device__ __forceinline__ unsigned long long operator()(uint32_t j) const {
-    return (unsigned long long)__ldg(ocol + j) | ((unsigned long long)j << 32);
+    return (unsigned long long)__ldg(oname + j) | ((unsigned long long)j << 32);
   }
 };
 

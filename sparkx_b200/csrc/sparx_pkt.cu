@@ -69,7 +69,7 @@ int status_from_flags(uint32_t f) {
 struct Tuning {
   uint32_t merge_ratio = 8;        // peel: merge the rows when the longer is <= ratio x the shorter
   uint32_t hub_min_degree = 1024;  // dense hub maps for vertices of at least this degree (0: none)
-  uint32_t sample_min = 64;        // support: longer out-lists from this length go through 64 samples
+  uint32_t sample_min = 64;        // support: longer out-lists from this length are searched through a rank index
   uint32_t support_kernel = 1;     // 1 balanced edge form, 2 vertex form
   uint32_t compact_pct = 85;       // rebuild the peel's rows when live entries fill <= this % of them
   uint32_t hash_min_degree = 128;  // rows of at least this degree get a hash table for the per-lane search (0: none)
@@ -518,12 +518,23 @@ void exclusive_scan(F f, unsigned long long count, T* out, T* tiles, T* grand, c
 // beyond what a CTA can hold the balanced form runs instead.
 constexpr size_t kHeavySmemLimit = 160u << 10;
 
+// What the balanced form needs besides the oriented lists.  The rank index of
+// the lists of at least `rank_min` entries lives in arrays the peel fills
+// later; `hdr` nullptr (no list is that long, or no room): the names are the
+// ids and every list is binary searched.
+struct SupportIndex {
+  const uint32_t* oname = nullptr;
+  unsigned long long* hdr = nullptr;   // one per vertex
+  unsigned long long* pool = nullptr;  // (m + 1) / 2 words
+  uint32_t* big = nullptr;             // lists longer than kWarpRow
+  uint32_t rank_min = Tuning{}.sample_min;
+};
+
 int launch_support(int sm_count, uint32_t support_kernel, uint32_t n, uint64_t m, uint32_t max_dplus,
                    const uint32_t* opos, const uint32_t* ocol, const uint32_t* osrc, int2* es,
                    unsigned long long* spref, unsigned long long* tiles, Counters* cnt, uint32_t* heavy_list,
-                   cudaStream_t s, uint32_t* launches, unsigned long long* support_elements,
-                   const uint32_t* mu = nullptr, uint32_t sample_min = Tuning{}.sample_min,
-                   const unsigned long long* hpool = nullptr, uint32_t hash_min = 0) {
+                   cudaStream_t s, uint32_t* launches, unsigned long long* support_elements, const SupportIndex& X,
+                   const uint32_t* mu = nullptr, const unsigned long long* hpool = nullptr, uint32_t hash_min = 0) {
   if (m == 0) return SPARX_OK;
   uint32_t slots = 8;
   while (slots < 2 * max_dplus) slots <<= 1;
@@ -541,22 +552,24 @@ int launch_support(int sm_count, uint32_t support_kernel, uint32_t n, uint64_t m
     *support_elements = 0;
     return SPARX_OK;
   }
+  if (X.hdr) {
+    CU(cudaMemsetAsync(&cnt->table_big, 0, 4, s));
+    k_rank_index<uint32_t><<<grid_for(n, 256, sm_count * 16), 256, 0, s>>>(opos, n, X.rank_min, X.oname, X.pool,
+                                                                           X.hdr, X.big, &cnt->table_big);
+    k_rank_index_big<uint32_t><<<sm_count * 4, 256, 0, s>>>(opos, X.oname, X.pool, X.hdr, X.big, &cnt->table_big);
+    *launches += 2;
+  }
   exclusive_scan<unsigned long long>(SupportWork{opos, osrc, ocol}, m, spref, tiles, &cnt->grand, s);
-  const int g = sm_count * 8;
+  const int g = sm_count * kSupBlocks;
   const uint32_t mm = (uint32_t)m;
+  auto go = [&](auto kernel) {
+    kernel<<<g, 256, 0, s>>>(opos, ocol, osrc, X.oname, spref, mm, es, &cnt->tri, mu, X.rank_min, X.hdr, X.pool,
+                             hpool, hash_min);
+  };
   if (hpool && hash_min) {
-    if (mu)
-      k_support_balanced<true, true><<<g, 256, 0, s>>>(opos, ocol, osrc, spref, mm, es, &cnt->tri, &cnt->err, mu,
-                                                       sample_min, hpool, hash_min);
-    else
-      k_support_balanced<false, true><<<g, 256, 0, s>>>(opos, ocol, osrc, spref, mm, es, &cnt->tri, &cnt->err,
-                                                        nullptr, sample_min, hpool, hash_min);
-  } else if (mu) {
-    k_support_balanced<true, false><<<g, 256, 0, s>>>(opos, ocol, osrc, spref, mm, es, &cnt->tri, &cnt->err, mu,
-                                                      sample_min, nullptr, 0);
+    if (mu) go(k_support_balanced<true, true>); else go(k_support_balanced<false, true>);
   } else {
-    k_support_balanced<false, false><<<g, 256, 0, s>>>(opos, ocol, osrc, spref, mm, es, &cnt->tri, &cnt->err,
-                                                       nullptr, sample_min, nullptr, 0);
+    if (mu) go(k_support_balanced<true, false>); else go(k_support_balanced<false, false>);
   }
   *launches += 4;
   CU(cudaMemcpyAsync(support_elements, spref + m, 8, cudaMemcpyDeviceToHost, s));
@@ -950,9 +963,23 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
   if (2 * m + hc.self_loops != Ws) { J.err = kErrAsym; return SPARX_E_INVALID_CSR; }
   for (const Member& M : J.members)
     if (M.m > kEidMask) { set_error("a graph has >= 2^28 edges"); return SPARX_E_TOO_LARGE; }
+  const Tuning T = resolve_tuning(tune_key(hist, hist_slots, Ws));
+  J.tuning = T;
+  // the support pass's rank index, in arrays that are idle until the peel
+  // (4-entry lists cannot fill a word's 32 buckets: 8 at least)
+  SupportIndex X;
+  X.rank_min = std::max<uint32_t>(T.sample_min, 8);
+  X.oname = ocol;
+  if (hc.max_dplus >= X.rank_min) {
+    X.oname = at<uint32_t>(E, L.act1);
+    X.hdr = at<unsigned long long>(E, L.vinfo);
+    X.pool = at<unsigned long long>(E, L.qd0);
+    X.big = at<uint32_t>(E, L.act0);
+  }
   {
     uint32_t* owner = at<uint32_t>(E, L.q0);  // in-slot owners; the q buffers are idle until the peel
-    k_orient_fill<<<vgrid, 256, 0, s>>>(J.off, J.nbr, N, opos, ocol, osrc, row0, owner, big, &cnt->big_count);
+    k_orient_fill<<<vgrid, 256, 0, s>>>(J.off, J.nbr, N, opos, ocol, osrc, row0, owner, big, &cnt->big_count,
+                                        const_cast<uint32_t*>(X.hdr ? X.oname : nullptr));
     k_orient_reverse<<<grid_for(Ws, 256, E.sm_count * 16), 256, 0, s>>>(J.nbr, owner, Ws, opos, ocol, row0, err);
     if (J.multi) {
       // multiplicity per edge id from its out-slot; the in-slot must agree
@@ -968,8 +995,6 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
   J.launches += 2;
   // hub maps: the smallest power-of-two degree bound (>= kHubMinDegree) whose
   // vertices fit the reserved maps; hist[b] counts degrees in [2^(b-1), 2^b)
-  const Tuning T = resolve_tuning(tune_key(hist, hist_slots, Ws));
-  J.tuning = T;
   uint32_t hubs = 0, hub_min_deg = 0;
   if (hubs_possible && T.hub_min_degree) {
     uint64_t above = 0;
@@ -1049,8 +1074,8 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
       sup_hash_min = T.sup_hash_min;
       CU(cudaMemsetAsync(big_count, 0, 4, s));
       k_table_fill<<<grid_for(N, kTableWarps * 32, E.sm_count * 16), kTableWarps * 32, 0, s>>>(
-          opos, N, sup_hash_min, nullptr, OutListSource{ocol}, spool, big_list, big_count);
-      k_table_fill_big<<<E.sm_count * 8, 256, 0, s>>>(opos, big_list, big_count, OutListSource{ocol}, spool);
+          opos, N, sup_hash_min, nullptr, OutListSource{X.oname}, spool, big_list, big_count);
+      k_table_fill_big<<<E.sm_count * 8, 256, 0, s>>>(opos, big_list, big_count, OutListSource{X.oname}, spool);
       J.launches += 2;
     }
   }
@@ -1062,7 +1087,7 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
     int rc = launch_support(E.sm_count, O.support_kernel ? O.support_kernel : T.support_kernel, N, m,
                             hc.max_dplus, opos, ocol, osrc, es, at<unsigned long long>(E, L.q0),
                             at<unsigned long long>(E, L.tiles), cnt, at<uint32_t>(E, L.act0), s, &J.launches,
-                            &J.support_elements, mu, T.sample_min, spool, sup_hash_min);
+                            &J.support_elements, X, mu, spool, sup_hash_min);
     if (rc) return rc;
   }
   CU(cudaEventRecord(E.tev[3], s));
@@ -3423,8 +3448,18 @@ int run_noalloc(const uint64_t* d_offsets, uint64_t n_plus_1, const uint32_t* d_
     set_error("a graph has >= 2^28 edges");
     return SPARX_E_TOO_LARGE;
   }
+  // the support pass's rank index, in arrays that are idle until the peel (the
+  // headers where one per vertex fits: no more vertices than slots)
+  SupportIndex X;
+  X.oname = ocol;
+  if (hc.max_dplus >= X.rank_min && N <= width) {
+    X.oname = (uint32_t*)P(L.act1);
+    X.hdr = (unsigned long long*)P(L.qd1);
+    X.pool = (unsigned long long*)P(L.qd0);
+    X.big = (uint32_t*)P(L.act0);
+  }
   k_orient_fill<<<vgrid, 256, 0, s>>>(off, d_nbr, N, opos, ocol, osrc, row0, (uint32_t*)P(L.q0), big,
-                                      &cnt->big_count);
+                                      &cnt->big_count, const_cast<uint32_t*>(X.hdr ? X.oname : nullptr));
   k_orient_reverse<<<grid_for(width, 256, sm * 16), 256, 0, s>>>(d_nbr, (uint32_t*)P(L.q0), width, opos, ocol,
                                                                 row0, err);
 
@@ -3433,7 +3468,7 @@ int run_noalloc(const uint64_t* d_offsets, uint64_t n_plus_1, const uint32_t* d_
     uint32_t launches = 0;
     unsigned long long elements = 0;
     rc = launch_support(sm, 0, N, m, hc.max_dplus, opos, ocol, osrc, es, (unsigned long long*)P(L.q0),
-                        (unsigned long long*)P(L.tiles), cnt, (uint32_t*)P(L.act0), s, &launches, &elements);
+                        (unsigned long long*)P(L.tiles), cnt, (uint32_t*)P(L.act0), s, &launches, &elements, X);
     if (rc) return rc;
   }
 
