@@ -81,10 +81,10 @@ typedef struct sparx_pkt_stats {
   uint64_t peel_scanned;      /* active-list entries read by level scans */
   uint64_t peel_edges;        /* frontier edges processed (= m minus zero-support edges) */
   uint32_t compactions;       /* rebuilds of the peel's working rows */
-  uint32_t hub_maps;          /* dense neighbour -> edge maps built for the highest-degree vertices */
-  uint64_t merge_iters;       /* peel warp iterations resolved by a row merge */
-  uint64_t lane_iters;        /* peel warp iterations resolved by per-lane searches */
-  uint64_t merge_chunks;      /* 32-entry chunks of longer rows read by the merges */
+  uint32_t hub_maps;          /* hub maps built (rows of the highest-degree vertices) */
+  uint64_t merge_iters;       /* peel: groups of 32 elements inside one frontier edge */
+  uint64_t lane_iters;        /* peel: groups of 32 elements over several edges */
+  uint64_t merge_chunks;      /* 0 (rows are no longer merged) */
 } sparx_pkt_stats;
 
 /* Fill `opts` with defaults (wide support, u8 output, device loop). */
@@ -237,9 +237,9 @@ int sparx_mtx_to_csr(const char* text, uint64_t len, uint64_t* offsets_out, uint
  */
 typedef struct sparx_tuning {
   uint32_t struct_size;     /* sizeof(sparx_tuning) */
-  uint32_t merge_ratio;     /* peel: merge the two rows when the longer is <= this x the shorter (8) */
-  uint32_t hub_min_degree;  /* dense neighbour -> edge maps for vertices of at least this degree,
-                               >= 256, or 0 for none (1024) */
+  uint32_t merge_ratio;     /* 1..1024; kept with the key, no effect: rows are no longer merged (8) */
+  uint32_t hub_min_degree;  /* hub maps (a rank index with twice the buckets) for the rows of vertices
+                               of at least this degree, >= 256, or 0 for none (1024) */
   uint32_t sample_min;      /* support: longer out-lists of at least this length (8 at least) are
                                searched through a rank index, shorter ones by binary search (64) */
   uint32_t support_kernel;  /* 1 balanced edge form, 2 vertex form (1; 2 for keys with no
@@ -247,10 +247,11 @@ typedef struct sparx_tuning {
                                which is what sparx_tuning_lookup reports for such a key) */
   uint32_t compact_pct;     /* peel: rebuild the working rows once live entries fill at most
                                this percentage of them (85) */
-  uint32_t hash_min_degree; /* peel: rows of at least this degree (>= 8) get a hash table that the
-                               per-lane search probes instead of a binary search; 0 = none (128).
-                               Skipped, with the same results, when its workspace (32 B per slot
-                               plus 16 B per edge) is over a batch's budget or cannot be allocated */
+  uint32_t hash_min_degree; /* peel: rows of at least a quarter of this many entries (>= 8; 8 at least)
+                               are searched through a rank index instead of by binary search; 0 = hub
+                               rows only (128).  Skipped, with the same results, when its workspace
+                               (8 B per slot plus 16 B per edge) is over a batch's budget or cannot be
+                               allocated */
   uint32_t sup_hash_min;    /* support: oriented out-lists of at least this length (>= 4) get a hash
                                table probed instead of the search; 0 = none (0) */
   uint32_t relabel;         /* graphs and batched unions without parallel edges: rebuild the CSR on vertex ids
@@ -275,8 +276,8 @@ int sparx_tuning_load(const char* path);
 /*
  * Autotune on one sample graph (host, the reference's layout): coordinate
  * descent from the defaults over the support form and sampling threshold
- * (timed by the support pass), then the hub floor, merge ratio and compaction
- * fill and row hash floor (timed by orientation + peel); `repeats` decompositions per candidate
+ * (timed by the support pass), then the hub floor, compaction
+ * fill and index floor (timed by orientation + peel); `repeats` decompositions per candidate
  * (median).  Stores the winner under the sample's key and returns it.
  */
 int sparx_autotune(const uint64_t* offsets, uint64_t n_plus_1, const uint64_t* neighbours, uint64_t width,
@@ -328,7 +329,7 @@ typedef struct sparx_server sparx_server;
  * the lane's second engine and placed behind the running members).  A union
  * takes no joins while it holds a graph of more than 2^26 slots or while its
  * waves average more than 60 us (newcomers then wait for a lane), and a union
- * without join room gets the row hash tables.  Every member's result goes back
+ * without join room gets the rank index.  Every member's result goes back
  * as soon as its own peel ends.  A request needing
  * more than any lane holds completes with SPARX_E_OOM.  Requests stay
  * addressable by ticket until sparx_server_destroy. */

@@ -9,8 +9,9 @@
 //
 // Layout in HBM (u32 indices: width < 2^32, m < 2^28 per member):
 //   off[n+1], nbr[width]        narrowed CSR, rows sorted ascending
-//   row0[width] (u64)           the same rows as (id | edge id << 32) pairs, in
-//                               slot order (edge id 0xFFFFFFFF: self-loop)
+//   row0[width] (u64)           the same rows as (name | edge id << 32) pairs, in
+//                               slot order (edge id 0xFFFFFFFF: self-loop); a
+//                               vertex's name is off[v], ascending with its id
 //   dplus[n], opos[n+1]         degree-ordered out-degree and its prefix
 //   ocol[m], osrc[m]            oriented edge e = (osrc[e] -> ocol[e]); e is the
 //                               undirected edge id; rank(osrc) < rank(ocol)
@@ -25,13 +26,9 @@
 //                               without processed edges whenever the live
 //                               edges fill at most 85% of it (two ping-pong
 //                               buffers)
-//   hub maps                    neighbour id -> edge id for the highest-degree
-//                               vertices (each spans its own member's ids)
-//   row hash tables (u64)       open-addressed (id | edge id << 32) entries,
-//                               2^(1+ceil(log2 d)) of them at 4 * off[v] for
-//                               rows of degree >= the tuning's floor
-//   vinfo[n] (u64)              per vertex: hub base (kVinfoHub set) or the
-//                               table's (log2 size << 32 | position), 0: none
+//   rank index (u64)            per row of the working CSR: where its names lie
+//                               (see rank_find); rebuilt with the rows
+//   vinfo[n] (u64)              per vertex: the header of its row's rank index
 #pragma once
 
 #include <cstdint>
@@ -63,11 +60,9 @@ enum : uint32_t {
 
 enum : uint32_t { kPhaseScan0 = 0, kPhaseScan = 1, kPhaseProc = 2, kPhaseDone = 3 };
 
-constexpr uint32_t kVinfoHub = 0x80000000u;  // Union::vinfo: the longer row's vertex has a hub map
-
 struct Union {  // the prepared concatenated graph, as the peel sees it
   const uint32_t* off;             // working row offsets
-  const unsigned long long* row;   // working rows: (id | edge id << 32)
+  const unsigned long long* row;   // working rows: (name | edge id << 32)
   const uint32_t* opos;
   const uint32_t* ocol;
   const uint32_t* osrc;
@@ -75,17 +70,9 @@ struct Union {  // the prepared concatenated graph, as the peel sees it
   uint32_t* act[2];
   unsigned long long* q[2];
   uint4* qd[2];                    // per queue entry {short row start, length, long row begin, end}
-  const uint32_t* hub_slot;        // vertex -> hub map index or kInvalid; nullptr = no hub maps
-  const uint32_t* hub_map;         // map pool: hub k's neighbour id w -> hub_map[hub_base[k] + w]
-  const uint32_t* hub_base;        // per hub: its map's start in the pool minus its member's first
-                                   // vertex id (u32 arithmetic, so base + w wraps into the map)
-  const unsigned long long* hpool; // row hash tables (nullptr = none): vertex v's at 4 * off0[v]
-  const uint32_t* off0;            // the rows' original offsets (hash table positions)
-  uint2* qh[2];                    // per queue entry: {hash table position, log2 capacity} or 0
-  const unsigned long long* vinfo; // per vertex, what a frontier edge's longer row offers (k_vinfo):
-                                   // kVinfoHub | hub map base, or {table position, log2 capacity},
-                                   // or 0; nullptr when there are neither hub maps nor tables
-  uint32_t hash_min;               // rows of at least this degree have a hash table (0: none)
+  const unsigned long long* rpool; // rank index of the working rows (nullptr = none)
+  const unsigned long long* vinfo; // per vertex: its row's index header {smallest name, scale}, scale 0: none
+  uint2* qh[2];                    // per queue entry: the longer row's index header (nullptr = no index)
   uint32_t n;
   uint32_t m;
   uint32_t width;
@@ -106,18 +93,10 @@ struct PeelArrays {
   unsigned long long* q1;
   uint4* qd0;
   uint4* qd1;
-  const uint32_t* hub_slot;
-  const uint32_t* hub_map;
-  const uint32_t* hub_base;
   const uint32_t* mu;    // multigraphs: multiplicity per edge id (nullptr: simple graph)
-  const unsigned long long* hpool;
-  const uint32_t* off0;
+  const unsigned long long* rpool;
   uint2* qh0;
   uint2* qh1;
-  uint32_t n;
-  uint32_t merge_ratio;  // merge the rows when the longer is at most this many times the shorter
-  uint32_t hash_min;
-  uint32_t pad;
 };
 
 // Field-by-field copy of a device-resident Union into registers (a struct
@@ -134,42 +113,27 @@ struct UnionRegs {
   unsigned long long* q1;
   uint4* qd0;
   uint4* qd1;
-  const uint32_t* __restrict__ hub_slot;
-  const uint32_t* __restrict__ hub_map;
-  const uint32_t* __restrict__ hub_base;
   const uint32_t* __restrict__ mu;
-  const unsigned long long* __restrict__ hpool;
-  const uint32_t* __restrict__ off0;
+  const unsigned long long* __restrict__ rpool;
   uint2* qh0;
   uint2* qh1;
   const unsigned long long* __restrict__ vinfo;
-  uint32_t n;
-  uint32_t hash_min;
   __device__ __forceinline__ explicit UnionRegs(const Union* p)
       : off(p->off), row(p->row), ocol(p->ocol), osrc(p->osrc), es(p->es),
         act0(p->act[0]), act1(p->act[1]), q0(p->q[0]), q1(p->q[1]),
-        qd0(p->qd[0]), qd1(p->qd[1]), hub_slot(p->hub_slot), hub_map(p->hub_map), hub_base(p->hub_base),
-        mu(nullptr), hpool(p->hpool), off0(p->off0), qh0(p->qh[0]), qh1(p->qh[1]), vinfo(p->vinfo), n(p->n),
-        hash_min(p->hash_min) {}
+        qd0(p->qd[0]), qd1(p->qd[1]), mu(nullptr), rpool(p->rpool), qh0(p->qh[0]), qh1(p->qh[1]), vinfo(p->vinfo) {}
   __device__ __forceinline__ UnionRegs(const Union* p, const PeelArrays& a)
       : off(p->off), row(p->row), ocol(a.ocol), osrc(a.osrc), es(a.es),
         act0(a.act0), act1(a.act1), q0(a.q0), q1(a.q1),
-        qd0(a.qd0), qd1(a.qd1), hub_slot(a.hub_slot), hub_map(a.hub_map), hub_base(a.hub_base), mu(a.mu),
-        hpool(a.hpool), off0(a.off0), qh0(a.qh0), qh1(a.qh1), vinfo(nullptr), n(a.n), hash_min(a.hash_min) {}
+        qd0(a.qd0), qd1(a.qd1), mu(a.mu), rpool(a.rpool), qh0(a.qh0), qh1(a.qh1), vinfo(nullptr) {}
 };
 
-// Row hash tables: vertex v of original degree d >= hash_min (and no hub map)
-// has an open-addressed table of its (neighbour id | edge id << 32) pairs with
-// 2^(1 + ceil(log2 d)) entries (at most 4d, so at 4 * off0[v] the tables of
-// consecutive vertices never overlap), probed linearly from a multiplicative
-// hash of the id; an empty entry is all ones.
+// Open-addressed hash tables of oriented lists (a tuned option of the support
+// pass): 2^(1 + ceil(log2 d)) entries (at most 4d, so at 4 * the list's start
+// consecutive tables never overlap), probed linearly from a multiplicative
+// hash of the name; an empty entry is all ones.
 __device__ __forceinline__ uint32_t hash_log2cap(uint32_t d) { return 1u + (d > 1 ? 32u - __clz(d - 1) : 0u); }
 __device__ __forceinline__ uint32_t hash_first(uint32_t w, uint32_t lg) { return (w * 0x9E3779B1u) >> (32 - lg); }
-
-// A queue-entry descriptor whose longer row belongs to a hub carries kHubDesc
-// in place of the longer row's begin and the hub's map base in place of its
-// end (row positions stay below 2^31 whenever hub maps are built).
-constexpr uint32_t kHubDesc = 0x80000000u;
 
 struct Member {  // static per-member ranges
   uint32_t vb, n;   // vertices [vb, vb + n)
@@ -210,9 +174,8 @@ struct Control {
   uint32_t compactions;
   uint32_t compact_pct;           // compact when live entries fill at most this % of the working rows
   uint32_t pad0;
-  unsigned long long merge_iters; // warp iterations resolved by the row merge
-  unsigned long long lane_iters;  // warp iterations resolved by per-lane searches
-  unsigned long long merge_chunks;// 32-entry chunks of longer rows read by merges
+  unsigned long long merge_iters; // groups of 32 elements inside one frontier edge
+  unsigned long long lane_iters;  // groups of 32 elements over several edges
   // optional wave trace: per planned wave {start time (ns), work, members in
   // a frontier step, members in a scan}; nullptr = off
   ulonglong4* trace;
@@ -254,8 +217,8 @@ __device__ __forceinline__ uint32_t lower_bound_u32(const uint32_t* __restrict__
   return lo;
 }
 
-// Position of id w in the sorted row pairs [lo, hi) or kInvalid.  Ids inside
-// a row are spread close to uniformly (vertex ids carry no degree order), so
+// Position of name w in the sorted row pairs [lo, hi) or kInvalid (rows without
+// a rank index).  Names inside a row are spread close to evenly, so
 // up to three interpolation probes narrow a long row before the binary search:
 // on a 160k-entry hub row that is ~6 dependent loads instead of ~17.
 __device__ __forceinline__ uint32_t find_in_row(const unsigned long long* __restrict__ row, uint32_t lo,
@@ -550,12 +513,20 @@ __global__ void __launch_bounds__(256) k_orient_count(const uint32_t* __restrict
 }
 
 // Kernel B2: fill oriented lists (kept in id order) and, for each vertex's
-// out-slots, the (id | edge id << 32) pair of row0; self-loop slots get edge id
-// 0xFFFFFFFF.  In-slots are left to B3: owner[s] = u marks them (kInvalid for
-// the others).  `oname` (nullptr: not wanted) takes the out-slots' names (the
+// out-slots, the (name | edge id << 32) pair of row0; self-loop slots get edge id
+// 0xFFFFFFFF.  In-slots get their name; their edge id is left to B3: owner[s] = u
+// marks them (kInvalid for the others).  `oname` (nullptr: not wanted) takes the out-slots' names (the
 // rank index's keys, off[v]).
-__device__ __forceinline__ unsigned long long make_pair(uint32_t id, uint32_t e) {
-  return (unsigned long long)id | ((unsigned long long)e << 32);
+__device__ __forceinline__ unsigned long long make_pair(uint32_t name, uint32_t e) {
+  return (unsigned long long)name | ((unsigned long long)e << 32);
+}
+
+// the two halves of a pair
+__device__ __forceinline__ uint32_t& pair_name(unsigned long long* row, unsigned long long s) {
+  return reinterpret_cast<uint32_t*>(row)[2 * s];
+}
+__device__ __forceinline__ uint32_t& pair_eid(unsigned long long* row, unsigned long long s) {
+  return reinterpret_cast<uint32_t*>(row)[2 * s + 1];
 }
 
 __global__ void __launch_bounds__(256) k_orient_fill(const uint32_t* __restrict__ off,
@@ -580,16 +551,18 @@ __global__ void __launch_bounds__(256) k_orient_fill(const uint32_t* __restrict_
       for (uint32_t s = b; s < e; ++s) {
         const uint32_t v = __ldg(nbr + s);
         uint32_t own = kInvalid;
+        const uint32_t name = v < n ? __ldg(off + v) : 0u;
         if (v == u || v >= n) {
-          row0[s] = make_pair(v, kInvalid);
-        } else if (rank_less(e - b, u, deg_of(off, v), v)) {
+          row0[s] = make_pair(name, kInvalid);
+        } else if (rank_less(e - b, u, __ldg(off + v + 1) - name, v)) {
           ocol[p] = v;
           osrc[p] = u;
-          if (oname) oname[p] = __ldg(off + v);
-          row0[s] = make_pair(v, p);
+          if (oname) oname[p] = name;
+          row0[s] = make_pair(name, p);
           ++p;
         } else {
           own = u;
+          pair_name(row0, s) = name;
         }
         owner[s] = own;
       }
@@ -604,13 +577,14 @@ __global__ void __launch_bounds__(256) k_orient_fill(const uint32_t* __restrict_
       for (uint32_t s0 = bb; s0 < be; s0 += 32) {
         const uint32_t s = s0 + lane;
         bool out = false;
-        uint32_t v = 0;
+        uint32_t v = 0, name = 0;
         if (s < be) {
           v = __ldg(nbr + s);
           uint32_t own = kInvalid;
-          if (v == bu || v >= n) row0[s] = make_pair(v, kInvalid);
-          else if (rank_less(du, bu, deg_of(off, v), v)) out = true;
-          else own = bu;
+          if (v < n) name = __ldg(off + v);
+          if (v == bu || v >= n) row0[s] = make_pair(name, kInvalid);
+          else if (rank_less(du, bu, __ldg(off + v + 1) - name, v)) out = true;
+          else { own = bu; pair_name(row0, s) = name; }
           owner[s] = own;
         }
         const unsigned bal = __ballot_sync(kFull, out);
@@ -618,8 +592,8 @@ __global__ void __launch_bounds__(256) k_orient_fill(const uint32_t* __restrict_
           const uint32_t p = p0 + __popc(bal & ((1u << lane) - 1));
           ocol[p] = v;
           osrc[p] = bu;
-          if (oname) oname[p] = __ldg(off + v);
-          row0[s] = make_pair(v, p);
+          if (oname) oname[p] = name;
+          row0[s] = make_pair(name, p);
         }
         p0 += __popc(bal);
       }
@@ -635,17 +609,18 @@ __global__ void __launch_bounds__(256) k_orient_fill(const uint32_t* __restrict_
     uint32_t p0 = __ldg(opos + bu);
     for (uint32_t base = bb; base < be; base += 4 * blockDim.x) {
       const uint32_t s0 = base + 4 * threadIdx.x;
-      uint32_t v[4], outm = 0, nout = 0;
+      uint32_t v[4], name[4], outm = 0, nout = 0;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        v[i] = 0;
+        v[i] = name[i] = 0;
         const uint32_t s = s0 + i;
         if (s < be) {
           v[i] = __ldg(nbr + s);
           uint32_t own = kInvalid;
-          if (v[i] == bu || v[i] >= n) row0[s] = make_pair(v[i], kInvalid);
-          else if (rank_less(du, bu, deg_of(off, v[i]), v[i])) { outm |= 1u << i; ++nout; }
-          else own = bu;
+          if (v[i] < n) name[i] = __ldg(off + v[i]);
+          if (v[i] == bu || v[i] >= n) row0[s] = make_pair(name[i], kInvalid);
+          else if (rank_less(du, bu, __ldg(off + v[i] + 1) - name[i], v[i])) { outm |= 1u << i; ++nout; }
+          else { own = bu; pair_name(row0, s) = name[i]; }
           owner[s] = own;
         }
       }
@@ -656,8 +631,8 @@ __global__ void __launch_bounds__(256) k_orient_fill(const uint32_t* __restrict_
         if (outm & (1u << i)) {
           ocol[p] = v[i];
           osrc[p] = bu;
-          if (oname) oname[p] = __ldg(off + v[i]);
-          row0[s0 + i] = make_pair(v[i], p);
+          if (oname) oname[p] = name[i];
+          row0[s0 + i] = make_pair(name[i], p);
           ++p;
         }
       p0 += total;
@@ -684,9 +659,9 @@ __global__ void __launch_bounds__(256) k_orient_reverse(const uint32_t* __restri
     const uint32_t lo = __ldg(opos + v), hi = __ldg(opos + v + 1);
     const uint32_t p = lower_bound_u32(ocol, lo, hi, u);
     if (p < hi && __ldg(ocol + p) == u) {
-      row0[s] = make_pair(v, p);
+      pair_eid(row0, s) = p;
     } else {
-      row0[s] = make_pair(v, kInvalid);
+      pair_eid(row0, s) = kInvalid;
       bad = true;
     }
   }
@@ -790,10 +765,16 @@ struct SupportWork {
 // what the linear map needs (ids sorted by degree would fill few buckets).
 // Consecutive elements of an edge ask ascending names, so a warp's 32 searches
 // fall on neighbouring words and neighbouring entries, as a merge's would.
-// Words lie at (start + 1) / 2 of the pool (fewer than d / 2 of them); the
-// header is {smallest name, scale}, scale 0: no index.
-__device__ __forceinline__ uint32_t rank_shift(uint32_t d) { return 30 - hash_log2cap(d); }  // 32 - lg
-__device__ __forceinline__ uint32_t rank_scale(uint32_t mn, uint32_t mx) { return 0xFFFFFFFFu / max(mx - mn, 1u); }
+// Words lie at the list's start in the pool (fewer than d of them); the header
+// is {smallest name, scale}, scale 0: no index.  kRankFine in the scale (which
+// stays below it: 8 names span at least 7): twice the buckets, for hubs.
+constexpr uint32_t kRankFine = 0x80000000u;
+__device__ __forceinline__ uint32_t rank_shift(uint32_t d, uint32_t scale) {  // 32 - lg
+  return 30 - hash_log2cap(d) - (scale >> 31);
+}
+__device__ __forceinline__ uint32_t rank_bucket(uint32_t name, uint32_t mn, uint32_t scale, uint32_t sh) {
+  return ((name - mn) * (scale & ~kRankFine)) >> sh;
+}
 __device__ __forceinline__ uint32_t list_name(uint32_t x) { return x; }
 __device__ __forceinline__ uint32_t list_name(unsigned long long x) { return (uint32_t)x; }
 
@@ -828,9 +809,9 @@ template <class E>
 __device__ __forceinline__ uint32_t rank_find(const unsigned long long* __restrict__ pool,
                                               const E* __restrict__ arr, uint32_t lb, uint32_t le, uint32_t mn,
                                               uint32_t scale, uint32_t name, E* en) {
-  const uint32_t sh = rank_shift(le - lb);
-  const uint32_t bk = ((name - mn) * scale) >> sh;
-  const unsigned long long* words = pool + ((lb + 1) >> 1);
+  const uint32_t sh = rank_shift(le - lb, scale);
+  const uint32_t bk = rank_bucket(name, mn, scale, sh);
+  const unsigned long long* words = pool + lb;
   const unsigned long long w = __ldg(words + (bk >> 5));
   const uint32_t bits = (uint32_t)w, bit = 1u << (bk & 31);
   if (!(bits & bit)) return kInvalid;
@@ -847,19 +828,19 @@ __device__ __forceinline__ uint32_t rank_find(const unsigned long long* __restri
 template <class E>
 __device__ __forceinline__ void rank_emit(const E* __restrict__ arr, uint32_t b, uint32_t e, uint32_t p, uint32_t mn,
                                           uint32_t scale, unsigned long long* __restrict__ pool) {
-  const uint32_t sh = rank_shift(e - b);
-  unsigned long long* wp = pool + ((b + 1) >> 1);
-  uint32_t bk = ((list_name(__ldg(arr + p)) - mn) * scale) >> sh;
+  const uint32_t sh = rank_shift(e - b, scale);
+  unsigned long long* wp = pool + b;
+  uint32_t bk = rank_bucket(list_name(__ldg(arr + p)), mn, scale, sh);
   const uint32_t j = bk >> 5;
   // words this entry is the first at or past: (word of the entry before, j]
-  uint32_t k = p == b ? 0u : ((((list_name(__ldg(arr + p - 1)) - mn) * scale) >> sh) >> 5) + 1;
+  uint32_t k = p == b ? 0u : (rank_bucket(list_name(__ldg(arr + p - 1)), mn, scale, sh) >> 5) + 1;
   if (k <= j) {
     for (; k < j; ++k) wp[k] = (unsigned long long)p << 32;
     uint32_t bits = 0;
     for (uint32_t q = p; (bk >> 5) == j;) {
       bits |= 1u << (bk & 31);
       if (++q == e) break;
-      bk = ((list_name(__ldg(arr + q)) - mn) * scale) >> sh;
+      bk = rank_bucket(list_name(__ldg(arr + q)), mn, scale, sh);
     }
     wp[j] = bits | ((unsigned long long)p << 32);
   }
@@ -868,14 +849,25 @@ __device__ __forceinline__ void rank_emit(const E* __restrict__ arr, uint32_t b,
 }
 
 // Headers of all lists and the words of those of at least `min_len` entries
-// (>= 8), 32 lists per warp: each qualifying list is walked by the whole warp,
-// lists longer than kWarpRow are listed for k_rank_index_big (chunks of 1024
-// entries spread over all blocks).
+// (>= 8), 32 lists per warp: each qualifying list is walked by the whole warp.
+// Lists longer than kRankWarpList are cut into chunks of kRankChunk entries for
+// k_rank_index_chunks: with degree-ordered vertices the long lists are
+// neighbours, and one warp walking 32 of 2000 entries held up the pass.  Rows of
+// vertices of original degree (off0) >= fine_min > 0 get the fine index, down to
+// 8 entries left; `fine_count` (or nullptr) counts them.
+constexpr uint32_t kRankWarpList = 128;
+constexpr uint32_t kRankChunk = 1024;
+// chunks listed for lists of `w` entries together
+__host__ __device__ constexpr unsigned long long rank_chunks_max(unsigned long long w) {
+  return w / kRankWarpList + w / kRankChunk + 1;
+}
 template <class E>
 __global__ void __launch_bounds__(256) k_rank_index(const uint32_t* __restrict__ off, uint32_t n, uint32_t min_len,
                                                     const E* __restrict__ arr, unsigned long long* __restrict__ pool,
                                                     unsigned long long* __restrict__ hdr,
-                                                    uint32_t* __restrict__ big, uint32_t* __restrict__ big_count) {
+                                                    uint2* __restrict__ chunks, uint32_t* __restrict__ chunk_count,
+                                                    const uint32_t* __restrict__ off0, uint32_t fine_min,
+                                                    uint32_t* __restrict__ fine_count) {
   const uint32_t lane = lane_id();
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -885,14 +877,23 @@ __global__ void __launch_bounds__(256) k_rank_index(const uint32_t* __restrict__
     if (u < n) {
       b = __ldg(off + u);
       e = __ldg(off + u + 1);
-      if (e - b >= min_len) {
+      const bool fine = fine_min && __ldg(off0 + u + 1) - __ldg(off0 + u) >= fine_min;
+      if (e - b >= (fine ? 8u : min_len)) {
         mn = list_name(__ldg(arr + b));
-        scale = rank_scale(mn, list_name(__ldg(arr + e - 1)));
+        scale = 0xFFFFFFFFu / max(list_name(__ldg(arr + e - 1)) - mn, 1u);
+        if (fine) {
+          scale |= kRankFine;
+          if (fine_count) atomicAdd(fine_count, 1u);
+        }
       }
       hdr[u] = mn | ((unsigned long long)scale << 32);
     }
-    const bool large = scale && e - b > kWarpRow;
-    if (large) big[atomicAdd(big_count, 1u)] = u;
+    const bool large = scale && e - b > kRankWarpList;
+    if (large) {
+      const uint32_t k = (e - b + kRankChunk - 1) / kRankChunk;
+      const uint32_t at = atomicAdd(chunk_count, k);
+      for (uint32_t x = 0; x < k; ++x) chunks[at + x] = make_uint2(u, x);
+    }
     unsigned todo = __ballot_sync(kFull, scale && !large);
     while (todo) {
       const int j = __ffs(todo) - 1;
@@ -905,24 +906,20 @@ __global__ void __launch_bounds__(256) k_rank_index(const uint32_t* __restrict__
 }
 
 template <class E>
-__global__ void __launch_bounds__(256) k_rank_index_big(const uint32_t* __restrict__ off,
-                                                        const E* __restrict__ arr,
-                                                        unsigned long long* __restrict__ pool,
-                                                        const unsigned long long* __restrict__ hdr,
-                                                        const uint32_t* __restrict__ big,
-                                                        const uint32_t* __restrict__ big_count) {
-  const uint32_t nb = *big_count;
-  uint32_t c0 = 0;  // chunks of the lists before list i
-  for (uint32_t i = 0; i < nb; ++i) {
-    const uint32_t u = big[i];
-    const uint32_t b = __ldg(off + u), e = __ldg(off + u + 1);
-    const uint32_t chunks = (e - b + 1023) / 1024;
-    const unsigned long long h = hdr[u];
-    // chunk x belongs to block (c0 + x) mod gridDim.x
-    for (uint32_t x = (blockIdx.x + gridDim.x - c0 % gridDim.x) % gridDim.x; x < chunks; x += gridDim.x)
-      for (uint32_t p = b + x * 1024 + threadIdx.x; p < min(e, b + (x + 1) * 1024); p += blockDim.x)
-        rank_emit(arr, b, e, p, (uint32_t)h, (uint32_t)(h >> 32), pool);
-    c0 += chunks;
+__global__ void __launch_bounds__(256) k_rank_index_chunks(const uint32_t* __restrict__ off,
+                                                           const E* __restrict__ arr,
+                                                           unsigned long long* __restrict__ pool,
+                                                           const unsigned long long* __restrict__ hdr,
+                                                           const uint2* __restrict__ chunks,
+                                                           const uint32_t* __restrict__ chunk_count) {
+  const uint32_t nc = *chunk_count;
+  for (uint32_t i = blockIdx.x; i < nc; i += gridDim.x) {
+    const uint2 c = chunks[i];
+    const uint32_t b = __ldg(off + c.x), e = __ldg(off + c.x + 1);
+    const unsigned long long h = hdr[c.x];
+    const uint32_t end = min(e, b + (c.y + 1) * kRankChunk);
+    for (uint32_t p = b + c.y * kRankChunk + threadIdx.x; p < end; p += blockDim.x)
+      rank_emit(arr, b, e, p, (uint32_t)h, (uint32_t)(h >> 32), pool);
   }
 }
 
@@ -1041,8 +1038,8 @@ __global__ void __launch_bounds__(256, kSupBlocks) k_support_balanced(
         if (scale && !hashed) {
           // kSupWays groups of 32 at a time: their words, then their entries,
           // are loaded together
-          const uint32_t sh = rank_shift(fle - flb);
-          const unsigned long long* words = pool + ((flb + 1) >> 1);
+          const uint32_t sh = rank_shift(fle - flb, scale);
+          const unsigned long long* words = pool + flb;
           for (uint32_t f = f0 + lane; f < f1; f += 32 * kSupWays) {
             uint32_t c[kSupWays], p[kSupWays], x[kSupWays];
             unsigned long long w[kSupWays];
@@ -1487,43 +1484,18 @@ struct WaveArgs {
 };
 
 // Rows of frontier edge x in the working CSR: {shorter row start, its length,
-// longer row begin, longer row end}, or {.., .., kHubDesc, hub map base} when
-// the longer row's vertex has a hub map.  The length is the edge's work.
-// *hq: the longer row's hash table {position, log2 capacity}, or {0, 0}.
+// longer row begin, longer row end}.  The length is the edge's work.  *hq: the
+// longer row's index header, or {0, 0}.
 __device__ __forceinline__ uint4 edge_desc(const UnionRegs& U, uint32_t x, uint2* hq) {
   const uint32_t u = __ldg(U.osrc + x), v = __ldg(U.ocol + x);
-  // row bounds and both vertices' longer-row offers, all in one round of loads
+  // row bounds and both rows' index headers, all in one round of loads
   const uint32_t ub = __ldg(U.off + u), ue = __ldg(U.off + u + 1);
   const uint32_t vb = __ldg(U.off + v), ve = __ldg(U.off + v + 1);
   const unsigned long long iu = U.vinfo ? __ldg(U.vinfo + u) : 0ull, iv = U.vinfo ? __ldg(U.vinfo + v) : 0ull;
   const bool u_short = ue - ub <= ve - vb;
   const unsigned long long li = u_short ? iv : iu;
-  const uint32_t lo = (uint32_t)li, hi = (uint32_t)(li >> 32);
-  *hq = make_uint2(0, 0);
-  if (hi & kVinfoHub)
-    return u_short ? make_uint4(ub, ue - ub, kHubDesc, lo) : make_uint4(vb, ve - vb, kHubDesc, lo);
-  if (hi) *hq = make_uint2(lo, hi);
+  *hq = make_uint2((uint32_t)li, (uint32_t)(li >> 32));
   return u_short ? make_uint4(ub, ue - ub, vb, ve) : make_uint4(vb, ve - vb, ub, ue);
-}
-
-// What each vertex's row offers when it is a frontier edge's longer row: its
-// hub map (kVinfoHub | the map's base), else its hash table (log2 capacity <<
-// 32 | the table's position), else nothing.
-__global__ void __launch_bounds__(256) k_vinfo(uint32_t n, const uint32_t* __restrict__ hub_slot,
-                                               const uint32_t* __restrict__ hub_base,
-                                               const uint32_t* __restrict__ off0, uint32_t hash_min,
-                                               unsigned long long* __restrict__ vinfo) {
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-    unsigned long long info = 0;
-    const uint32_t hs = hub_slot ? __ldg(hub_slot + v) : kInvalid;
-    if (hs != kInvalid) {
-      info = ((unsigned long long)kVinfoHub << 32) | __ldg(hub_base + hs);
-    } else if (hash_min) {
-      const uint32_t b0 = __ldg(off0 + v), d0 = __ldg(off0 + v + 1) - b0;
-      if (d0 >= hash_min) info = ((unsigned long long)hash_log2cap(d0) << 32) | (4u * b0);
-    }
-    vinfo[v] = info;
-  }
 }
 
 // PKT sub-level rule for one triangle (e, f, h) of frontier edge e at level l,
@@ -1541,10 +1513,9 @@ __global__ void __launch_bounds__(256) k_vinfo(uint32_t n, const uint32_t* __res
 // removes mu_e * mu_h of them from each copy of f (mu_e * mu_f from h): the
 // charge is that product, applied at once.
 template <bool kMulti>
-__device__ __forceinline__ void pkt_rule(const UnionRegs& U, uint32_t e, uint32_t f, int2 es_f, uint32_t h,
+__device__ __forceinline__ void pkt_rule(const UnionRegs& U, uint32_t e, uint32_t f, int2 es_f, uint32_t h, int2 es_h,
                                          uint32_t l, uint32_t W, bool& pf, bool& ph) {
   pf = ph = false;
-  const int2 es_h = U.es[h];
   const uint32_t tf = (uint32_t)es_f.y, th = (uint32_t)es_h.y;
   if (tf < W || th < W) return;
   const int32_t sf = es_f.x, sh = es_h.x;
@@ -1622,13 +1593,14 @@ enum : int { kCtxEb = 0, kCtxM, kCtxLevel, kCtxQsel, kCtxQcount, kCtxSegLen, kCt
 // kept active-list entries staged per warp before one atomic reserves their
 // place: every kept entry of a large scan goes through one counter per member
 constexpr int kKeepBuf = 256;
-#ifndef SPARX_MERGE_CHUNKS
-#define SPARX_MERGE_CHUNKS 2  // long-row chunks of 32 entries loaded per merge round
-#endif
-constexpr int kMergeChunks = SPARX_MERGE_CHUNKS;
-#ifndef SPARX_STATE_AFTER_SEARCH
-#define SPARX_STATE_AFTER_SEARCH 1  // read the other edges' states after the search, on hits only
-#endif
+// A run of at least kWaveRun elements of one frontier edge goes kWaveWays groups
+// of 32 at a time, their row entries, index words, found entries and states
+// loaded side by side: the wave waits for memory (19 long-scoreboard stall
+// cycles per issue in a large wave, DRAM at 28%), so loads in flight count most
+// (R-MAT-22's peel 277 ms with one group, 257 with two; 272 / 285 ms with two
+// groups at 6 / 5 blocks per SM instead of 8).
+constexpr int kWaveWays = 2;
+constexpr uint32_t kWaveRun = 24;
 
 struct PushStage {
   uint32_t* eid;  // this warp's kPushBuf staged edges
@@ -1665,7 +1637,7 @@ __device__ __noinline__ void push_flush_cold(const uint32_t* eid, uint32_t n, co
     if (pos + lane < M.m) {
       qnext[M.eb + pos + lane] = ((ws + p0 - d0.y) << kEidBits) | (x0 - M.eb);
       qdnext[M.eb + pos + lane] = d0;
-      if (U.hash_min) qhnext[M.eb + pos + lane] = h0;
+      if (U.qh0) qhnext[M.eb + pos + lane] = h0;
     } else {
       atomicOr(err, kErrCapacity);
     }
@@ -1674,7 +1646,7 @@ __device__ __noinline__ void push_flush_cold(const uint32_t* eid, uint32_t n, co
     if (pos + 32 + lane < M.m) {
       qnext[M.eb + pos + 32 + lane] = ((ws + t0 + p1 - d1.y) << kEidBits) | (x1 - M.eb);
       qdnext[M.eb + pos + 32 + lane] = d1;
-      if (U.hash_min) qhnext[M.eb + pos + 32 + lane] = h1;
+      if (U.qh0) qhnext[M.eb + pos + 32 + lane] = h1;
     } else {
       atomicOr(err, kErrCapacity);
     }
@@ -1929,6 +1901,12 @@ __device__ __noinline__ void wave_scan_segment(const Union* Up, MemberState* st,
 //                       <= level -> queued for this level; else kept
 //   frontier element j  element o of the shorter working row of frontier
 //                       edge e, searched in the longer row; a hit is a triangle
+// The search is one word of the longer row's rank index for most absent names
+// and one entry more for the others; it replaced a row merge (similar lengths),
+// per-row hash tables and dense hub maps, whose probes were random DRAM sectors:
+// R-MAT-22's peel 315 -> 257 ms, its first large wave 0.87 -> 0.68 ms on R-MAT-20
+// with 0.60 -> 0.36 G instructions and 2.7 -> 1.4 GB read.  The index is rebuilt
+// with the rows at every compaction, so it shrinks with what is left.
 template <bool kMulti>
 __global__ void __launch_bounds__(kWaveThreads, SPARX_WAVE_MINB) k_wave(WaveArgs a) {
   __shared__ uint32_t s_push_eid[kWaveWarps][kPushBuf];
@@ -1944,16 +1922,15 @@ __global__ void __launch_bounds__(kWaveThreads, SPARX_WAVE_MINB) k_wave(WaveArgs
   const unsigned long long warp = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const unsigned long long nwarps = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
   const UnionRegs U(a.Up, a.arr);
-  const bool hubs = U.hub_map != nullptr;  // descriptors carry kHubDesc only when maps exist
   // one chunk per warp: finer chunks (and any cap on their size) measured
   // slower, the search for a chunk's first entry is paid once per warp;
   // ch * nwarps >= total, so the chunk below is the warp's only one
   const unsigned long long ch = max(((total + nwarps - 1) / nwarps + 31) & ~31ull, 32ull);
-  // work counters live in shared memory (per warp: hits, merge iterations,
-  // lane iterations, merge chunks) rather than in four registers held across
-  // the loop; lane 0 adds to them
-  __shared__ uint32_t s_cnt[4][kWaveWarps];
-  if (lane < 4) s_cnt[lane][wib] = 0;
+  // work counters live in shared memory (per warp: hits, groups of 32 elements
+  // inside one edge, groups over several edges) rather than in registers held
+  // across the loop; lane 0 adds to them
+  __shared__ uint32_t s_cnt[3][kWaveWarps];
+  if (lane < 3) s_cnt[lane][wib] = 0;
   __syncwarp();
   PushStage ps{s_push_eid[wib], 0};
   // Warp-uniform state of the frontier loop lives in shared memory and is read
@@ -2008,13 +1985,10 @@ __global__ void __launch_bounds__(kWaveThreads, SPARX_WAVE_MINB) k_wave(WaveArgs
         }
         __syncwarp();
         uint32_t i = i0;
-        // merge cursor carried across iterations that continue the same edge
-        uint32_t m_e = kInvalid, m_next_o = 0, m_cur = 0;
-        for (uint32_t r = 0; r < w32[kCtxSegLen]; r += 32) {
+        uint32_t found = 0;
+        for (uint32_t r = 0; r < w32[kCtxSegLen];) {
           const uint32_t seg_len = w32[kCtxSegLen];
           const uint32_t qcount = w32[kCtxQcount];
-          const unsigned long long* q = (w32[kCtxQsel] ? U.q1 : U.q0) + w32[kCtxEb];
-          const bool valid = r + lane < seg_len;
           // the window's entries, loaded once: each lane picks its own by a
           // shuffle search on the work starts (entries own >= 1 element, so
           // 32 consecutive elements span at most 32 entries).  The search runs
@@ -2024,153 +1998,121 @@ __global__ void __launch_bounds__(kWaveThreads, SPARX_WAVE_MINB) k_wave(WaveArgs
           // past the queue's end clamp to the most negative.  Lane l's
           // element jr + l lies in entry x iff jr - start(x) >= -l.
           const unsigned long long jr = w64[kCtxJb] + r;
-          const unsigned long long qv = (i + lane < qcount) ? q[i + lane] : ~0ull;
+          const unsigned long long qv =
+              (i + lane < qcount) ? ((w32[kCtxQsel] ? U.q1 : U.q0) + w32[kCtxEb])[i + lane] : ~0ull;
           const int32_t dq = (int32_t)max((long long)(jr - (qv >> kEidBits)), (long long)INT32_MIN);
-          uint32_t t = 0;
+          // elements of entry i from jr on (an end past the queue is 2^31)
+          const uint32_t rem = min(seg_len - r, 0u - (uint32_t)__shfl_sync(kFull, dq, 1));
+          bool valid;
+          uint32_t e = 0, o = 0;
+          uint4 dsc = make_uint4(0, 0, 0, 0);
+          uint2 hq = make_uint2(0, 0);
+          uint32_t o_end;       // the lane's elements o, o + 32, ... below o_end
+          const bool run = (int32_t)rem >= (int32_t)kWaveRun;
+          uint32_t x = i;
+          if (run) {
+            // the rest of entry i: one edge, the same rows for the whole warp
+            e = w32[kCtxEb] + __shfl_sync(kFull, (uint32_t)qv & kEidMask, 0);
+            o = (uint32_t)__shfl_sync(kFull, dq, 0) + lane;
+            valid = true;
+            o_end = o - lane + rem;
+            r += rem;
+            i += 1;
+            if (lane == 0) s_cnt[1][wib] += (rem + 31) / 32;
+          } else {
+            uint32_t t = 0;
 #pragma unroll
-          for (int d = 16; d > 0; d >>= 1) {
-            const int32_t cand = __shfl_sync(kFull, dq, t + d);
-            if (cand >= -(int32_t)lane) t += d;
+            for (int d = 16; d > 0; d >>= 1) {
+              const int32_t cand = __shfl_sync(kFull, dq, t + d);
+              if (cand >= -(int32_t)lane) t += d;
+            }
+            o = (uint32_t)(__shfl_sync(kFull, dq, t) + (int32_t)lane);
+            e = w32[kCtxEb] + __shfl_sync(kFull, (uint32_t)qv & kEidMask, t);
+            x = i + t;
+            const uint32_t last = min(31u, seg_len - 1 - r);
+            i = __shfl_sync(kFull, x, last);
+            valid = r + lane < seg_len;
+            o_end = o + 1;
+            r += 32;
+            if (lane == 0) s_cnt[2][wib]++;
           }
-          const int32_t dt = __shfl_sync(kFull, dq, t);
-          const uint32_t eid_t = __shfl_sync(kFull, (uint32_t)qv & kEidMask, t);
-          const uint32_t x = i + t;
-          const uint32_t last = min(31u, seg_len - 1 - r);
-          const uint32_t x_last = __shfl_sync(kFull, x, last);
-          uint32_t e = 0, o = 0, sb = 0, slen = 0, lb = 0, le = 0;
           if (valid) {
-            e = w32[kCtxEb] + eid_t;
-            o = (uint32_t)(dt + (int32_t)lane);
-            const uint4 dsc = ((w32[kCtxQsel] ? U.qd1 : U.qd0) + w32[kCtxEb])[x];
-            sb = dsc.x;
-            slen = dsc.y;
-            lb = dsc.z;
-            le = dsc.w;
+            dsc = ((w32[kCtxQsel] ? U.qd1 : U.qd0) + w32[kCtxEb])[x];
+            if (U.qh0) hq = ((w32[kCtxQsel] ? U.qh1 : U.qh0) + w32[kCtxEb])[x];
           }
           // rows may have been compacted since the entry's work was counted
-          const bool el = valid && o < slen;
-          unsigned long long pr = el ? __ldg(U.row + sb + o) : 0ull;
-          const uint32_t w = (uint32_t)pr;
-          uint32_t f = (uint32_t)(pr >> 32), h = kInvalid, p = kInvalid;
-          // f == kInvalid: a self-loop entry; f == e: the frontier edge itself
-          bool look = el && f != kInvalid && f != e;
-          int2 es_f = make_int2(0, 0);
-#if !SPARX_STATE_AFTER_SEARCH
-          // the other edge of the short row: already processed -> nothing to resolve
-          if (look) {
-            es_f = U.es[f];
-            look = (uint32_t)es_f.y >= w32[kCtxW];
-          }
-#endif
-          // lane 0 is always valid: its rows decide, so the branch and the
-          // merge below are warp-uniform
-          const uint32_t e0 = __shfl_sync(kFull, e, 0);
-          const uint32_t L_beg = __shfl_sync(kFull, lb, 0), L_end = __shfl_sync(kFull, le, 0);
-          const uint32_t s_len0 = __shfl_sync(kFull, slen, 0);
-          const bool one_edge = __all_sync(kFull, !valid || e == e0);
-          const bool hub0 = hubs && (L_beg & kHubDesc);
-          if (one_edge && !hub0 && (L_end - L_beg) <= a.arr.merge_ratio * s_len0) {
-            // similar row lengths: walk the longer row with a warp-wide cursor;
-            // every chunk of 32 entries is matched against the 32 sorted
-            // elements by a shuffle search
-            const unsigned elb = __ballot_sync(kFull, el);
-            if (elb) {
-              const uint32_t o0 = __shfl_sync(kFull, o, 0);
-              const uint32_t wmax = __shfl_sync(kFull, w, 31 - __clz(elb));
-              uint32_t cur;
-              if (m_e == e0 && m_next_o == o0) {
-                cur = m_cur;
-              } else {
-                const uint32_t wmin = __shfl_sync(kFull, w, __ffs(elb) - 1);
-                cur = warp_lower_bound(RowIdKey{U.row}, L_beg, L_end, wmin);
-              }
-              // kMergeChunks chunks are loaded per round, so most rows cost
-              // one dependent load instead of one per chunk
-              const uint32_t cap = (L_end - L_beg) / 32 + 2;
-              uint32_t nch = 0;  // chunks matched (work counter)
-              for (uint32_t it = 0;; ++it) {
-                if (it > cap) {
-                  if (lane == 0) atomicOr(a.err, kErrInternal);
-                  break;
-                }
-                unsigned long long lp[kMergeChunks];
+          o_end = valid ? min(o_end, dsc.y) : 0u;
+          const unsigned long long* words = U.rpool + dsc.z;
+          const uint32_t sh = rank_shift(dsc.w - dsc.z, hq.y);
+          // warp-uniform trips: all lanes of a run share o_end; otherwise one trip
+          const uint32_t o0 = o - lane;
+          for (uint32_t og = 0; run ? o0 + og < o_end : og == 0; og += 32 * kWaveWays, o += 32 * kWaveWays) {
+            uint32_t w[kWaveWays], f[kWaveWays], h[kWaveWays];
+            unsigned long long en[kWaveWays];
 #pragma unroll
-                for (int c = 0; c < kMergeChunks; ++c) {
-                  const uint32_t idx = cur + 32 * c + lane;
-                  lp[c] = idx < L_end ? __ldg(U.row + idx) : ~0ull;
-                }
-                uint32_t adv = 0;
-#pragma unroll
-                for (int c = 0; c < kMergeChunks; ++c) {
-                  if (c > 0 && adv < 32u * c) break;  // the row passed wmax in an earlier chunk
-                  const uint32_t lv = (uint32_t)lp[c];
-                  uint32_t tt = 0;
-#pragma unroll
-                  for (int d = 16; d > 0; d >>= 1) {
-                    const uint32_t cv = __shfl_sync(kFull, lv, tt + d);
-                    if (cv <= w) tt += d;
-                  }
-                  const uint32_t lvt = __shfl_sync(kFull, lv, tt);
-                  const uint32_t ht = (uint32_t)(__shfl_sync(kFull, lp[c], tt) >> 32);
-                  if (look && lvt == w) { p = cur + 32 * c + tt; h = ht; }
-                  adv += __popc(__ballot_sync(kFull, lv <= wmax));
-                  ++nch;
-                }
-                cur += adv;
-                if (adv < 32u * kMergeChunks) break;
-              }
-              if (lane == 0) s_cnt[3][wib] += nch;
-              m_e = e0;
-              m_next_o = o0 + 32;
-              m_cur = cur;
+            for (int j = 0; j < kWaveWays; ++j) {
+              en[j] = o + 32 * j < o_end ? __ldg(U.row + dsc.x + o + 32 * j) : ~0ull;
+              h[j] = kInvalid;
             }
-            if (lane == 0) s_cnt[1][wib]++;
-          } else {
-            if (lane == 0) s_cnt[2][wib]++;
-            m_e = kInvalid;
-            if (look) {
-              const uint2 hq = U.hash_min ? (w32[kCtxQsel] ? U.qh1 : U.qh0)[w32[kCtxEb] + x] : make_uint2(0, 0);
-              if (hubs && (lb & kHubDesc)) {
-                // the longer row's vertex has a hub map: one lookup
-                h = __ldg(U.hub_map + (uint32_t)(le + w));
-                p = h != kInvalid ? 0u : kInvalid;
-              } else if (hq.y) {
-                // the longer row has a hash table: probe from the id's hash
-                const unsigned long long* tb = U.hpool + hq.x;
-                const uint32_t mask = (1u << hq.y) - 1;
-                uint32_t at = hash_first(w, hq.y);
-#pragma unroll 1
-                for (uint32_t it = 0; it <= mask; ++it) {
-                  const unsigned long long en = __ldg(tb + at);
-                  const uint32_t id = (uint32_t)en;
-                  if (id == w) { h = (uint32_t)(en >> 32); p = 0; break; }
-                  if (id == kInvalid) break;
-                  at = (at + 1) & mask;
+            if (hq.y) {
+              // the longer row's rank index: its words, then its entries, side by side
+#pragma unroll
+              for (int j = 0; j < kWaveWays; ++j) {
+                w[j] = (uint32_t)en[j];
+                f[j] = (uint32_t)(en[j] >> 32);
+                // f == kInvalid: a self-loop entry; f == e: the frontier edge itself
+                const bool look = f[j] != kInvalid && f[j] != e;
+                en[j] = look ? __ldg(words + (rank_bucket(w[j], hq.x, hq.y, sh) >> 5)) : 0ull;
+              }
+#pragma unroll
+              for (int j = 0; j < kWaveWays; ++j) {
+                const uint32_t bit = 1u << (rank_bucket(w[j], hq.x, hq.y, sh) & 31);
+                uint32_t p = (uint32_t)(en[j] >> 32) + __popc((uint32_t)en[j] & (bit - 1));
+                if ((uint32_t)en[j] & bit) {
+                  unsigned long long at = __ldg(U.row + p);
+                  if ((uint32_t)at < w[j])
+                    p = rank_later(U.row, p, dsc.w, words, rank_bucket(w[j], hq.x, hq.y, sh), sh, w[j], &at);
+                  // h == kInvalid: the long row's own vertex (a self-loop entry)
+                  if (p != kInvalid && (uint32_t)at == w[j]) h[j] = (uint32_t)(at >> 32);
                 }
-              } else {
-                p = find_in_row(U.row, lb, le, w);
-                if (p != kInvalid) h = (uint32_t)(__ldg(U.row + p) >> 32);
+              }
+            } else {
+#pragma unroll
+              for (int j = 0; j < kWaveWays; ++j) {
+                w[j] = (uint32_t)en[j];
+                f[j] = (uint32_t)(en[j] >> 32);
+                if (f[j] != kInvalid && f[j] != e) {
+                  const uint32_t p = find_in_row(U.row, dsc.z, dsc.w, w[j]);
+                  if (p != kInvalid) h[j] = (uint32_t)(__ldg(U.row + p) >> 32);
+                }
+              }
+            }
+            // both other edges' states are read only for a found triangle (a
+            // third of the elements on R-MAT)
+            int2 sf[kWaveWays], sh2[kWaveWays];
+#pragma unroll
+            for (int j = 0; j < kWaveWays; ++j) {
+              sf[j] = sh2[j] = make_int2(0, 0);
+              if (h[j] != kInvalid) { sf[j] = U.es[f[j]]; sh2[j] = U.es[h[j]]; }
+            }
+#pragma unroll
+            for (int j = 0; j < kWaveWays; ++j) {
+              bool pf = false, ph = false;
+              if (h[j] != kInvalid) {
+                ++found;
+                pkt_rule<kMulti>(U, e, f[j], sf[j], h[j], sh2[j], w32[kCtxLevel], w32[kCtxW], pf, ph);
+              }
+              if (__any_sync(kFull, pf || ph)) {
+                push_edge(ps, U, a.Up, w32[kCtxEb], w32[kCtxM], a.st + w32[kCtxG], a.err, w32[kCtxQsel], pf, f[j],
+                          w32[kCtxW]);
+                push_edge(ps, U, a.Up, w32[kCtxEb], w32[kCtxM], a.st + w32[kCtxG], a.err, w32[kCtxQsel], ph, h[j],
+                          w32[kCtxW]);
               }
             }
           }
-          bool pf = false, ph = false;
-          // h == kInvalid: w was the long row's own vertex (a self-loop entry)
-          const bool hit = look && p != kInvalid && h != kInvalid;
-          const uint32_t nhit = __popc(__ballot_sync(kFull, hit));
-          if (lane == 0) s_cnt[0][wib] += nhit;
-#if SPARX_STATE_AFTER_SEARCH
-          // both other edges' states are read only for a found triangle (a
-          // quarter of the elements on R-MAT); the search may run for an f
-          // that is already processed, which pkt_rule then skips
-          if (hit) es_f = U.es[f];
-#endif
-          if (hit) pkt_rule<kMulti>(U, e, f, es_f, h, w32[kCtxLevel], w32[kCtxW], pf, ph);
-          push_edge(ps, U, a.Up, w32[kCtxEb], w32[kCtxM], a.st + w32[kCtxG], a.err, w32[kCtxQsel], pf, f,
-                    w32[kCtxW]);
-          push_edge(ps, U, a.Up, w32[kCtxEb], w32[kCtxM], a.st + w32[kCtxG], a.err, w32[kCtxQsel], ph, h,
-                    w32[kCtxW]);
-          i = x_last;
         }
+        found = __reduce_add_sync(kFull, found);
+        if (lane == 0) s_cnt[0][wib] += found;
         // entries belong to this member: publish before moving on
         push_flush(ps, a.Up, w32[kCtxEb], w32[kCtxM], a.st + w32[kCtxG], a.err, w32[kCtxQsel]);
         k = w64[kCtxSegEnd];
@@ -2188,14 +2130,12 @@ __global__ void __launch_bounds__(kWaveThreads, SPARX_WAVE_MINB) k_wave(WaveArgs
   // work counters: summed per block, then one atomic per counter and block
   // (per-warp atomics on four addresses serialise on large waves)
   __syncthreads();
-  if (threadIdx.x < 4) {
+  if (threadIdx.x < 3) {
     unsigned long long sum = 0;
 #pragma unroll
     for (int w = 0; w < kWaveWarps; ++w) sum += s_cnt[threadIdx.x][w];
     unsigned long long* dst = threadIdx.x == 0 ? &a.ctl->hits
-                              : threadIdx.x == 1 ? &a.ctl->merge_iters
-                              : threadIdx.x == 2 ? &a.ctl->lane_iters
-                                                 : &a.ctl->merge_chunks;
+                              : threadIdx.x == 1 ? &a.ctl->merge_iters : &a.ctl->lane_iters;
     if (sum) atomicAdd(dst, sum);
   }
   // the last block to finish plans the next wave (threadfence-reduction
@@ -2214,18 +2154,8 @@ __global__ void __launch_bounds__(kWaveThreads, SPARX_WAVE_MINB) k_wave(WaveArgs
   }
 }
 
-// Hub maps: the vertices of highest degree (at least `min_deg`, at most the
-// reserved number of maps) get a dense map from neighbour id to edge id, so a
-// frontier element whose longer row is a hub's resolves its triangle with one
-// load instead of a search of the long row.  A hub's map covers its own
-// member's vertex range only, so maps are as small as their graph, and unions
-// of many graphs get maps for the hubs of each.
-//   k_hub_hist    vertices and slots per floor(log2(degree)) (also the
-//                 degree signature the tuning is keyed on)
-//   k_hub_assign  hub index per vertex (kInvalid below the chosen degree)
-//   k_hub_layout  each hub's map base in the pool (a prefix over its member's
-//                 vertex count); hubs past the pool lose their map
-//   k_hub_fill    scatter each hub's row into its map (block per hub)
+// Vertices and slots per floor(log2(degree)): the degree signature the tuning
+// is keyed on.
 __global__ void __launch_bounds__(256) k_hub_hist(const uint32_t* __restrict__ off, uint32_t n,
                                                   uint32_t* __restrict__ hist,
                                                   unsigned long long* __restrict__ hist_slots) {
@@ -2244,74 +2174,6 @@ __global__ void __launch_bounds__(256) k_hub_hist(const uint32_t* __restrict__ o
   if (threadIdx.x < 33 && sh[threadIdx.x]) {
     atomicAdd(&hist[threadIdx.x], sh[threadIdx.x]);
     atomicAdd(&hist_slots[threadIdx.x], sl[threadIdx.x]);
-  }
-}
-
-__global__ void __launch_bounds__(256) k_hub_assign(const uint32_t* __restrict__ off, uint32_t n,
-                                                    uint32_t min_deg, uint32_t max_hubs,
-                                                    uint32_t* __restrict__ hub_slot,
-                                                    uint32_t* __restrict__ hub_vertex,
-                                                    uint32_t* __restrict__ hub_count) {
-  for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < n; u += gridDim.x * blockDim.x) {
-    const uint32_t d = __ldg(off + u + 1) - __ldg(off + u);
-    uint32_t slot = kInvalid;
-    if (d >= min_deg) {
-      slot = atomicAdd(hub_count, 1u);
-      if (slot < max_hubs) hub_vertex[slot] = u;
-      else slot = kInvalid;  // cannot happen: the host sized max_hubs from the histogram
-    }
-    hub_slot[u] = slot;
-  }
-}
-
-// One block: base of each hub's map = exclusive prefix of its member's vertex
-// count, minus the member's first vertex; a hub whose map would end past
-// `pool` entries gets none (hub_slot back to kInvalid).
-__global__ void __launch_bounds__(1024) k_hub_layout(const uint32_t* __restrict__ hub_vertex, uint32_t hubs,
-                                                     const Member* __restrict__ mem, uint32_t G,
-                                                     unsigned long long pool, uint32_t* __restrict__ hub_base,
-                                                     uint32_t* __restrict__ hub_slot) {
-  __shared__ unsigned long long sw[32];
-  unsigned long long carry = 0;
-  for (uint32_t b = 0; b < hubs; b += blockDim.x) {
-    const uint32_t k = b + threadIdx.x;
-    unsigned long long size = 0;
-    uint32_t u = 0, vb = 0;
-    if (k < hubs) {
-      u = hub_vertex[k];
-      uint32_t lo = 0, hi = G - 1;
-      while (lo < hi) {
-        const uint32_t mid = (lo + hi + 1) >> 1;
-        if (mem[mid].vb <= u) lo = mid; else hi = mid - 1;
-      }
-      vb = mem[lo].vb;
-      size = mem[lo].n;
-    }
-    unsigned long long total;
-    const unsigned long long at = carry + block_exclusive_scan<unsigned long long>(size, sw, total);
-    if (k < hubs) {
-      if (at + size <= pool) hub_base[k] = (uint32_t)at - vb;
-      else hub_slot[u] = kInvalid;
-    }
-    carry += total;
-  }
-}
-
-__global__ void __launch_bounds__(256) k_hub_fill(const uint32_t* __restrict__ off,
-                                                  const unsigned long long* __restrict__ row0,
-                                                  const uint32_t* __restrict__ hub_vertex, uint32_t hubs,
-                                                  const uint32_t* __restrict__ hub_slot,
-                                                  const uint32_t* __restrict__ hub_base,
-                                                  uint32_t* __restrict__ hub_map) {
-  for (uint32_t k = blockIdx.x; k < hubs; k += gridDim.x) {
-    const uint32_t u = hub_vertex[k];
-    if (__ldg(hub_slot + u) != k) continue;  // no room in the pool
-    const uint32_t b = __ldg(off + u), e = __ldg(off + u + 1), base = __ldg(hub_base + k);
-    for (uint32_t s = b + threadIdx.x; s < e; s += blockDim.x) {
-      const unsigned long long pr = __ldg(row0 + s);
-      const uint32_t id = (uint32_t)pr, eid = (uint32_t)(pr >> 32);
-      if (eid != kInvalid) hub_map[(uint32_t)(base + id)] = eid;
-    }
   }
 }
 
@@ -2485,7 +2347,7 @@ __global__ void __launch_bounds__(256) k_refresh_desc(const Union* __restrict__ 
   const Member M = mem[g];
   const unsigned long long* q = (s.q_sel ? U.q1 : U.q0) + M.eb;
   uint4* qd = (s.q_sel ? U.qd1 : U.qd0) + M.eb;
-  uint2* qh = U.hash_min ? (s.q_sel ? U.qh1 : U.qh0) + M.eb : nullptr;
+  uint2* qh = U.qh0 ? (s.q_sel ? U.qh1 : U.qh0) + M.eb : nullptr;
   for (uint32_t x = part * blockDim.x + threadIdx.x; x < cnt; x += per * blockDim.x) {
     uint2 hq;
     qd[x] = edge_desc(U, M.eb + (uint32_t)(q[x] & kEidMask), &hq);
@@ -2971,14 +2833,14 @@ __global__ void k_shift_u32(uint32_t* __restrict__ dst, const uint32_t* __restri
     dst[i] = src[i] + add;
 }
 
-// row pairs (id | edge id << 32): id + id_add, edge id + eid_add (self-loops keep kInvalid)
+// row pairs (name | edge id << 32): name + name_add, edge id + eid_add (self-loops keep kInvalid)
 __global__ void k_shift_pairs(unsigned long long* __restrict__ dst, const unsigned long long* __restrict__ src,
-                              unsigned long long count, uint32_t id_add, uint32_t eid_add) {
+                              unsigned long long count, uint32_t name_add, uint32_t eid_add) {
   for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < count;
        i += (unsigned long long)gridDim.x * blockDim.x) {
     const unsigned long long pr = src[i];
-    const uint32_t id = (uint32_t)pr + id_add, e = (uint32_t)(pr >> 32);
-    dst[i] = make_pair(id, e == kInvalid ? kInvalid : e + eid_add);
+    const uint32_t name = (uint32_t)pr + name_add, e = (uint32_t)(pr >> 32);
+    dst[i] = make_pair(name, e == kInvalid ? kInvalid : e + eid_add);
   }
 }
 
@@ -3037,30 +2899,18 @@ __global__ void k_replan(const Member* __restrict__ mem, const MemberState* __re
   }
 }
 
-// Hash tables per row (see hash_log2cap): the rows of at least `min_len`
-// entries (the peel: original rows without a hub map; the support pass:
-// oriented out-lists) get an open-addressed table of 2^(1+ceil(log2 d)) 8-byte
-// entries at 4 * the row's start in `pool`.  A warp reads the lengths of 32
-// consecutive rows at once and builds each qualifying row's table in turn in
-// its own slice of shared memory (cleared, filled by compare-and-swap, then
-// stored coalesced).  Rows whose table is larger than the slice are listed
-// for k_table_fill_big, a block per row, which builds them in place: one warp
-// issuing a long row's global compare-and-swaps one round trip at a time took
-// milliseconds on R-MAT's largest non-hub rows.  Every table is written whole,
-// so the pool needs no clearing beforehand; entries outside the tables are
-// never read.
+// Hash tables per oriented list (see hash_log2cap; a tuned option of the support
+// pass): the lists of at least `min_len` entries get an open-addressed table of
+// 2^(1+ceil(log2 d)) 8-byte entries at 4 * the list's start in `pool`.  A warp
+// reads the lengths of 32 consecutive lists at once and builds each qualifying
+// table in turn in its own slice of shared memory (cleared, filled by
+// compare-and-swap, then stored coalesced).  Lists whose table is larger than
+// the slice are listed for k_table_fill_big, a block per list, which builds them
+// in place.  Every table is written whole, so the pool needs no clearing
+// beforehand; entries outside the tables are never read.
 constexpr uint32_t kTableSmem = 1024;  // entries per warp (8 KB)
 constexpr int kTableWarps = 4;
 
-// peel: (column id | edge id << 32) from the original rows; self-loop slots
-// (edge id kInvalid) stay out
-struct RowPairSource {
-  const unsigned long long* row0;
-  __device__ __forceinline__ unsigned long long operator()(uint32_t s) const {
-    const unsigned long long pr = __ldg(row0 + s);
-    return (uint32_t)(pr >> 32) == kInvalid ? ~0ull : pr;
-  }
-};
 // support: (name | position << 32) from the oriented out-lists
 struct OutListSource {
   const uint32_t* oname;
@@ -3072,7 +2922,6 @@ struct OutListSource {
 template <class Source>
 __global__ void __launch_bounds__(kTableWarps * 32) k_table_fill(const uint32_t* __restrict__ off, uint32_t n,
                                                                   uint32_t min_len,
-                                                                  const uint32_t* __restrict__ hub_slot,
                                                                   Source src, unsigned long long* __restrict__ pool,
                                                                   uint32_t* __restrict__ big, uint32_t* big_count) {
   __shared__ unsigned long long s_tab[kTableWarps][kTableSmem];
@@ -3087,7 +2936,7 @@ __global__ void __launch_bounds__(kTableWarps * 32) k_table_fill(const uint32_t*
     if (u < n) {
       b = __ldg(off + u);
       d = __ldg(off + u + 1) - b;
-      want = d >= min_len && !(hub_slot && __ldg(hub_slot + u) != kInvalid);
+      want = d >= min_len;
     }
     const bool large = want && hash_log2cap(d) > 31 - __clz(kTableSmem);
     if (large) big[atomicAdd(big_count, 1u)] = (uint32_t)u;

@@ -67,12 +67,12 @@ int status_from_flags(uint32_t f) {
 // on the graph's degree distribution (filled by the autotuner, sparx_autotune;
 // defaults otherwise).  None of them changes a result, only the time.
 struct Tuning {
-  uint32_t merge_ratio = 8;        // peel: merge the rows when the longer is <= ratio x the shorter
-  uint32_t hub_min_degree = 1024;  // dense hub maps for vertices of at least this degree (0: none)
+  uint32_t merge_ratio = 8;        // read and kept, no effect (rows are no longer merged)
+  uint32_t hub_min_degree = 1024;  // hub maps (the finer rank index) for vertices of at least this degree (0: none)
   uint32_t sample_min = 64;        // support: longer out-lists from this length are searched through a rank index
   uint32_t support_kernel = 1;     // 1 balanced edge form, 2 vertex form
   uint32_t compact_pct = 85;       // rebuild the peel's rows when live entries fill <= this % of them
-  uint32_t hash_min_degree = 128;  // rows of at least this degree get a hash table for the per-lane search (0: none)
+  uint32_t hash_min_degree = 128;  // rows of a quarter of this many entries have a rank index (0: hubs only)
   uint32_t sup_hash_min = 0;       // support: out-lists of at least this length are probed in a hash table (0: none)
   uint32_t relabel = 0;            // rebuild the CSR on degree-ordered vertex ids first (0/1)
 };
@@ -189,10 +189,10 @@ struct Counters {  // device scalars
   uint32_t vcursor;      // vertex-form support: next light vertex batch
   uint32_t hcursor;      //                      next heavy vertex
   uint32_t heavy_count;  //                      heavy vertices listed
-  uint32_t hub_count;    // hub maps assigned
+  uint32_t hub_count;    // rows given the finer rank index
   uint32_t big_count;    // rows compacted by a block each
   uint32_t fin_err;      // served unions: error flags of one member's finalize
-  uint32_t table_big;    // hash tables: rows listed for the block-per-row fill
+  uint32_t table_big;    // rank index, hash tables: what is listed for whole blocks
   double cc_possible;    // clustering: sum of d(d - 1)/2 over vertices
   double cc_local;       //             sum of local coefficients
   unsigned long long cc_slots;  //      sum of slot supports
@@ -203,31 +203,15 @@ struct Counters {  // device scalars
 struct Layout {
   size_t off, nbr, row0, dplus, opos, ocol, osrc, es, act0, act1, q0, q1, qd0, qd1, out, stage0, stage1;
   size_t offA, offB, rowA, rowB;  // compaction ping-pong buffers (0 when compaction is off)
-  size_t vinfo;                   // per vertex: what its row offers as a longer row (hub map / hash table)
+  size_t vinfo;                   // per vertex: its list's or row's rank index header
   size_t alive;                   // compaction: one bit per edge, set while it is unprocessed
   size_t big;                     // compaction: rows longer than kWarpRow (a block each)
-  size_t hub_slot, hub_vertex, hub_base, hub_hist, hub_map;  // hub maps (hub_cap == 0: none)
-  uint32_t hub_cap;
-  unsigned long long hub_pool;    // map entries reserved for all hubs together
+  size_t hub_hist;                // the degree signature's histogram
   size_t tiles, ctl, mem, st, wpref, cnt, mem_tri, mem_maxsup, uni;
   size_t total;
 };
 
-// Hub maps: at most kHubMaxCount maps, each of its member's vertex count in
-// u32 entries, within kHubBudgetBytes, for vertices of degree >= the tuned
-// floor (never below kHubFloor, so never more than W / kHubFloor of them).
-constexpr uint64_t kHubBudgetBytes = 4ull << 30;
-constexpr uint32_t kHubFloor = 256;
-constexpr uint32_t kHubMaxCount = 1024;
-
-// maps reserved for a union whose largest member has `max_n` vertices
-uint32_t hub_capacity(uint64_t max_n, uint64_t W) {
-  if (max_n == 0 || W >= (1ull << 31)) return 0;
-  const uint64_t k = std::min<uint64_t>({kHubMaxCount, W / kHubFloor, kHubBudgetBytes / (4 * max_n)});
-  return (uint32_t)k;
-}
-
-Layout make_layout(uint64_t N, uint64_t W, uint32_t G, bool own_nbr, size_t out_bytes, uint64_t max_n = 0) {
+Layout make_layout(uint64_t N, uint64_t W, uint32_t G, bool own_nbr, size_t out_bytes) {
   Layout L{};
   size_t p = 0;
   auto take = [&](size_t bytes) {
@@ -257,17 +241,8 @@ Layout make_layout(uint64_t N, uint64_t W, uint32_t G, bool own_nbr, size_t out_
   L.rowB = take(8 * W);
   L.alive = take(4 * ((M + 31) / 32));
   L.big = take(4 * (W / kWarpRow + 1));
-  if (max_n == 0) max_n = N;
-  L.hub_cap = hub_capacity(max_n, W);
-  L.hub_hist = take(4 * 34 + 8 * 34);  // vertices, then slots, per log2 degree (always: the tuning key)
-  L.vinfo = take(8ull * N);              // per vertex: its row's hub map or hash table (k_vinfo)
-  if (L.hub_cap) {
-    L.hub_pool = std::min<unsigned long long>(4ull * L.hub_cap * max_n, kHubBudgetBytes) / 4;
-    L.hub_slot = take(4 * N);
-    L.hub_vertex = take(4ull * L.hub_cap);
-    L.hub_base = take(4ull * L.hub_cap);
-    L.hub_map = take(4ull * L.hub_pool);
-  }
+  L.hub_hist = take(4 * 34 + 8 * 34);  // vertices, then slots, per log2 degree (the tuning key)
+  L.vinfo = take(8ull * N);
   L.stage0 = take(kStageBytes);
   L.stage1 = take(kStageBytes);
   const uint64_t tiles = (std::max<uint64_t>(N + 1, M + 1) + kScanTile - 1) / kScanTile + 2;
@@ -283,6 +258,8 @@ Layout make_layout(uint64_t N, uint64_t W, uint32_t G, bool own_nbr, size_t out_
   L.total = p;
   return L;
 }
+
+constexpr uint32_t kHubFloor = 256;  // least degree of a hub (the finer rank index)
 
 struct PeelGraph {
   cudaGraphExec_t exec = nullptr;
@@ -306,7 +283,7 @@ struct Engine {
   int wave_blocks_multi = 0;  // k_wave<true> grid (multigraphs)
   char* ws2 = nullptr;        // multigraph rows, multiplicities and slot map (allocated on first use)
   size_t ws2_cap = 0;
-  char* ws3 = nullptr;        // row hash tables and their queue descriptors (allocated on first use)
+  char* ws3 = nullptr;        // rank index of the working rows and the queues' headers (allocated on first use)
   size_t ws3_cap = 0;
   ulonglong4* trace = nullptr;  // wave trace records (SPARX_TRACE_FILE set)
   std::mutex mu;
@@ -388,7 +365,7 @@ int ensure_ws3(Engine& E, size_t bytes) {
   cudaError_t e = cudaMalloc(&E.ws3, bytes);
   if (e != cudaSuccess) {
     cudaGetLastError();
-    set_error(std::string("hash table workspace of ") + std::to_string(bytes) + " bytes: " + cudaGetErrorString(e));
+    set_error(std::string("rank index workspace of ") + std::to_string(bytes) + " bytes: " + cudaGetErrorString(e));
     E.ws3 = nullptr;
     return SPARX_E_OOM;
   }
@@ -526,7 +503,7 @@ struct SupportIndex {
   const uint32_t* oname = nullptr;
   unsigned long long* hdr = nullptr;   // one per vertex
   unsigned long long* pool = nullptr;  // (m + 1) / 2 words
-  uint32_t* big = nullptr;             // lists longer than kWarpRow
+  uint2* chunks = nullptr;             // long lists' chunks, rank_chunks_max(m) at most
   uint32_t rank_min = Tuning{}.sample_min;
 };
 
@@ -555,8 +532,10 @@ int launch_support(int sm_count, uint32_t support_kernel, uint32_t n, uint64_t m
   if (X.hdr) {
     CU(cudaMemsetAsync(&cnt->table_big, 0, 4, s));
     k_rank_index<uint32_t><<<grid_for(n, 256, sm_count * 16), 256, 0, s>>>(opos, n, X.rank_min, X.oname, X.pool,
-                                                                           X.hdr, X.big, &cnt->table_big);
-    k_rank_index_big<uint32_t><<<sm_count * 4, 256, 0, s>>>(opos, X.oname, X.pool, X.hdr, X.big, &cnt->table_big);
+                                                                           X.hdr, X.chunks, &cnt->table_big, nullptr, 0,
+                                                                           nullptr);
+    k_rank_index_chunks<uint32_t><<<sm_count * 8, 256, 0, s>>>(opos, X.oname, X.pool, X.hdr, X.chunks,
+                                                               &cnt->table_big);
     *launches += 2;
   }
   exclusive_scan<unsigned long long>(SupportWork{opos, osrc, ocol}, m, spref, tiles, &cnt->grand, s);
@@ -642,7 +621,7 @@ struct UnionJob {
   bool prep_only = false;        // stop after the support pass (members about to join a served union)
   const uint32_t* smap = nullptr;  // multigraphs: caller slot -> deduplicated slot (device)
   uint64_t budget = 0;             // device bytes the launch may hold (batched and served unions); 0: no bound
-  bool hook_hash = false;          // served union that takes no joins: row hash tables allowed
+  bool hook_hash = false;          // served union that takes no joins: rank index allowed
   uint64_t prep_m = 0, prep_Ws = 0;  // prep_only: edges and slots prepared
   std::vector<Member> members;  // vb, n, sb, w set; eb, m filled by the pipeline
   Layout L{};
@@ -668,7 +647,7 @@ struct UnionJob {
   float ms_orient = 0, ms_support = 0, ms_peel = 0, ms_finalize = 0;
   uint32_t launches = 0;
   unsigned long long support_elements = 0;
-  uint32_t hubs = 0;  // hub maps built
+  uint32_t hubs = 0;  // rows given the finer rank index
   Tuning tuning;      // the knobs this launch used
   Control ctl{};
 };
@@ -687,18 +666,10 @@ PeelArrays peel_arrays(const Union& U) {
   a.q1 = U.q[1];
   a.qd0 = U.qd[0];
   a.qd1 = U.qd[1];
-  a.hub_slot = U.hub_slot;
-  a.hub_map = U.hub_map;
-  a.hub_base = U.hub_base;
   a.mu = nullptr;
-  a.hpool = U.hpool;
-  a.off0 = U.off0;
+  a.rpool = U.rpool;
   a.qh0 = U.qh[0];
   a.qh1 = U.qh[1];
-  a.n = U.n;
-  a.merge_ratio = Tuning{}.merge_ratio;
-  a.hash_min = U.hash_min;
-  a.pad = 0;
   return a;
 }
 
@@ -876,8 +847,7 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
     if (*herr) { J.err = *herr; return status_from_flags(*herr); }
   }
   // -- orientation (Kernel B) --
-  const bool hubs_possible = L.hub_cap > 0 && !J.support_only;
-  uint32_t* hub_hist = at<uint32_t>(E, L.hub_hist);  // degree signature (tuning key) and hub choice
+  uint32_t* hub_hist = at<uint32_t>(E, L.hub_hist);  // degree signature (tuning key)
   unsigned long long* hub_hist_slots = reinterpret_cast<unsigned long long*>(hub_hist + 34);
   uint32_t* big = at<uint32_t>(E, L.big);
   // multigraphs: deduplicated rows, copies per slot, caller slot -> slot and
@@ -974,7 +944,7 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
     X.oname = at<uint32_t>(E, L.act1);
     X.hdr = at<unsigned long long>(E, L.vinfo);
     X.pool = at<unsigned long long>(E, L.qd0);
-    X.big = at<uint32_t>(E, L.act0);
+    X.chunks = at<uint2>(E, L.act0);
   }
   {
     uint32_t* owner = at<uint32_t>(E, L.q0);  // in-slot owners; the q buffers are idle until the peel
@@ -993,89 +963,51 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
     }
   }
   J.launches += 2;
-  // hub maps: the smallest power-of-two degree bound (>= kHubMinDegree) whose
-  // vertices fit the reserved maps; hist[b] counts degrees in [2^(b-1), 2^b)
-  uint32_t hubs = 0, hub_min_deg = 0;
-  if (hubs_possible && T.hub_min_degree) {
-    uint64_t above = 0;
-    const uint64_t floor_deg = std::max<uint32_t>(T.hub_min_degree, kHubFloor);
-    for (int b = 32; b >= 1; --b) {
-      const uint64_t lo = 1ull << (b - 1);
-      if (lo < floor_deg || above + hist[b] > L.hub_cap) break;
-      above += hist[b];
-      hub_min_deg = (uint32_t)lo;
-    }
-    hubs = (uint32_t)above;
-  }
-  const uint32_t* d_hub_slot = nullptr;
-  const uint32_t* d_hub_map = nullptr;
-  const uint32_t* d_hub_base = nullptr;
-  if (hubs) {
-    uint32_t* hslot = at<uint32_t>(E, L.hub_slot);
-    uint32_t* hvert = at<uint32_t>(E, L.hub_vertex);
-    uint32_t* hbase = at<uint32_t>(E, L.hub_base);
-    uint32_t* hmap = at<uint32_t>(E, L.hub_map);
-    uint64_t max_n = 0;
-    for (const Member& M : J.members) max_n = std::max<uint64_t>(max_n, M.n);
-    CU(cudaMemsetAsync(&cnt->hub_count, 0, 4, s));
-    k_hub_assign<<<grid_for(N, 256, E.sm_count * 8), 256, 0, s>>>(J.off, N, hub_min_deg, hubs, hslot, hvert,
-                                                                  &cnt->hub_count);
-    k_hub_layout<<<1, 1024, 0, s>>>(hvert, hubs, dmem, G, L.hub_pool, hbase, hslot);
-    CU(cudaMemsetAsync(hmap, 0xFF, 4ull * std::min<unsigned long long>(L.hub_pool, hubs * max_n), s));
-    k_hub_fill<<<std::min<uint32_t>(hubs, E.sm_count * 8), 256, 0, s>>>(J.off, row0, hvert, hubs, hslot, hbase,
-                                                                        hmap);
-    J.launches += 3;
-    d_hub_slot = hslot;
-    d_hub_map = hmap;
-    d_hub_base = hbase;
-  }
-  J.hubs = hubs;
-  // row hash tables for the peel's per-lane search (tuned; in a served union
-  // only when it takes no joins, since joining rows would have none) and
-  // out-list hash tables for the support pass (tuned)
-  unsigned long long* hpool = nullptr;
+  // the peel's rank index of the working rows (in a served union only when it
+  // takes no joins, since joining rows would have none) and, as a tuned option,
+  // hash tables of the support pass's out-lists.  Both are optional: when their
+  // workspace does not fit the launch's budget or cannot be allocated, the
+  // launch runs without them (same results).
+  unsigned long long* rpool = nullptr;
   unsigned long long* spool = nullptr;
   uint2* qh0 = nullptr;
   uint2* qh1 = nullptr;
-  uint32_t hash_min = 0, sup_hash_min = 0;
-  // Both are optional: when their workspace does not fit the launch's budget
-  // or cannot be allocated, the launch runs without them (same results).
+  uint2* index_chunks = nullptr;
+  const uint32_t fine_min = T.hub_min_degree ? std::max<uint32_t>(T.hub_min_degree, kHubFloor) : 0;
+  const uint32_t rank_min = T.hash_min_degree ? std::max<uint32_t>(T.hash_min_degree / 4, 8) : kInvalid;
+  uint32_t sup_hash_min = 0;
   {
-    bool peel_hash = T.hash_min_degree && !J.support_only && !J.prep_only && (!J.hook || J.hook_hash) &&
-                     Ws < (1ull << 30) && Ws;
+    uint32_t dmax_log = 0;  // largest degree < 2^dmax_log
+    for (uint32_t b = 1; b <= 32; ++b)
+      if (hist[b]) dmax_log = b;
+    const bool any_row = dmax_log >= 32 || (1ull << dmax_log) > std::min(rank_min, fine_min ? fine_min : kInvalid);
+    bool index = any_row && !J.support_only && !J.prep_only && (!J.hook || J.hook_hash) && Ws < (1ull << 30) && Ws;
     bool sup_hash = T.sup_hash_min && m > 0 && m < (1ull << 28);
     const uint64_t Mx = std::max<uint64_t>(W / 2, 1);
-    size_t pool_b = peel_hash ? align_up(32ull * Ws) : 0, qh_b = peel_hash ? align_up(8ull * Mx) : 0;
+    size_t pool_b = index ? align_up(8ull * Ws) : 0, qh_b = index ? align_up(8ull * Mx) : 0;
     size_t spool_b = sup_hash ? align_up(32ull * m) : 0;
-    // rows with tables past a warp's shared slice (more than kTableSmem / 2
-    // entries) are listed for the block-per-row fill: at most W / 512 rows
-    const size_t big_b = align_up(4ull * (W / (kTableSmem / 2) + 2));
-    if ((peel_hash || sup_hash) &&
-        ((J.budget && L.total + pool_b + 2 * qh_b + spool_b + big_b > J.budget) ||
-         ensure_ws3(E, pool_b + 2 * qh_b + spool_b + big_b) != SPARX_OK)) {
-      peel_hash = sup_hash = false;
+    // long rows' chunks, and lists with tables past a warp's shared slice (more
+    // than kTableSmem / 2 entries: fewer of them)
+    const size_t big_b = align_up(sizeof(uint2) * rank_chunks_max(W));
+    if ((index || sup_hash) && ((J.budget && L.total + pool_b + 2 * qh_b + spool_b + big_b > J.budget) ||
+                                ensure_ws3(E, pool_b + 2 * qh_b + spool_b + big_b) != SPARX_OK)) {
+      index = sup_hash = false;
       pool_b = qh_b = spool_b = 0;
     }
     uint32_t* big_list = (uint32_t*)(E.ws3 + pool_b + 2 * qh_b + spool_b);
-    uint32_t* big_count = &cnt->table_big;
-    if (peel_hash) {
-      hpool = (unsigned long long*)E.ws3;
+    if (index) {
+      rpool = (unsigned long long*)E.ws3;
       qh0 = (uint2*)(E.ws3 + pool_b);
       qh1 = (uint2*)(E.ws3 + pool_b + qh_b);
-      hash_min = T.hash_min_degree;
-      CU(cudaMemsetAsync(big_count, 0, 4, s));
-      k_table_fill<<<grid_for(N, kTableWarps * 32, E.sm_count * 16), kTableWarps * 32, 0, s>>>(
-          J.off, N, hash_min, d_hub_slot, RowPairSource{row0}, hpool, big_list, big_count);
-      k_table_fill_big<<<E.sm_count * 8, 256, 0, s>>>(J.off, big_list, big_count, RowPairSource{row0}, hpool);
-      J.launches += 2;
+      index_chunks = (uint2*)big_list;
     }
     if (sup_hash) {
       spool = (unsigned long long*)(E.ws3 + pool_b + 2 * qh_b);
       sup_hash_min = T.sup_hash_min;
-      CU(cudaMemsetAsync(big_count, 0, 4, s));
+      CU(cudaMemsetAsync(&cnt->table_big, 0, 4, s));
       k_table_fill<<<grid_for(N, kTableWarps * 32, E.sm_count * 16), kTableWarps * 32, 0, s>>>(
-          opos, N, sup_hash_min, nullptr, OutListSource{X.oname}, spool, big_list, big_count);
-      k_table_fill_big<<<E.sm_count * 8, 256, 0, s>>>(opos, big_list, big_count, OutListSource{X.oname}, spool);
+          opos, N, sup_hash_min, OutListSource{X.oname}, spool, big_list, &cnt->table_big);
+      k_table_fill_big<<<E.sm_count * 8, 256, 0, s>>>(opos, big_list, &cnt->table_big, OutListSource{X.oname}, spool);
       J.launches += 2;
     }
   }
@@ -1125,20 +1057,24 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
     U.q[1] = at<unsigned long long>(E, L.q1);
     U.qd[0] = at<uint4>(E, L.qd0);
     U.qd[1] = at<uint4>(E, L.qd1);
-    U.hub_slot = d_hub_slot;
-    U.hub_map = d_hub_map;
-    U.hub_base = d_hub_base;
-    U.hpool = hpool;
-    U.off0 = J.off;
+    U.rpool = rpool;
     U.qh[0] = qh0;
     U.qh[1] = qh1;
-    U.hash_min = hash_min;
     U.vinfo = nullptr;
-    if (d_hub_slot || hash_min) {
+    auto index_rows = [&](const uint32_t* roff, const unsigned long long* rows, uint32_t* fine_count) -> int {
       unsigned long long* vinfo = at<unsigned long long>(E, L.vinfo);
-      k_vinfo<<<grid_for(N, 256, E.sm_count * 16), 256, 0, s>>>(N, d_hub_slot, d_hub_base, J.off, hash_min, vinfo);
-      J.launches += 1;
-      U.vinfo = vinfo;
+      CU(cudaMemsetAsync(&cnt->table_big, 0, 4, s));
+      k_rank_index<unsigned long long><<<grid_for(N, 256, E.sm_count * 16), 256, 0, s>>>(
+          roff, N, rank_min, rows, rpool, vinfo, index_chunks, &cnt->table_big, J.off, fine_min, fine_count);
+      k_rank_index_chunks<unsigned long long><<<E.sm_count * 8, 256, 0, s>>>(roff, rows, rpool, vinfo, index_chunks,
+                                                                             &cnt->table_big);
+      J.launches += 2;
+      return SPARX_OK;
+    };
+    if (rpool) {
+      U.vinfo = at<unsigned long long>(E, L.vinfo);
+      const int rc = index_rows(J.off, row0, &cnt->hub_count);
+      if (rc) return rc;
     }
     U.n = N;
     U.m = (uint32_t)m;
@@ -1180,8 +1116,6 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
     wa.Up = at<Union>(E, L.uni);
     wa.arr = peel_arrays(U);
     wa.arr.mu = mu;
-    wa.arr.merge_ratio = T.merge_ratio;
-    if (J.hook) wa.arr.n = 0;  // unused by the kernels; a constant keeps the graph across joins
     wa.mem = dmem;
     wa.st = at<MemberState>(E, L.st);
     wa.ctl = at<Control>(E, L.ctl);
@@ -1262,6 +1196,10 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
       k_compact_fill_big<<<E.sm_count * 2, 1024, 0, s>>>(cur_off, cur_row, alive, off2, row2, big,
                                                          &cnt->big_count);
       k_compact_commit<<<1, 1, 0, s>>>(at<Union>(E, L.uni), off2, row2, off2 + pN, wa.ctl);
+      if (rpool) {
+        const int rc = index_rows(off2, row2, nullptr);
+        if (rc) return rc;
+      }
       const uint32_t per = std::max<uint32_t>(1, (uint32_t)(E.sm_count * 8) / std::max<uint32_t>(pG, 1));
       k_refresh_desc<<<pG * per, 256, 0, s>>>(wa.Up, dmem, wa.st, pG, per);
       J.launches += 8;
@@ -1306,6 +1244,7 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
   CU(cudaMemcpyAsync(&hc, cnt, sizeof(Counters), cudaMemcpyDeviceToHost, s));
   CU(cudaStreamSynchronize(s));
   J.tri = hc.tri;
+  J.hubs = hc.hub_count;
   J.kmax = hc.kmax;
   J.cc_possible = hc.cc_possible;
   J.cc_local = hc.cc_local;
@@ -1371,7 +1310,6 @@ void fill_stats(const UnionJob& J, uint32_t g, sparx_pkt_stats* st) {
     st->hub_maps = J.hubs;
     st->merge_iters = J.ctl.merge_iters;
     st->lane_iters = J.ctl.lane_iters;
-    st->merge_chunks = J.ctl.merge_chunks;
   }
   st->ms_orient = J.ms_orient;
   st->ms_support = J.ms_support;
@@ -1768,17 +1706,16 @@ int run_batch_union(Engine& E, std::vector<HostMember>& hm, const Opts& O, int* 
   const size_t G = hm.size();
   UnionJob J;
   J.budget = budget;
-  uint64_t N = 0, Wt = 0, max_n = 0;
+  uint64_t N = 0, Wt = 0;
   for (const HostMember& h : hm) {
     J.members.push_back(Member{(uint32_t)N, (uint32_t)h.n, (uint32_t)Wt, (uint32_t)h.w, 0, 0});
     N += h.n;
     Wt += h.w;
-    max_n = std::max<uint64_t>(max_n, h.n);
   }
   J.N = N;
   J.W = Wt;
   const size_t out_bytes = (O.out_bits / 8) * Wt;
-  J.L = make_layout(N, Wt, (uint32_t)G, true, out_bytes, max_n);
+  J.L = make_layout(N, Wt, (uint32_t)G, true, out_bytes);
   int rc = ensure_ws(E, J.L.total);
   auto fail_all = [&](int code) {
     for (size_t g = 0; g < G; ++g) {
@@ -1832,16 +1769,16 @@ int run_batch_union(Engine& E, std::vector<HostMember>& hm, const Opts& O, int* 
   return SPARX_OK;
 }
 
-// workspace of the peel's row hash tables for W slots (run_union's pool, the
-// two queue descriptor arrays and the list of rows built a block each), and
-// of the relabelled copy of N vertices' rows (relabel_graph, bounded above)
+// workspace of the peel's rank index for W slots (run_union's pool, the two
+// queue header arrays and the list of rows indexed by blocks), and of the
+// relabelled copy of N vertices' rows (relabel_graph, bounded above)
 size_t table_bytes(uint64_t W) {
-  return align_up(32ull * W) + 2 * align_up(8ull * std::max<uint64_t>(W / 2, 1)) +
-         align_up(4ull * (W / (kTableSmem / 2) + 2));
+  return align_up(8ull * W) + 2 * align_up(8ull * std::max<uint64_t>(W / 2, 1)) +
+         align_up(sizeof(uint2) * rank_chunks_max(W));
 }
 size_t relabel_bytes(uint64_t N, uint64_t W) { return 8 * W + 30 * N + (64ull << 20); }
 #ifndef SPARX_BATCH_FOR_TABLES
-#define SPARX_BATCH_FOR_TABLES 1  // size batched unions so the row hash tables fit
+#define SPARX_BATCH_FOR_TABLES 1  // size batched unions so the rank index fits
 #endif
 constexpr bool kBatchForTables = SPARX_BATCH_FOR_TABLES;
 
@@ -1891,14 +1828,14 @@ int run_batch(const sparx_graph_view* graphs, uint64_t count, uint64_t budget, c
   size_t at_i = 0;
   while (at_i < valid.size()) {
     std::vector<HostMember> wave;
-    uint64_t N = 0, Wt = 0, max_n = 0;
+    uint64_t N = 0, Wt = 0;
     while (at_i < valid.size()) {
       const HostMember& h = valid[at_i];
-      const uint64_t N2 = N + h.n, W2 = Wt + h.w, mx2 = std::max<uint64_t>(max_n, h.n);
+      const uint64_t N2 = N + h.n, W2 = Wt + h.w;
       const size_t bytes =
-          make_layout(N2, W2, (uint32_t)wave.size() + 1, true, (O.out_bits / 8) * W2, mx2).total;
+          make_layout(N2, W2, (uint32_t)wave.size() + 1, true, (O.out_bits / 8) * W2).total;
       const bool fits = N2 < 0xFFFFFFFFull && W2 < 0xFFFFFFFFull && bytes <= budget && wave.size() < 65536;
-      // a union grows only while its row hash tables fit as well (below 2^30
+      // a union grows only while its rank index fits as well (below 2^30
       // slots, and within the budget with them): on the mix the tables take
       // more off the peel than the extra unions' waves cost.  A graph too large
       // for that still runs, alone, without them.
@@ -1915,7 +1852,6 @@ int run_batch(const sparx_graph_view* graphs, uint64_t count, uint64_t budget, c
       wave.push_back(h);
       N = N2;
       Wt = W2;
-      max_n = mx2;
       ++at_i;
     }
     if (!wave.empty()) run_batch_union(E, wave, O, status_out, stats_out, &first_fail, budget);
@@ -2011,8 +1947,8 @@ void server_finish(sparx_server* S, ServerReq* r, int status) {
 
 uint64_t prep_budget(uint64_t lane_budget) { return lane_budget / 5; }
 
-bool layout_fits(uint64_t N, uint64_t W, uint32_t G, size_t esz, uint64_t max_n, uint64_t budget) {
-  return N < 0xFFFFFFFFull && W < 0xFFFFFFFFull && make_layout(N, W, G, true, esz * W, max_n).total <= budget;
+bool layout_fits(uint64_t N, uint64_t W, uint32_t G, size_t esz, uint64_t budget) {
+  return N < 0xFFFFFFFFull && W < 0xFFFFFFFFull && make_layout(N, W, G, true, esz * W).total <= budget;
 }
 
 // The lane's hook: delivers members as they finish and joins waiting requests.
@@ -2023,7 +1959,6 @@ struct LaneHook : ServeHook {
   std::vector<ServerReq*> reqs;     // per member of the union
   std::vector<char> delivered;
   uint64_t N_cap = 0, W_cap = 0;    // the union's room
-  uint64_t max_n0 = 0;              // largest initial member (the hub pool was sized for it)
   uint64_t max_member_w = 0;        // slots of the union's largest member
   // the union's wave pace, measured between stops (host work at a stop excluded)
   std::chrono::steady_clock::time_point t_mark{};
@@ -2110,17 +2045,17 @@ struct LaneHook : ServeHook {
       const uint64_t mine = S->lane_budget[lane] - prep_budget(S->lane_budget[lane]);
       if (other > 0 && mine > other)
         for (const ServerReq* r : S->queue)
-          if (!layout_fits(r->h.n, r->h.w, kServeMaxMembers, 4, r->h.n, other) &&
-              layout_fits(r->h.n, r->h.w, kServeMaxMembers, 4, r->h.n, mine))
+          if (!layout_fits(r->h.n, r->h.w, kServeMaxMembers, 4, other) &&
+              layout_fits(r->h.n, r->h.w, kServeMaxMembers, 4, mine))
             return SPARX_OK;
-      uint64_t N = ctx.N, W = ctx.Ws, pn = 0, pw = 0, pmax = 0;
+      uint64_t N = ctx.N, W = ctx.Ws, pn = 0, pw = 0;
       uint32_t G = ctx.G;
       for (auto it = S->queue.begin(); it != S->queue.end();) {
         ServerReq* r = *it;
         const uint64_t n2 = N + r->h.n, w2 = W + r->h.w;
         const bool fits = !r->fresh_only && G + 1 <= kServeMaxMembers && n2 <= N_cap && w2 <= W_cap &&
                           layout_fits(pn + r->h.n, pw + r->h.w, (uint32_t)take.size() + 1, 4,
-                                      std::max<uint64_t>(pmax, r->h.n), prep_budget(S->lane_budget[lane]));
+                                      prep_budget(S->lane_budget[lane]));
         if (!fits) { ++it; continue; }
         it = S->queue.erase(it);
         r->running = true;
@@ -2130,7 +2065,6 @@ struct LaneHook : ServeHook {
         W = w2;
         pn += r->h.n;
         pw += r->h.w;
-        pmax = std::max<uint64_t>(pmax, r->h.n);
         ++G;
       }
     }
@@ -2185,18 +2119,16 @@ struct LaneHook : ServeHook {
   int join_group(Engine& E, UnionJob& J, PeelCtx& ctx, cudaStream_t s, std::vector<HostMember>& hm,
                  std::vector<ServerReq*>& ok, uint32_t* joined) {
     UnionJob PJ;
-    uint64_t Np = 0, Wp = 0, maxn = 0;
+    uint64_t Np = 0, Wp = 0;
     for (const HostMember& h : hm) {
       PJ.members.push_back(Member{(uint32_t)Np, (uint32_t)h.n, (uint32_t)Wp, (uint32_t)h.w, 0, 0});
       Np += h.n;
       Wp += h.w;
-      maxn = std::max<uint64_t>(maxn, h.n);
     }
     PJ.N = Np;
     PJ.W = Wp;
     PJ.prep_only = true;
-    PJ.L = make_layout(Np, Wp, (uint32_t)hm.size(), true, 4 * Wp, maxn);
-    PJ.L.hub_cap = 0;  // joining members get no hub maps
+    PJ.L = make_layout(Np, Wp, (uint32_t)hm.size(), true, 4 * Wp);
     int rc = ensure_ws(*P, PJ.L.total, false);
     int prc = rc;
     if (!rc) {
@@ -2222,14 +2154,15 @@ struct LaneHook : ServeHook {
     uint32_t* off = J.off;
     unsigned long long* row0 = at<unsigned long long>(E, L.row0);
     k_shift_u32<<<gridN, 256, 0, s>>>(off + N0, at<uint32_t>(*P, PJ.L.off), Np + 1, (uint32_t)W0);
-    if (Wp) k_shift_pairs<<<gridW, 256, 0, s>>>(row0 + W0, at<unsigned long long>(*P, PJ.L.row0), Wp, N0,
+    if (Wp) k_shift_pairs<<<gridW, 256, 0, s>>>(row0 + W0, at<unsigned long long>(*P, PJ.L.row0), Wp, (uint32_t)W0,
                                                 (uint32_t)m0);
     if (ctx.cur_row != row0) {  // compacted working rows: the new rows go behind their live entries
       k_shift_u32<<<gridN, 256, 0, s>>>((uint32_t*)ctx.cur_off + N0, at<uint32_t>(*P, PJ.L.off), Np + 1,
                                         (uint32_t)ctx.csr_slots);
       if (Wp)
         k_shift_pairs<<<gridW, 256, 0, s>>>((unsigned long long*)ctx.cur_row + ctx.csr_slots,
-                                            at<unsigned long long>(*P, PJ.L.row0), Wp, N0, (uint32_t)m0);
+                                            at<unsigned long long>(*P, PJ.L.row0), Wp, (uint32_t)W0,
+                                            (uint32_t)m0);
     }
     k_shift_u32<<<gridN, 256, 0, s>>>(at<uint32_t>(E, L.opos) + N0, at<uint32_t>(*P, PJ.L.opos), Np + 1,
                                       (uint32_t)m0);
@@ -2238,9 +2171,6 @@ struct LaneHook : ServeHook {
       k_shift_u32<<<gridM, 256, 0, s>>>(at<uint32_t>(E, L.osrc) + m0, at<uint32_t>(*P, PJ.L.osrc), mp, N0);
       CU(cudaMemcpyAsync(at<int2>(E, L.es) + m0, at<int2>(*P, PJ.L.es), 8 * mp, cudaMemcpyDeviceToDevice, s));
     }
-    if (ctx.U.hub_slot && Np) CU(cudaMemsetAsync(at<uint32_t>(E, L.hub_slot) + N0, 0xFF, 4 * Np, s));
-    // joining rows offer neither hub maps nor tables
-    if (ctx.U.vinfo && Np) CU(cudaMemsetAsync(at<unsigned long long>(E, L.vinfo) + N0, 0, 8 * Np, s));
     Counters* cnt = at<Counters>(E, L.cnt);
     if (Np) k_big_rows_range<<<grid_for(Np, 256, E.sm_count * 8), 256, 0, s>>>(off, N0, N0 + (uint32_t)Np,
                                                                                  at<uint32_t>(E, L.big),
@@ -2360,15 +2290,15 @@ void server_worker(sparx_server* S, int lane) {
         continue;
       }
       // FIFO; a request too large for this lane is left for a larger one
-      uint64_t N = 0, W = 0, mx = 0;
+      uint64_t N = 0, W = 0;
       for (auto it = S->queue.begin(); it != S->queue.end() && batch.size() < kServeMaxMembers;) {
         ServerReq* r = *it;
         if (!batch.empty() && r->fresh_only != fresh) { ++it; continue; }
-        const uint64_t N2 = N + r->h.n, W2 = W + r->h.w, mx2 = std::max<uint64_t>(mx, r->h.n);
-        if (!layout_fits(N2, W2, kServeMaxMembers, esz, mx2, main_budget)) {
+        const uint64_t N2 = N + r->h.n, W2 = W + r->h.w;
+        if (!layout_fits(N2, W2, kServeMaxMembers, esz, main_budget)) {
           bool fits_any = false;
           for (uint64_t b : S->lane_budget)
-            fits_any |= layout_fits(r->h.n, r->h.w, kServeMaxMembers, esz, r->h.n, b - prep_budget(b));
+            fits_any |= layout_fits(r->h.n, r->h.w, kServeMaxMembers, esz, b - prep_budget(b));
           if (!fits_any) {  // no lane can ever hold it
             it = S->queue.erase(it);
             server_finish(S, r, SPARX_E_OOM);
@@ -2385,7 +2315,6 @@ void server_worker(sparx_server* S, int lane) {
         batch.push_back(r);
         N = N2;
         W = W2;
-        mx = mx2;
       }
       if (batch.empty()) {
         // nothing fits this lane now: wait for a change
@@ -2420,28 +2349,26 @@ void server_worker(sparx_server* S, int lane) {
     S->cv_done.notify_all();
     if (hm.empty()) continue;
     UnionJob J;
-    uint64_t N = 0, W = 0, mx = 0;
+    uint64_t N = 0, W = 0;
     for (const HostMember& h : hm) {
       J.members.push_back(Member{(uint32_t)N, (uint32_t)h.n, (uint32_t)W, (uint32_t)h.w, 0, 0});
       N += h.n;
       W += h.w;
-      mx = std::max<uint64_t>(mx, h.n);
     }
     for (const HostMember& h : hm) hook.max_member_w = std::max<uint64_t>(hook.max_member_w, h.w);
     // a union holding a member past kJoinMaxMemberSlots never takes joins: it
-    // gets no room for them, and its rows are final, so the row hash tables
+    // gets no room for them, and its rows are final, so the rank index
     // (built once, before the peel) are safe for it within the lane's budget
     const bool no_joins = hook.max_member_w > kJoinMaxMemberSlots;
     // room: the largest extra (slots e, vertices e / 2) the lane's budget holds
     uint64_t extra = 0;
     for (uint64_t step = 1ull << 40; step && !no_joins; step >>= 1) {
       const uint64_t e2 = extra + step;
-      if (W + e2 < (1ull << 31) && layout_fits(N + e2 / 2, W + e2, kServeMaxMembers, esz, mx, main_budget))
+      if (W + e2 < (1ull << 31) && layout_fits(N + e2 / 2, W + e2, kServeMaxMembers, esz, main_budget))
         extra = e2;
     }
     hook.N_cap = N + extra / 2;
     hook.W_cap = W + extra;
-    hook.max_n0 = mx;
     hook.delivered.assign(hook.reqs.size(), 0);
     J.N = N;
     J.W = W;
@@ -2449,7 +2376,7 @@ void server_worker(sparx_server* S, int lane) {
     J.hook_hash = no_joins;
     J.budget = main_budget;
     S->unions += 1;
-    J.L = make_layout(hook.N_cap, hook.W_cap, kServeMaxMembers, true, esz * hook.W_cap, mx);
+    J.L = make_layout(hook.N_cap, hook.W_cap, kServeMaxMembers, true, esz * hook.W_cap);
     int rc = ensure_ws(E, J.L.total, false);
     if (!rc) {
       cudaStream_t s = E.stream;
@@ -2462,7 +2389,7 @@ void server_worker(sparx_server* S, int lane) {
       if (!rc) rc = run_union(E, J, S->O, s);
     }
     if (E.ws3) {
-      // the hash tables of a union without join room leave with it, so the
+      // the rank index of a union without join room leaves with it, so the
       // lane holds no more than its share while its next union runs
       cudaStreamSynchronize(E.stream);
       cudaFree(E.ws3);
@@ -3000,8 +2927,7 @@ namespace {
 
 // Coordinate descent over the knobs, one group at a time from the defaults:
 // the support form and sampling threshold by the support pass's device time,
-// then the hub-map floor (orientation + peel, since the maps are built with
-// the orientation), the merge ratio and the compaction fill by the peel's.
+// then the hub floor and the compaction fill by orientation + peel.
 // `run(t, &ms_support, &ms_rest)` decomposes the sample once with knobs t.
 // The best knobs are stored under the sample's key (and written to the file
 // SPARX_TUNE_FILE names, if any).
@@ -3059,11 +2985,8 @@ int autotune_core(RunF run, uint32_t repeats, Tuning* best_out, TuneKey* key_out
   for (uint32_t h : {0u, 512u, 4096u}) { Tuning t = cur; t.hub_min_degree = h; c2.push_back(t); }
   if ((rc = try_group(c2, false))) return rc;
   std::vector<Tuning> c3;
-  for (uint32_t mr : {4u, 16u}) { Tuning t = cur; t.merge_ratio = mr; c3.push_back(t); }
+  for (uint32_t cp : {75u, 95u}) { Tuning t = cur; t.compact_pct = cp; c3.push_back(t); }
   if ((rc = try_group(c3, false))) return rc;
-  std::vector<Tuning> c4;
-  for (uint32_t cp : {75u, 95u}) { Tuning t = cur; t.compact_pct = cp; c4.push_back(t); }
-  if ((rc = try_group(c4, false))) return rc;
   {
     // the relabelling changes the support pass and the peel (and costs a pass
     // in the orientation): judged on the whole decomposition
@@ -3077,9 +3000,9 @@ int autotune_core(RunF run, uint32_t repeats, Tuning* best_out, TuneKey* key_out
       rest = y;
     }
   }
-  std::vector<Tuning> c5;
-  for (uint32_t hm : {0u, 32u, 512u}) { Tuning t = cur; t.hash_min_degree = hm; c5.push_back(t); }
-  if ((rc = try_group(c5, false))) return rc;
+  std::vector<Tuning> c4;
+  for (uint32_t hm : {0u, 32u, 512u}) { Tuning t = cur; t.hash_min_degree = hm; c4.push_back(t); }
+  if ((rc = try_group(c4, false))) return rc;
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     g_tune[key] = cur;
@@ -3456,7 +3379,7 @@ int run_noalloc(const uint64_t* d_offsets, uint64_t n_plus_1, const uint32_t* d_
     X.oname = (uint32_t*)P(L.act1);
     X.hdr = (unsigned long long*)P(L.qd1);
     X.pool = (unsigned long long*)P(L.qd0);
-    X.big = (uint32_t*)P(L.act0);
+    X.chunks = (uint2*)P(L.act0);
   }
   k_orient_fill<<<vgrid, 256, 0, s>>>(off, d_nbr, N, opos, ocol, osrc, row0, (uint32_t*)P(L.q0), big,
                                       &cnt->big_count, const_cast<uint32_t*>(X.hdr ? X.oname : nullptr));
@@ -3472,7 +3395,7 @@ int run_noalloc(const uint64_t* d_offsets, uint64_t n_plus_1, const uint32_t* d_
     if (rc) return rc;
   }
 
-  Union U{};  // no hub maps in the fixed scratch
+  Union U{};  // no rank index in the fixed scratch
   U.off = off;
   U.row = row0;
   U.opos = opos;
