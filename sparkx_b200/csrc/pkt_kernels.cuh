@@ -1587,6 +1587,7 @@ constexpr int kWaveThreads = 256;
 #define SPARX_WAVE_MINB 7  // resident 256-thread blocks per SM the register budget targets
 #endif
 constexpr int kWaveWarps = kWaveThreads / 32;
+constexpr int kTailThreads = 512;  // threads per block of the small waves' cluster (1024: R-MAT-12 6% slower)
 // slots of the per-warp loop state in shared memory (k_wave)
 enum : int { kCtxJb = 0, kCtxSegEnd = 1, kCtxKend = 2 };
 enum : int { kCtxEb = 0, kCtxM, kCtxLevel, kCtxQsel, kCtxQcount, kCtxSegLen, kCtxG, kCtxW };
@@ -1696,93 +1697,179 @@ struct PlanShared {
   unsigned long long proc, scan, edges, live_edges;
 };
 
+// A member's state after the wave that just ran; returns the next wave's work.
+__device__ __forceinline__ unsigned long long advance_member(MemberState& s, uint32_t m) {
+  const unsigned long long cnt = s.next >> kWorkBits;
+  switch (s.phase) {
+    case kPhaseScan0:
+      s.act_sel ^= 1u;
+      s.act_count = s.kept;
+      s.kept = 0;
+      if (s.processed >= m) s.phase = kPhaseDone;
+      else { s.level = s.min_kept; s.min_kept = 0xFFFFFFFFu; s.phase = kPhaseScan; }
+      break;
+    case kPhaseScan:
+      s.act_sel ^= 1u;
+      s.act_count = s.kept;
+      s.kept = 0;
+      if (cnt) {
+        s.curr = s.next;
+        s.next = 0;
+        s.q_sel ^= 1u;
+        s.phase = kPhaseProc;
+        s.levels++;
+        s.max_level = s.level;
+      } else if (s.act_count == 0) {
+        s.phase = kPhaseDone;
+      } else {
+        s.level = s.min_kept;  // no edge at this level: jump to the next occupied one
+      }
+      s.min_kept = 0xFFFFFFFFu;
+      break;
+    case kPhaseProc:
+      s.processed += (uint32_t)(s.curr >> kWorkBits);
+      if (cnt) {
+        s.curr = s.next;
+        s.next = 0;
+        s.q_sel ^= 1u;
+      } else {
+        s.curr = 0;
+        if (s.processed >= m) s.phase = kPhaseDone;
+        else { s.level += 1; s.phase = kPhaseScan; s.min_kept = 0xFFFFFFFFu; }
+      }
+      break;
+    default:
+      return 0;
+  }
+  if (s.phase != kPhaseDone) s.waves++;
+  return s.phase == kPhaseDone ? 0 : s.phase == kPhaseProc ? s.curr & kWorkMask : s.act_count;
+}
+
+// The loop's side of a planned wave: work counters, the bounds, and whether the
+// loop stops here.  One thread calls it; returns ctl->done.
+struct WavePlan {
+  unsigned long long total, proc, scan, edges, live_edges;
+  uint32_t live, newly_done;
+};
+__device__ __forceinline__ uint32_t plan_commit(Control* ctl, uint32_t* __restrict__ err, const WavePlan& P) {
+  // one round of loads, then one of stores
+  const unsigned long long waves = ctl->waves_run + 1, max_waves = ctl->max_waves, t_start = ctl->t_start,
+                           timeout = ctl->timeout_ns, el_proc = ctl->el_proc, el_scan = ctl->el_scan,
+                           edges = ctl->edges_proc, slots = ctl->csr_slots, compact_min = ctl->compact_min;
+  const uint32_t wave = ctl->wave, pct = ctl->compact_pct, notify = ctl->notify_done;
+  const volatile uint32_t* admit = ctl->admit;
+  ulonglong4* trace = ctl->trace;
+  const uint32_t e = __ldcg(err);
+  if (trace && waves - 1 < ctl->trace_cap) trace[waves - 1] = make_ulonglong4(globaltimer(), P.total, P.proc, P.scan);
+  ctl->el_proc = el_proc + P.proc;
+  ctl->el_scan = el_scan + P.scan;
+  ctl->edges_proc = edges + P.edges;
+  ctl->total_work = P.total;
+  ctl->wave = wave + 1;
+  ctl->waves_run = waves;
+  uint32_t done = 0, reason = kExitNone;
+  if (P.live == 0) { done = 1; reason = kExitDone; }
+  if (e) { done = 1; reason = kExitError; }
+  if (waves > max_waves) { atomicOr(err, kErrWaves); done = 1; reason = kExitError; }
+  if (globaltimer() - t_start > timeout) { atomicOr(err, kErrTimeout); done = 1; reason = kExitError; }
+  // live edges fill at most compact_pct % of the working rows (85 unless
+  // tuned): stop so the host can compact them (a compaction is a few passes
+  // over the rows, which the shorter rows repay at this fill; 78% and 90%
+  // measured slower on R-MAT-22)
+  if (!done && slots >= compact_min && 200 * P.live_edges <= (unsigned long long)pct * slots) {
+    done = 1;
+    reason = kExitCompact;
+  }
+  if (!done && notify && P.newly_done) { done = 1; reason = kExitMember; }
+  if (!done && admit && *admit) { done = 1; reason = kExitAdmit; }
+  ctl->done = done;
+  ctl->exit_reason = reason;
+  return done;
+}
+
 // Planner: one block advances every member's state machine after a wave and
 // lays out the next wave's work; sets the CUDA-graph loop condition.  Runs in
 // the last block of each wave (see k_wave), after every other block's writes.
+// Up to 32 members are planned by one warp: no block scans and no barriers, and
+// the loads go out in one round (a small wave spent 2.0 of its 8.1 us here).
 __device__ __forceinline__ void plan_wave(const Member* __restrict__ mem, MemberState* __restrict__ st,
                                           Control* ctl, unsigned long long* __restrict__ wpref,
                                           uint32_t* __restrict__ err, cudaGraphConditionalHandle handle,
-                                          int use_handle, PlanShared& ps) {
-  unsigned long long* sw = ps.sw;
-  uint32_t& s_live = ps.live;
-  unsigned long long &s_proc = ps.proc, &s_scan = ps.scan, &s_edges = ps.edges, &s_live_edges = ps.live_edges;
-  const uint32_t G = ctl->G;
-  if (threadIdx.x == 0) { s_live = 0; s_proc = 0; s_scan = 0; s_edges = 0; s_live_edges = 0; ps.newly_done = 0; }
-  __syncthreads();
-  const bool was_done = ctl->done;
+                                          int use_handle, PlanShared& ps, uint32_t G, bool was_done) {
   if (was_done) {
     // the loop is stopped (host-launched waves keep coming until the host
     // looks): the planned wave must survive untouched for a resume
     if (threadIdx.x == 0 && use_handle) cudaGraphSetConditional(handle, 0u);
     return;
   }
+  if (G <= 32) {
+    if (threadIdx.x >= 32) return;
+    const uint32_t g = threadIdx.x;
+    MemberState s{};
+    s.phase = kPhaseDone;
+    uint32_t m = 0;
+    if (g < G) {
+      s = load_state_cg(st + g);
+      m = mem[g].m;
+    }
+    const uint32_t before = s.phase;
+    const unsigned long long w = advance_member(s, m);
+    const bool live = s.phase != kPhaseDone, proc = s.phase == kPhaseProc;
+    if (g < G) st[g] = s;
+    WavePlan P{};
+    if (G == 1) {
+      if (g > 0) return;
+      P.total = w;
+      P.proc = proc ? w : 0;
+      P.edges = proc ? s.curr >> kWorkBits : 0;
+      P.live_edges = live ? m - s.processed : 0;
+      P.live = live;
+      P.newly_done = !live && before != kPhaseDone;
+      wpref[0] = 0;
+      wpref[1] = w;
+    } else {
+      const unsigned long long incl = warp_incl_scan(w);
+      if (g < G) wpref[g] = incl - w;
+      P.total = __shfl_sync(kFull, incl, 31);
+      // frontier edges of a union stay below 2^32 (edge ids are 32-bit), live edges too
+      P.edges = __reduce_add_sync(kFull, proc ? (uint32_t)(s.curr >> kWorkBits) : 0u);
+      P.live_edges = __reduce_add_sync(kFull, live ? m - s.processed : 0u);
+      P.live = __popc(__ballot_sync(kFull, live));
+      P.newly_done = __popc(__ballot_sync(kFull, !live && before != kPhaseDone));
+      P.proc = proc ? w : 0;
+#pragma unroll
+      for (int d = 16; d > 0; d >>= 1) P.proc += __shfl_xor_sync(kFull, P.proc, d);
+      if (g > 0) return;
+      wpref[G] = P.total;
+    }
+    P.scan = P.total - P.proc;
+    const uint32_t done = plan_commit(ctl, err, P);
+    if (use_handle) cudaGraphSetConditional(handle, done ? 0u : 1u);
+    return;
+  }
+  unsigned long long* sw = ps.sw;
+  if (threadIdx.x == 0) { ps.live = 0; ps.proc = 0; ps.scan = 0; ps.edges = 0; ps.live_edges = 0; ps.newly_done = 0; }
+  __syncthreads();
   unsigned long long carry = 0;
   for (uint32_t b = 0; b < G; b += blockDim.x) {
     const uint32_t g = b + threadIdx.x;
     unsigned long long w = 0;
-    if (g < G && !was_done) {
+    if (g < G) {
       MemberState s = load_state_cg(st + g);
-      const uint32_t m = mem[g].m;
-      const uint32_t phase_before = s.phase;
-      switch (s.phase) {
-        case kPhaseScan0:
-          s.act_sel ^= 1u;
-          s.act_count = s.kept;
-          s.kept = 0;
-          if (s.processed >= m) s.phase = kPhaseDone;
-          else { s.level = s.min_kept; s.min_kept = 0xFFFFFFFFu; s.phase = kPhaseScan; }
-          break;
-        case kPhaseScan: {
-          s.act_sel ^= 1u;
-          s.act_count = s.kept;
-          s.kept = 0;
-          const unsigned long long cnt = s.next >> kWorkBits;
-          if (cnt) {
-            s.curr = s.next;
-            s.next = 0;
-            s.q_sel ^= 1u;
-            s.phase = kPhaseProc;
-            s.levels++;
-            s.max_level = s.level;
-          } else if (s.act_count == 0) {
-            s.phase = kPhaseDone;
-          } else {
-            s.level = s.min_kept;  // no edge at this level: jump to the next occupied one
-          }
-          s.min_kept = 0xFFFFFFFFu;
-          break;
-        }
-        case kPhaseProc: {
-          s.processed += (uint32_t)(s.curr >> kWorkBits);
-          const unsigned long long cnt = s.next >> kWorkBits;
-          if (cnt) {
-            s.curr = s.next;
-            s.next = 0;
-            s.q_sel ^= 1u;
-          } else {
-            s.curr = 0;
-            if (s.processed >= m) s.phase = kPhaseDone;
-            else { s.level += 1; s.phase = kPhaseScan; s.min_kept = 0xFFFFFFFFu; }
-          }
-          break;
-        }
-        default:
-          break;
-      }
-      if (s.phase != kPhaseDone) s.waves++;
-      else if (phase_before != kPhaseDone) atomicAdd(&ps.newly_done, 1u);
+      const uint32_t m = mem[g].m, before = s.phase;
+      w = advance_member(s, m);
       st[g] = s;
-      if (s.phase == kPhaseScan0 || s.phase == kPhaseScan) {
-        w = s.act_count;
-        if (w) atomicAdd(&s_scan, w);
-      } else if (s.phase == kPhaseProc) {
-        w = s.curr & kWorkMask;
-        atomicAdd(&s_proc, w);
-        atomicAdd(&s_edges, s.curr >> kWorkBits);
+      if (s.phase == kPhaseProc) {
+        atomicAdd(&ps.proc, w);
+        atomicAdd(&ps.edges, s.curr >> kWorkBits);
+      } else if (w) {
+        atomicAdd(&ps.scan, w);
       }
       if (s.phase != kPhaseDone) {
-        atomicAdd(&s_live, 1u);
-        atomicAdd(&s_live_edges, (unsigned long long)(m - s.processed));
+        atomicAdd(&ps.live, 1u);
+        atomicAdd(&ps.live_edges, (unsigned long long)(m - s.processed));
+      } else if (before != kPhaseDone) {
+        atomicAdd(&ps.newly_done, 1u);
       }
     }
     unsigned long long total;
@@ -1793,36 +1880,8 @@ __device__ __forceinline__ void plan_wave(const Member* __restrict__ mem, Member
   __syncthreads();
   if (threadIdx.x == 0) {
     wpref[G] = carry;
-    uint32_t done = was_done;
-    if (!was_done) {
-      if (ctl->trace && ctl->waves_run < ctl->trace_cap)
-        ctl->trace[ctl->waves_run] = make_ulonglong4(globaltimer(), carry, s_proc, s_scan);
-      ctl->el_proc += s_proc;
-      ctl->el_scan += s_scan;
-      ctl->edges_proc += s_edges;
-      ctl->total_work = carry;
-      ctl->wave += 1;
-      ctl->waves_run += 1;
-      const uint32_t e = __ldcg(err);
-      uint32_t reason = kExitNone;
-      if (s_live == 0) { done = 1; reason = kExitDone; }
-      if (e) { done = 1; reason = kExitError; }
-      if (ctl->waves_run > ctl->max_waves) { atomicOr(err, kErrWaves); done = 1; reason = kExitError; }
-      if (globaltimer() - ctl->t_start > ctl->timeout_ns) { atomicOr(err, kErrTimeout); done = 1; reason = kExitError; }
-      // live edges fill at most compact_pct % of the working rows (85 unless
-      // tuned): stop so the host can compact them (a compaction is a few passes
-      // over the rows, which the shorter rows repay at this fill; 78% and 90%
-      // measured slower on R-MAT-22)
-      if (!done && ctl->csr_slots >= ctl->compact_min &&
-          200 * s_live_edges <= (unsigned long long)ctl->compact_pct * ctl->csr_slots) {
-        done = 1;
-        reason = kExitCompact;
-      }
-      if (!done && ctl->notify_done && ps.newly_done) { done = 1; reason = kExitMember; }
-      if (!done && ctl->admit && *ctl->admit) { done = 1; reason = kExitAdmit; }
-      ctl->done = done;
-      ctl->exit_reason = reason;
-    }
+    const uint32_t done =
+        plan_commit(ctl, err, WavePlan{carry, ps.proc, ps.scan, ps.edges, ps.live_edges, ps.live, ps.newly_done});
     if (use_handle) cudaGraphSetConditional(handle, done ? 0u : 1u);
   }
 }
@@ -1907,39 +1966,36 @@ __device__ __noinline__ void wave_scan_segment(const Union* Up, MemberState* st,
 // R-MAT-22's peel 315 -> 257 ms, its first large wave 0.87 -> 0.68 ms on R-MAT-20
 // with 0.60 -> 0.36 G instructions and 2.7 -> 1.4 GB read.  The index is rebuilt
 // with the rows at every compaction, so it shrinks with what is left.
-template <bool kMulti>
-__global__ void __launch_bounds__(kWaveThreads, SPARX_WAVE_MINB) k_wave(WaveArgs a) {
-  __shared__ uint32_t s_push_eid[kWaveWarps][kPushBuf];
-  __shared__ uint32_t s_keep[kWaveWarps][kKeepBuf];
-  const Control* ctl = a.ctl;
-  // a stopped loop (host-launched waves run on until the host looks) does no
-  // work, but its blocks still hand over to the planner
-  const unsigned long long total = ctl->done ? 0ull : ctl->total_work;
-  const uint32_t W = ctl->wave;
-  const uint32_t G = ctl->G;
+template <int kWarps>
+struct WaveShared {
+  uint32_t push_eid[kWarps][kPushBuf];
+  uint32_t keep[kWarps][kKeepBuf];
+  // work counters (per warp: hits, groups of 32 elements inside one edge, groups
+  // over several edges), here rather than in registers held across the loop;
+  // lane 0 adds to them
+  uint32_t cnt[3][kWarps];
+  // warp-uniform state of the frontier loop, read back where it is used: held
+  // in registers it was spilled to local memory, whose lines the loop's random
+  // row and state loads evict from L1
+  unsigned long long w64[kWarps][3];  // kCtxJb, kCtxSegEnd, kCtxKend
+  uint32_t w32[kWarps][8];            // kCtxEb .. kCtxW
+};
+
+// This warp's share of wave W (warp `warp` of `nwarps`).
+template <bool kMulti, int kWarps>
+__device__ __forceinline__ void wave_work(const WaveArgs& a, WaveShared<kWarps>& sh, unsigned long long total,
+                                          uint32_t W, uint32_t G, unsigned long long warp,
+                                          unsigned long long nwarps) {
   const uint32_t lane = lane_id();
   const uint32_t wib = threadIdx.x >> 5;
-  const unsigned long long warp = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const unsigned long long nwarps = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
   const UnionRegs U(a.Up, a.arr);
-  // one chunk per warp: finer chunks (and any cap on their size) measured
-  // slower, the search for a chunk's first entry is paid once per warp;
-  // ch * nwarps >= total, so the chunk below is the warp's only one
+  // one chunk per warp: finer chunks (handed out by a block counter too: R-MAT-22
+  // 303 -> 321 to 361 ms with 1 to 8 pieces per warp) measured slower, the search
+  // for a chunk's first entry is paid once per warp; ch * nwarps >= total, so the chunk below is the warp's only one
   const unsigned long long ch = max(((total + nwarps - 1) / nwarps + 31) & ~31ull, 32ull);
-  // work counters live in shared memory (per warp: hits, groups of 32 elements
-  // inside one edge, groups over several edges) rather than in registers held
-  // across the loop; lane 0 adds to them
-  __shared__ uint32_t s_cnt[3][kWaveWarps];
-  if (lane < 3) s_cnt[lane][wib] = 0;
-  __syncwarp();
-  PushStage ps{s_push_eid[wib], 0};
-  // Warp-uniform state of the frontier loop lives in shared memory and is read
-  // back where it is used: held in registers it was spilled to local memory,
-  // whose lines the loop's random row and state loads evict from L1.
-  __shared__ unsigned long long s_w64[kWaveWarps][3];  // kCtxJb, kCtxSegEnd, kCtxKend
-  __shared__ uint32_t s_w32[kWaveWarps][8];            // kCtxEb .. kCtxW
-  volatile unsigned long long* const w64 = s_w64[wib];
-  volatile uint32_t* const w32 = s_w32[wib];
+  PushStage ps{sh.push_eid[wib], 0};
+  volatile unsigned long long* const w64 = sh.w64[wib];
+  volatile uint32_t* const w32 = sh.w32[wib];
 
   if (warp * ch < total) {
     const unsigned long long c0 = warp * ch;
@@ -1950,9 +2006,9 @@ __global__ void __launch_bounds__(kWaveThreads, SPARX_WAVE_MINB) k_wave(WaveArgs
     while (k < w64[kCtxKend]) {
       const unsigned long long kend = w64[kCtxKend];
       while (g + 1 < G && a.wpref[g + 1] <= k) ++g;
-      const unsigned long long mbeg = a.wpref[g];
+      const unsigned long long mbeg = G > 1 ? a.wpref[g] : 0ull;
       // a segment spans < 2^31 elements, so offsets inside it are 32-bit
-      const unsigned long long seg_end = min(min(kend, a.wpref[g + 1]), k + (1ull << 31));
+      const unsigned long long seg_end = min(min(kend, G > 1 ? a.wpref[g + 1] : total), k + (1ull << 31));
       if (seg_end <= k || mbeg > k) {  // layout does not cover k: stop rather than spin
         if (lane == 0) atomicOr(a.err, kErrInternal);
         break;
@@ -2018,7 +2074,7 @@ __global__ void __launch_bounds__(kWaveThreads, SPARX_WAVE_MINB) k_wave(WaveArgs
             o_end = o - lane + rem;
             r += rem;
             i += 1;
-            if (lane == 0) s_cnt[1][wib] += (rem + 31) / 32;
+            if (lane == 0) sh.cnt[1][wib] += (rem + 31) / 32;
           } else {
             uint32_t t = 0;
 #pragma unroll
@@ -2034,7 +2090,7 @@ __global__ void __launch_bounds__(kWaveThreads, SPARX_WAVE_MINB) k_wave(WaveArgs
             valid = r + lane < seg_len;
             o_end = o + 1;
             r += 32;
-            if (lane == 0) s_cnt[2][wib]++;
+            if (lane == 0) sh.cnt[2][wib]++;
           }
           if (valid) {
             dsc = ((w32[kCtxQsel] ? U.qd1 : U.qd0) + w32[kCtxEb])[x];
@@ -2112,7 +2168,7 @@ __global__ void __launch_bounds__(kWaveThreads, SPARX_WAVE_MINB) k_wave(WaveArgs
           }
         }
         found = __reduce_add_sync(kFull, found);
-        if (lane == 0) s_cnt[0][wib] += found;
+        if (lane == 0) sh.cnt[0][wib] += found;
         // entries belong to this member: publish before moving on
         push_flush(ps, a.Up, w32[kCtxEb], w32[kCtxM], a.st + w32[kCtxG], a.err, w32[kCtxQsel]);
         k = w64[kCtxSegEnd];
@@ -2121,23 +2177,42 @@ __global__ void __launch_bounds__(kWaveThreads, SPARX_WAVE_MINB) k_wave(WaveArgs
       } else if (phase == kPhaseScan0 || phase == kPhaseScan) {
         // active-list positions are below the member's edge count (< 2^28)
         wave_scan_segment(a.Up, st, M.eb, M.m, phase, level, act_sel, q_sel, W, (uint32_t)(k - mbeg),
-                          (uint32_t)(seg_end - k), s_keep[wib], ps.eid, a.err);
+                          (uint32_t)(seg_end - k), sh.keep[wib], ps.eid, a.err);
       }
       push_flush(ps, a.Up, M.eb, M.m, st, a.err, q_sel);  // entries belong to this member: publish before moving on
       k = seg_end;
     }
   }
-  // work counters: summed per block, then one atomic per counter and block
-  // (per-warp atomics on four addresses serialise on large waves)
-  __syncthreads();
+}
+
+// Work counters: summed per block, then one atomic per counter and block
+// (per-warp atomics on three addresses serialise on large waves).  All threads
+// call it, after a block barrier.
+template <int kWarps>
+__device__ __forceinline__ void flush_counts(const WaveArgs& a, const WaveShared<kWarps>& sh) {
   if (threadIdx.x < 3) {
     unsigned long long sum = 0;
-#pragma unroll
-    for (int w = 0; w < kWaveWarps; ++w) sum += s_cnt[threadIdx.x][w];
+#pragma unroll 8
+    for (int w = 0; w < kWarps; ++w) sum += sh.cnt[threadIdx.x][w];
     unsigned long long* dst = threadIdx.x == 0 ? &a.ctl->hits
                               : threadIdx.x == 1 ? &a.ctl->merge_iters : &a.ctl->lane_iters;
     if (sum) atomicAdd(dst, sum);
   }
+}
+
+template <bool kMulti>
+__global__ void __launch_bounds__(kWaveThreads, SPARX_WAVE_MINB) k_wave(WaveArgs a) {
+  __shared__ WaveShared<kWaveWarps> sh;
+  const uint32_t lane = lane_id();
+  if (lane < 3) sh.cnt[lane][threadIdx.x >> 5] = 0;
+  __syncwarp();
+  // a stopped loop (host-launched waves run on until the host looks) does no
+  // work, but its blocks still hand over to the planner
+  wave_work<kMulti>(a, sh, a.ctl->done ? 0ull : a.ctl->total_work, a.ctl->wave, a.ctl->G,
+                    ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5,
+                    ((unsigned long long)gridDim.x * blockDim.x) >> 5);
+  __syncthreads();
+  flush_counts(a, sh);
   // the last block to finish plans the next wave (threadfence-reduction
   // pattern: every thread fences its writes, the block takes a ticket; the
   // block holding the last ticket sees every other block's writes)
@@ -2149,9 +2224,48 @@ __global__ void __launch_bounds__(kWaveThreads, SPARX_WAVE_MINB) k_wave(WaveArgs
   __syncthreads();
   if (s_last) {
     __threadfence();
-    plan_wave(a.mem, a.st, a.ctl, a.wpref, a.err, a.handle, a.use_handle, s_plan);
+    plan_wave(a.mem, a.st, a.ctl, a.wpref, a.err, a.handle, a.use_handle, s_plan, a.ctl->G, a.ctl->done);
     if (threadIdx.x == 0) a.ctl->blocks_done = 0;
   }
+}
+
+// Small waves in one launch: a single thread-block cluster runs wave after wave
+// while the planned one has at most `max_work` elements, its blocks meeting at
+// the cluster's hardware barrier instead of at a kernel boundary, and block 0
+// planning between two of them.  A wave of 100 elements takes 7 us here, 13 to 14
+// as a kernel of 1,184 blocks (launch gap 3, block start 1, ticket 2); what is
+// left is its chain of dependent round trips to L2.  The barrier's release and
+// acquire order the waves' memory; everything a wave reads through the read-only
+// path (rows, index, edges) does not change between compactions.  Every block
+// leaves the loop on the same values, read after the same barrier, and the
+// planner's bounds (waves, time) end it as they end the loop of k_wave.
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <bool kMulti>
+__global__ void __launch_bounds__(kTailThreads, 1) k_wave_tail(WaveArgs a, unsigned long long max_work) {
+  __shared__ WaveShared<kTailThreads / 32> sh;
+  __shared__ PlanShared s_plan;
+  const uint32_t wib = threadIdx.x >> 5;
+  if (lane_id() < 3) sh.cnt[lane_id()][wib] = 0;
+  __syncwarp();
+  for (;;) {
+    const unsigned long long total = __ldcg(&a.ctl->total_work);
+    const uint32_t W = __ldcg(&a.ctl->wave);
+    const uint32_t G = __ldcg(&a.ctl->G);
+    if (__ldcg(&a.ctl->done) || total > max_work) break;
+    wave_work<kMulti>(a, sh, total, W, G, wib * gridDim.x + blockIdx.x, (kTailThreads / 32) * gridDim.x);
+    __syncwarp();
+    cluster_barrier();
+    if (blockIdx.x == 0) plan_wave(a.mem, a.st, a.ctl, a.wpref, a.err, a.handle, 0, s_plan, G, false);
+    __syncwarp();
+    cluster_barrier();
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0 && a.use_handle)
+    cudaGraphSetConditional(a.handle, __ldcg(&a.ctl->done) ? 0u : 1u);
+  __syncthreads();
+  flush_counts(a, sh);
 }
 
 // Vertices and slots per floor(log2(degree)): the degree signature the tuning

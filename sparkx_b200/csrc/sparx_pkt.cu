@@ -281,6 +281,7 @@ struct Engine {
   PeelGraph peel;
   int wave_blocks = 0;        // k_wave<false> grid (resident blocks per SM x SMs)
   int wave_blocks_multi = 0;  // k_wave<true> grid (multigraphs)
+  int tail_blocks = 0;        // k_wave_tail: blocks of its cluster (0: the device takes none)
   char* ws2 = nullptr;        // multigraph rows, multiplicities and slot map (allocated on first use)
   size_t ws2_cap = 0;
   char* ws3 = nullptr;        // rank index of the working rows and the queues' headers (allocated on first use)
@@ -289,10 +290,55 @@ struct Engine {
   std::mutex mu;
 };
 
+// Elements of the largest wave the cluster takes: 16 SMs run 3 groups of 32 per
+// warp in about the time the whole chip needs to start, run and hand over one
+// (16 to 48 thousand elements 13 us either way; R-MAT-12 3.83 / 3.61 / 3.49 ms at
+// a bound of 16, 32 and 48 thousand, R-MAT-19 and 22 within noise).
+constexpr unsigned long long kTailMaxWork = 49152;
+
 constexpr unsigned long long kTraceRecords = 1ull << 20;
 
 std::mutex g_engines_mu;
 std::map<int, Engine*> g_engines;
+
+// The small waves' cluster: one of 16 blocks, else of 8 (the portable size), on
+// the current device; 0 when neither can be resident.
+template <bool kMulti>
+cudaError_t launch_tail(int blocks, const WaveArgs& wa, cudaStream_t s) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(kTailThreads);
+  cfg.stream = s;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = blocks;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_wave_tail<kMulti>, wa, kTailMaxWork);
+}
+
+int tail_cluster() {
+  for (int blocks : {16, 8}) {
+    int clusters = 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(kTailThreads);
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = blocks;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    if (cudaFuncSetAttribute(k_wave_tail<false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+        cudaFuncSetAttribute(k_wave_tail<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&clusters, k_wave_tail<true>, &cfg) == cudaSuccess && clusters > 0 &&
+        cudaOccupancyMaxActiveClusters(&clusters, k_wave_tail<false>, &cfg) == cudaSuccess && clusters > 0)
+      return blocks;
+  }
+  cudaGetLastError();
+  return 0;
+}
 
 int engine_init(Engine& E, int device) {
   E.device = device;
@@ -308,10 +354,11 @@ int engine_init(Engine& E, int device) {
   for (auto& e : E.tev) CU(cudaEventCreate(&e));
   CU(cudaHostAlloc(&E.pinned_small, 4096, cudaHostAllocDefault));
   int per_sm = 0;
-  CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_wave<false>, 256, 0));
+  CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_wave<false>, kWaveThreads, 0));
   E.wave_blocks = std::max(1, per_sm) * E.sm_count;
-  CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_wave<true>, 256, 0));
+  CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_wave<true>, kWaveThreads, 0));
   E.wave_blocks_multi = std::max(1, per_sm) * E.sm_count;
+  E.tail_blocks = tail_cluster();
   return SPARX_OK;
 }
 
@@ -677,6 +724,10 @@ PeelArrays peel_arrays(const Union& U) {
 #define SPARX_WAVES_PER_ITERATION 4
 #endif
 constexpr int kWavesPerIteration = SPARX_WAVES_PER_ITERATION;
+// One small-wave launch (about 2 us when the planned wave is too large for it)
+// per this many wave kernels of the loop body: R-MAT-22 302.6 / 304.9 / 309 ms
+// at 4 / 2 / 1.
+constexpr int kWavesPerTail = 4;
 
 int build_peel_graph(Engine& E, const UnionJob& J, const PeelArrays& arr) {
   const Layout& L = J.L;
@@ -718,8 +769,10 @@ int build_peel_graph(Engine& E, const UnionJob& J, const PeelArrays& arr) {
   // several waves per loop iteration: a wave that finds the loop stopped does
   // nothing, and the condition is read once per iteration
   for (int i = 0; i < kWavesPerIteration; ++i) {
-    if (arr.mu) k_wave<true><<<E.wave_blocks_multi, 256, 0, E.capture>>>(wa);
-    else k_wave<false><<<E.wave_blocks, 256, 0, E.capture>>>(wa);
+    if (E.tail_blocks && i % kWavesPerTail == 0)
+      CU(arr.mu ? launch_tail<true>(E.tail_blocks, wa, E.capture) : launch_tail<false>(E.tail_blocks, wa, E.capture));
+    if (arr.mu) k_wave<true><<<E.wave_blocks_multi, kWaveThreads, 0, E.capture>>>(wa);
+    else k_wave<false><<<E.wave_blocks, kWaveThreads, 0, E.capture>>>(wa);
   }
   cudaGraph_t captured;
   CU(cudaStreamEndCapture(E.capture, &captured));
@@ -1163,8 +1216,8 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
       } else {
         for (;;) {
           for (int i = 0; i < 16; ++i) {
-            if (mu) k_wave<true><<<E.wave_blocks_multi, 256, 0, s>>>(wa);
-            else k_wave<false><<<E.wave_blocks, 256, 0, s>>>(wa);
+            if (mu) k_wave<true><<<E.wave_blocks_multi, kWaveThreads, 0, s>>>(wa);
+            else k_wave<false><<<E.wave_blocks, kWaveThreads, 0, s>>>(wa);
           }
           J.launches += 16;
           CU(cudaMemcpyAsync(hctl, wa.ctl, sizeof(Control), cudaMemcpyDeviceToHost, s));
@@ -3329,7 +3382,7 @@ int run_noalloc(const uint64_t* d_offsets, uint64_t n_plus_1, const uint32_t* d_
   uint32_t* err = &cnt->err;
   int sm = 148, per_sm = 1;
   CU(cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, device));
-  CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_wave<false>, 256, 0));
+  CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_wave<false>, kWaveThreads, 0));
   const int wave_blocks = std::max(1, per_sm) * sm;
   const uint32_t N = (uint32_t)n;
 
@@ -3446,7 +3499,7 @@ int run_noalloc(const uint64_t* d_offsets, uint64_t n_plus_1, const uint32_t* d_
   wa.handle = cudaGraphConditionalHandle{};
   wa.use_handle = 0;
   for (;;) {
-    for (int i = 0; i < 16; ++i) k_wave<false><<<wave_blocks, 256, 0, s>>>(wa);
+    for (int i = 0; i < 16; ++i) k_wave<false><<<wave_blocks, kWaveThreads, 0, s>>>(wa);
     uint32_t done = 0;
     CU(cudaMemcpyAsync(&done, &dC->done, 4, cudaMemcpyDeviceToHost, s));
     CU(cudaStreamSynchronize(s));
