@@ -169,6 +169,7 @@ struct Control {
   unsigned long long edges_proc;  // frontier edges processed
   unsigned long long csr_slots;   // entries in the working rows
   unsigned long long compact_min; // do not compact working rows smaller than this
+  unsigned long long compact_el;  // el_proc at the last compaction
   uint32_t exit_reason;           // why the loop stopped: kExit*
   uint32_t blocks_done;           // wave blocks finished (the last one plans the next wave)
   uint32_t compactions;
@@ -399,9 +400,8 @@ __device__ __forceinline__ T block_exclusive_scan(T x, T* smem_warp, T& total) {
 // lanes busy.
 constexpr uint32_t kLaneRow = 32;
 
-// Rows longer than kWarpRow entries (by original degree) are oriented and
-// compacted by a block each (the *_big kernels over the list k_big_rows
-// builds); the others by their lane or their warp.
+// Rows longer than kWarpRow entries are oriented by a block each (over the list
+// k_big_rows builds); the others by their lane or their warp.
 constexpr uint32_t kWarpRow = 2048;
 
 __device__ __forceinline__ bool big_row(const uint32_t* __restrict__ off0, uint32_t u) {
@@ -1747,6 +1747,9 @@ __device__ __forceinline__ unsigned long long advance_member(MemberState& s, uin
 
 // The loop's side of a planned wave: work counters, the bounds, and whether the
 // loop stops here.  One thread calls it; returns ctl->done.
+// 1, 2 and 8 measured alike on R-MAT-19, R-MAT-22 and the mix of 24 graphs.
+constexpr unsigned long long kCompactPay = 2;
+
 struct WavePlan {
   unsigned long long total, proc, scan, edges, live_edges;
   uint32_t live, newly_done;
@@ -1755,7 +1758,8 @@ __device__ __forceinline__ uint32_t plan_commit(Control* ctl, uint32_t* __restri
   // one round of loads, then one of stores
   const unsigned long long waves = ctl->waves_run + 1, max_waves = ctl->max_waves, t_start = ctl->t_start,
                            timeout = ctl->timeout_ns, el_proc = ctl->el_proc, el_scan = ctl->el_scan,
-                           edges = ctl->edges_proc, slots = ctl->csr_slots, compact_min = ctl->compact_min;
+                           edges = ctl->edges_proc, slots = ctl->csr_slots, compact_min = ctl->compact_min,
+                           compact_el = ctl->compact_el;
   const uint32_t wave = ctl->wave, pct = ctl->compact_pct, notify = ctl->notify_done;
   const volatile uint32_t* admit = ctl->admit;
   ulonglong4* trace = ctl->trace;
@@ -1776,7 +1780,11 @@ __device__ __forceinline__ uint32_t plan_commit(Control* ctl, uint32_t* __restri
   // tuned): stop so the host can compact them (a compaction is a few passes
   // over the rows, which the shorter rows repay at this fill; 78% and 90%
   // measured slower on R-MAT-22)
-  if (!done && slots >= compact_min && 200 * P.live_edges <= (unsigned long long)pct * slots) {
+  // ... once the waves since the last one have searched at least a kCompactPay-th
+  // as many elements as it would move: a graph whose peel ends in a few small
+  // waves (de Bruijn: 305 elements, 49 M slots, 0.6 of its 5.2 ms) never pays it
+  if (!done && slots >= compact_min && 200 * P.live_edges <= (unsigned long long)pct * slots &&
+      kCompactPay * (el_proc + P.proc - compact_el) >= slots) {
     done = 1;
     reason = kExitCompact;
   }
@@ -2293,9 +2301,17 @@ __global__ void __launch_bounds__(256) k_hub_hist(const uint32_t* __restrict__ o
 
 // Working-row compaction (between waves): keep the entries whose edge is not
 // processed (tag >= the next wave).  The edges' states are first condensed
-// into a bitmap (one bit per edge, small enough to stay in L2), so the row
-// passes look up a bit instead of a random 8-byte state.  Mark, count, scan
-// (host), fill; 32 vertices per warp for the row passes.
+// into a bitmap (one bit per edge, small enough to stay in L2); the rows are then
+// one flat array whose kept entries move up, whatever rows they belong to, so no
+// row's length matters: with a lane, a warp or a block per row the passes waited
+// for warps whose 32 neighbouring rows were all long (degree-ordered vertices):
+// the 28 compactions of R-MAT-22 20 -> 5 ms, mix of 24 graphs 212 -> 192 ms.  Bound
+// by the bitmap's lookups (one per slot, L2) and 24 bytes of HBM per slot.
+//   k_compact_mark     edges -> bitmap
+//   k_compact_count    slots -> bitmap, kept slots per tile (then scanned)
+//   k_compact_move     kept entries to their new place, kept slots before each
+//                      32-slot word
+//   k_compact_offsets  each row's start: the kept slots before its old start
 __global__ void __launch_bounds__(256) k_compact_mark(const int2* __restrict__ es, uint32_t m,
                                                       const Control* ctl, uint32_t* __restrict__ alive) {
   const uint32_t lane = lane_id();
@@ -2315,133 +2331,68 @@ __device__ __forceinline__ bool is_alive(const uint32_t* __restrict__ alive, uin
   return x != kInvalid && ((__ldg(alive + (x >> 5)) >> (x & 31)) & 1u);
 }
 
-__global__ void __launch_bounds__(256) k_compact_count(const uint32_t* __restrict__ off,
-                                                       const unsigned long long* __restrict__ row, uint32_t n,
+constexpr uint32_t kCompactTile = 8192;  // slots per block of 256 threads: a 32-slot word each
+
+__global__ void __launch_bounds__(256) k_compact_count(const unsigned long long* __restrict__ row,
+                                                       unsigned long long slots,
                                                        const uint32_t* __restrict__ alive,
-                                                       uint32_t* __restrict__ cnt,
-                                                       const uint32_t* __restrict__ off0) {
-  const uint32_t lane = lane_id();
-  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t base = warp * 32; base < n; base += nwarps * 32) {
-    const uint32_t u = base + lane;
-    uint32_t b = 0, e = 0;
-    if (u < n) { b = __ldg(off + u); e = __ldg(off + u + 1); }
-    uint32_t c = 0;
-    if (u < n && e - b <= kLaneRow)
-      for (uint32_t s = b; s < e; ++s) c += is_alive(alive, (uint32_t)(__ldg(row + s) >> 32));
-    const bool blk = u < n && e - b > kLaneRow && big_row(off0, u);
-    unsigned big = __ballot_sync(kFull, u < n && e - b > kLaneRow && !blk);
-    while (big) {
-      const int j = __ffs(big) - 1;
-      big &= big - 1;
-      const uint32_t bb = __shfl_sync(kFull, b, j), be = __shfl_sync(kFull, e, j);
-      uint32_t cc = 0;
-      for (uint32_t s = bb + lane; s < be; s += 32) cc += is_alive(alive, (uint32_t)(__ldg(row + s) >> 32));
+                                                       uint32_t* __restrict__ kept, uint32_t* __restrict__ tiles) {
+  __shared__ uint32_t s_sum[8];
+  const uint32_t lane = lane_id(), wid = threadIdx.x >> 5;
+  const unsigned long long base = (unsigned long long)blockIdx.x * kCompactTile;
+  uint32_t sum = 0;
+#pragma unroll 8
+  for (uint32_t x = wid; x < kCompactTile / 32; x += 8) {
+    const unsigned long long i = base + 32 * x + lane;
+    const bool k = i < slots && is_alive(alive, (uint32_t)(__ldg(row + i) >> 32));
+    const uint32_t bits = __ballot_sync(kFull, k);
+    if (lane == 0 && base + 32 * x < slots) kept[(base >> 5) + x] = bits;
+    sum += __popc(bits);
+  }
+  if (lane == 0) s_sum[wid] = sum;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    uint32_t t = 0;
 #pragma unroll
-      for (int d = 16; d > 0; d >>= 1) cc += __shfl_xor_sync(kFull, cc, d);
-      if (lane == (uint32_t)j) c = cc;
-    }
-    if (u < n && !blk) cnt[u] = c;
+    for (int w = 0; w < 8; ++w) t += s_sum[w];
+    tiles[blockIdx.x] = t;
   }
 }
 
-__global__ void __launch_bounds__(256) k_compact_fill(const uint32_t* __restrict__ off,
-                                                      const unsigned long long* __restrict__ row, uint32_t n,
-                                                      const uint32_t* __restrict__ alive,
-                                                      const uint32_t* __restrict__ off2,
-                                                      unsigned long long* __restrict__ row2,
-                                                      const uint32_t* __restrict__ off0) {
-  const uint32_t lane = lane_id();
-  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t base = warp * 32; base < n; base += nwarps * 32) {
-    const uint32_t u = base + lane;
-    uint32_t b = 0, e = 0;
-    if (u < n) { b = __ldg(off + u); e = __ldg(off + u + 1); }
-    if (u < n && e - b <= kLaneRow) {
-      uint32_t at = __ldg(off2 + u);
-      for (uint32_t s = b; s < e; ++s) {
-        const unsigned long long pr = __ldg(row + s);
-        if (is_alive(alive, (uint32_t)(pr >> 32))) row2[at++] = pr;
-      }
-    }
-    unsigned big = __ballot_sync(kFull, u < n && e - b > kLaneRow && !big_row(off0, u));
-    while (big) {
-      const int j = __ffs(big) - 1;
-      big &= big - 1;
-      const uint32_t bb = __shfl_sync(kFull, b, j), be = __shfl_sync(kFull, e, j);
-      uint32_t at = __ldg(off2 + base + j);
-      for (uint32_t s0 = bb; s0 < be; s0 += 32) {
-        const uint32_t s = s0 + lane;
-        unsigned long long pr = 0;
-        bool keep = false;
-        if (s < be) {
-          pr = __ldg(row + s);
-          keep = is_alive(alive, (uint32_t)(pr >> 32));
-        }
-        const unsigned bal = __ballot_sync(kFull, keep);
-        if (keep) row2[at + __popc(bal & ((1u << lane) - 1))] = pr;
-        at += __popc(bal);
-      }
-    }
+__global__ void __launch_bounds__(256) k_compact_move(const unsigned long long* __restrict__ row,
+                                                      unsigned long long slots,
+                                                      const uint32_t* __restrict__ kept,
+                                                      const uint32_t* __restrict__ tiles,
+                                                      uint32_t* __restrict__ before,
+                                                      unsigned long long* __restrict__ row2) {
+  __shared__ uint32_t s_scan[32], s_bits[256], s_at[256];
+  const uint32_t lane = lane_id(), wid = threadIdx.x >> 5;
+  const unsigned long long base = (unsigned long long)blockIdx.x * kCompactTile;
+  const unsigned long long word = (base >> 5) + threadIdx.x;
+  const uint32_t bits = 32 * word < slots ? __ldg(kept + word) : 0u;
+  uint32_t total;
+  const uint32_t at = __ldg(tiles + blockIdx.x) + block_exclusive_scan<uint32_t>(__popc(bits), s_scan, total);
+  if (32 * word < slots) before[word] = at;
+  s_bits[threadIdx.x] = bits;
+  s_at[threadIdx.x] = at;
+  __syncthreads();
+#pragma unroll 8
+  for (uint32_t x = wid; x < kCompactTile / 32; x += 8) {
+    const uint32_t m = s_bits[x];
+    if (m >> lane & 1) row2[s_at[x] + __popc(m & ((1u << lane) - 1))] = __ldg(row + base + 32 * x + lane);
   }
 }
 
-// Big rows, a block of 1024 threads each.  Count: block sum.  Fill: chunks of
-// 4096 entries, four consecutive per thread, placed by a block-wide exclusive
-// scan so the row keeps its order.
-__global__ void __launch_bounds__(1024) k_compact_count_big(const uint32_t* __restrict__ off,
-                                                           const unsigned long long* __restrict__ row,
-                                                           const uint32_t* __restrict__ alive,
-                                                           uint32_t* __restrict__ cnt,
-                                                           const uint32_t* __restrict__ list,
-                                                           const uint32_t* __restrict__ count) {
-  __shared__ unsigned long long sw[32];
-  const uint32_t nbig = *count;
-  for (uint32_t r = blockIdx.x; r < nbig; r += gridDim.x) {
-    const uint32_t u = list[r];
-    const uint32_t b = __ldg(off + u), e = __ldg(off + u + 1);
-    unsigned long long c = 0;
-#pragma unroll 4
-    for (uint32_t s = b + threadIdx.x; s < e; s += blockDim.x) c += is_alive(alive, (uint32_t)(__ldg(row + s) >> 32));
-    unsigned long long total;
-    block_exclusive_scan<unsigned long long>(c, sw, total);
-    if (threadIdx.x == 0) cnt[u] = (uint32_t)total;
-  }
-}
-
-__global__ void __launch_bounds__(1024) k_compact_fill_big(const uint32_t* __restrict__ off,
-                                                          const unsigned long long* __restrict__ row,
-                                                          const uint32_t* __restrict__ alive,
-                                                          const uint32_t* __restrict__ off2,
-                                                          unsigned long long* __restrict__ row2,
-                                                          const uint32_t* __restrict__ list,
-                                                          const uint32_t* __restrict__ count) {
-  __shared__ uint32_t sw[32];
-  const uint32_t nbig = *count;
-  for (uint32_t r = blockIdx.x; r < nbig; r += gridDim.x) {
-    const uint32_t u = list[r];
-    const uint32_t b = __ldg(off + u), e = __ldg(off + u + 1);
-    uint32_t at = __ldg(off2 + u);
-    for (uint32_t base = b; base < e; base += 4 * blockDim.x) {
-      const uint32_t s0 = base + 4 * threadIdx.x;
-      unsigned long long pr[4];
-      uint32_t keep = 0, nk = 0;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        pr[i] = s0 + i < e ? __ldg(row + s0 + i) : 0ull;
-        const bool k = s0 + i < e && is_alive(alive, (uint32_t)(pr[i] >> 32));
-        keep |= (uint32_t)k << i;
-        nk += k;
-      }
-      uint32_t total;
-      uint32_t pos = at + block_exclusive_scan<uint32_t>(nk, sw, total);
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-        if (keep & (1u << i)) row2[pos++] = pr[i];
-      at += total;
-    }
+// `total`: kept slots (a row may start at the array's end)
+__global__ void __launch_bounds__(256) k_compact_offsets(const uint32_t* __restrict__ off, uint32_t n,
+                                                         unsigned long long slots,
+                                                         const uint32_t* __restrict__ kept,
+                                                         const uint32_t* __restrict__ before,
+                                                         const uint32_t* __restrict__ total,
+                                                         uint32_t* __restrict__ off2) {
+  for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u <= n; u += gridDim.x * blockDim.x) {
+    const uint32_t s = __ldg(off + u);
+    off2[u] = s < slots ? __ldg(before + (s >> 5)) + __popc(__ldg(kept + (s >> 5)) & ((1u << (s & 31)) - 1)) : *total;
   }
 }
 
@@ -2476,6 +2427,7 @@ __global__ void k_compact_commit(Union* U, const uint32_t* off2, const unsigned 
   U->row = row2;
   ctl->csr_slots = *new_slots;
   ctl->compactions += 1;
+  ctl->compact_el = ctl->el_proc;
   ctl->exit_reason = kExitNone;
   ctl->done = 0;
 }
@@ -2956,13 +2908,6 @@ __global__ void k_shift_pairs(unsigned long long* __restrict__ dst, const unsign
     const uint32_t name = (uint32_t)pr + name_add, e = (uint32_t)(pr >> 32);
     dst[i] = make_pair(name, e == kInvalid ? kInvalid : e + eid_add);
   }
-}
-
-// rows longer than kWarpRow among vertices [v0, v1), appended to the list
-__global__ void __launch_bounds__(256) k_big_rows_range(const uint32_t* __restrict__ off0, uint32_t v0, uint32_t v1,
-                                                        uint32_t* __restrict__ list, uint32_t* __restrict__ count) {
-  for (uint32_t u = v0 + blockIdx.x * blockDim.x + threadIdx.x; u < v1; u += gridDim.x * blockDim.x)
-    if (big_row(off0, u)) list[atomicAdd(count, 1u)] = u;
 }
 
 // new members' states (the first wave of a member is its level-0 scan)

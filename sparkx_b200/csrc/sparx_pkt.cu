@@ -190,7 +190,7 @@ struct Counters {  // device scalars
   uint32_t hcursor;      //                      next heavy vertex
   uint32_t heavy_count;  //                      heavy vertices listed
   uint32_t hub_count;    // rows given the finer rank index
-  uint32_t big_count;    // rows compacted by a block each
+  uint32_t big_count;    // rows oriented by a block each
   uint32_t fin_err;      // served unions: error flags of one member's finalize
   uint32_t table_big;    // rank index, hash tables: what is listed for whole blocks
   double cc_possible;    // clustering: sum of d(d - 1)/2 over vertices
@@ -205,7 +205,8 @@ struct Layout {
   size_t offA, offB, rowA, rowB;  // compaction ping-pong buffers (0 when compaction is off)
   size_t vinfo;                   // per vertex: its list's or row's rank index header
   size_t alive;                   // compaction: one bit per edge, set while it is unprocessed
-  size_t big;                     // compaction: rows longer than kWarpRow (a block each)
+  size_t kept, before;            // compaction: kept slots as a bitmap, and counted before each of its words
+  size_t big;                     // rows longer than kWarpRow (a block each)
   size_t hub_hist;                // the degree signature's histogram
   size_t tiles, ctl, mem, st, wpref, cnt, mem_tri, mem_maxsup, uni;
   size_t total;
@@ -240,12 +241,14 @@ Layout make_layout(uint64_t N, uint64_t W, uint32_t G, bool own_nbr, size_t out_
   L.rowA = take(8 * W);
   L.rowB = take(8 * W);
   L.alive = take(4 * ((M + 31) / 32));
+  L.kept = take(4 * ((W + 31) / 32));
+  L.before = take(4 * ((W + 31) / 32));
   L.big = take(4 * (W / kWarpRow + 1));
   L.hub_hist = take(4 * 34 + 8 * 34);  // vertices, then slots, per log2 degree (the tuning key)
   L.vinfo = take(8ull * N);
   L.stage0 = take(kStageBytes);
   L.stage1 = take(kStageBytes);
-  const uint64_t tiles = (std::max<uint64_t>(N + 1, M + 1) + kScanTile - 1) / kScanTile + 2;
+  const uint64_t tiles = (std::max<uint64_t>({N + 1, M + 1, W / (kCompactTile / kScanTile)}) + kScanTile - 1) / kScanTile + 2;
   L.tiles = take(8 * tiles);
   L.ctl = take(sizeof(Control));
   L.mem = take(sizeof(Member) * G);
@@ -917,7 +920,7 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
     CU(cudaMemsetAsync(hub_hist, 0, 4 * 34 + 8 * 34, s));
     k_hub_hist<<<grid_for(N, 256, E.sm_count * 4), 256, 0, s>>>(J.off, N, hub_hist, hub_hist_slots);
     J.launches += 1;
-    // rows orientation and compaction give a block each (listed by original degree)
+    // rows the orientation gives a block each
     CU(cudaMemsetAsync(&cnt->big_count, 0, 4, s));
     k_big_rows<<<grid_for(N, 256, E.sm_count * 8), 256, 0, s>>>(J.off, N, big, &cnt->big_count);
     k_orient_count<<<vgrid, 256, 0, s>>>(J.off, J.nbr, N, dplus, &cnt->self_loops, err, &cnt->max_dplus, big,
@@ -1239,15 +1242,18 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
       uint32_t* off2 = at<uint32_t>(E, next_buf ? L.offB : L.offA);
       unsigned long long* row2 = at<unsigned long long>(E, next_buf ? L.rowB : L.rowA);
       uint32_t* alive = at<uint32_t>(E, L.alive);
-      const int pvgrid = grid_for(pN, 256, E.sm_count * 32);
+      uint32_t* kept = at<uint32_t>(E, L.kept);
+      uint32_t* before = at<uint32_t>(E, L.before);
+      uint32_t* tiles = at<uint32_t>(E, L.tiles);
+      const unsigned long long slots = hctl->csr_slots;
+      const uint32_t ntiles = (uint32_t)((slots + kCompactTile - 1) / kCompactTile);
       k_compact_mark<<<grid_for((pm + 31) / 32 * 32ull, 256, E.sm_count * 16), 256, 0, s>>>(es, (uint32_t)pm,
                                                                                            wa.ctl, alive);
-      k_compact_count<<<pvgrid, 256, 0, s>>>(cur_off, cur_row, pN, alive, dplus, J.off);
-      k_compact_count_big<<<E.sm_count * 2, 1024, 0, s>>>(cur_off, cur_row, alive, dplus, big, &cnt->big_count);
-      exclusive_scan<uint32_t>(LoadU32{dplus}, pN, off2, at<uint32_t>(E, L.tiles), (uint32_t*)&cnt->grand, s);
-      k_compact_fill<<<pvgrid, 256, 0, s>>>(cur_off, cur_row, pN, alive, off2, row2, J.off);
-      k_compact_fill_big<<<E.sm_count * 2, 1024, 0, s>>>(cur_off, cur_row, alive, off2, row2, big,
-                                                         &cnt->big_count);
+      k_compact_count<<<ntiles, 256, 0, s>>>(cur_row, slots, alive, kept, tiles);
+      k_scan_tiles<uint32_t><<<1, kScanThreads, 0, s>>>(tiles, ntiles, (uint32_t*)&cnt->grand);
+      k_compact_move<<<ntiles, 256, 0, s>>>(cur_row, slots, kept, tiles, before, row2);
+      k_compact_offsets<<<grid_for(pN + 1ull, 256, E.sm_count * 16), 256, 0, s>>>(cur_off, pN, slots, kept, before,
+                                                                                  (uint32_t*)&cnt->grand, off2);
       k_compact_commit<<<1, 1, 0, s>>>(at<Union>(E, L.uni), off2, row2, off2 + pN, wa.ctl);
       if (rpool) {
         const int rc = index_rows(off2, row2, nullptr);
@@ -1255,7 +1261,7 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
       }
       const uint32_t per = std::max<uint32_t>(1, (uint32_t)(E.sm_count * 8) / std::max<uint32_t>(pG, 1));
       k_refresh_desc<<<pG * per, 256, 0, s>>>(wa.Up, dmem, wa.st, pG, per);
-      J.launches += 8;
+      J.launches += 7;
       cur_off = off2;
       cur_row = row2;
       U.off = off2;
@@ -2225,9 +2231,6 @@ struct LaneHook : ServeHook {
       CU(cudaMemcpyAsync(at<int2>(E, L.es) + m0, at<int2>(*P, PJ.L.es), 8 * mp, cudaMemcpyDeviceToDevice, s));
     }
     Counters* cnt = at<Counters>(E, L.cnt);
-    if (Np) k_big_rows_range<<<grid_for(Np, 256, E.sm_count * 8), 256, 0, s>>>(off, N0, N0 + (uint32_t)Np,
-                                                                                 at<uint32_t>(E, L.big),
-                                                                                 &cnt->big_count);
     std::vector<Member> nm;
     for (const Member& M : PJ.members)
       nm.push_back(Member{M.vb + N0, M.n, M.sb + (uint32_t)W0, M.w, M.eb + (uint32_t)m0, M.m});
