@@ -2471,6 +2471,18 @@ __global__ void k_finalize(const unsigned long long* __restrict__ row0, const in
 // peeled with core k, and peeling it decrements each neighbour's degree only
 // while that degree exceeds k; a neighbour whose degree drops from k + 1 to k
 // joins the next sub-level.  The result does not depend on the order.
+//
+// The level loop runs on the device: one wave is either the scan of level k (live
+// vertices of degree <= k join the frontier, the smallest degree left is
+// recorded) or one sub-level, and the last block of each wave advances the state
+// (the next sub-level, the next level, or a jump past empty levels to the
+// smallest degree left) and sets the CUDA-graph loop condition.  Bounded by a
+// wave count and the device clock, like the PKT peel.
+//
+// A sub-level's work is the frontier's row entries, spread evenly over the warps
+// through each queue entry's work start: with a warp per frontier vertex one hub
+// row of 10^5 entries was 3,000 round trips of one warp (R-MAT-20 42 ms of
+// peel, 7.5 now).  Small waves run in one cluster (k_kcore_tail), as the PKT peel's do.
 __global__ void __launch_bounds__(256) k_kcore_init(const uint32_t* __restrict__ off, uint32_t n, int u8mode,
                                                     uint32_t* __restrict__ deg, uint32_t* __restrict__ alive,
                                                     uint32_t* __restrict__ core,
@@ -2483,105 +2495,21 @@ __global__ void __launch_bounds__(256) k_kcore_init(const uint32_t* __restrict__
     core[u] = 0;
     live += d != 0;
   }
-#pragma unroll
-  for (int d = 16; d > 0; d >>= 1) live += __shfl_xor_sync(kFull, live, d);
+  live = __reduce_add_sync(kFull, live);
   if (lane_id() == 0 && live) atomicAdd(remaining, (unsigned long long)live);
 }
 
-// Level k: live vertices with degree <= k form the first sub-level; the
-// smallest degree left is recorded so that empty levels are skipped.
-__global__ void __launch_bounds__(256) k_kcore_scan(const uint32_t* __restrict__ deg, uint32_t* __restrict__ alive,
-                                                    uint32_t n, uint32_t k, uint32_t* __restrict__ frontier,
-                                                    uint32_t* __restrict__ count, uint32_t* __restrict__ min_left) {
-  const uint32_t lane = lane_id();
-  uint32_t mn = 0xFFFFFFFFu;
-  for (uint32_t b = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; b < n; b += gridDim.x * blockDim.x) {
-    const uint32_t u = b + lane;
-    bool take = false;
-    if (u < n && alive[u]) {
-      const uint32_t d = deg[u];
-      if (d <= k) {
-        take = true;
-        alive[u] = 0;
-      } else {
-        mn = min(mn, d);
-      }
-    }
-    const unsigned bal = __ballot_sync(kFull, take);
-    if (bal) {
-      uint32_t at = 0;
-      if (lane == 0) at = atomicAdd(count, (uint32_t)__popc(bal));
-      at = __shfl_sync(kFull, at, 0);
-      if (take) frontier[at + __popc(bal & ((1u << lane) - 1))] = u;
-    }
-  }
-#pragma unroll
-  for (int d = 16; d > 0; d >>= 1) mn = min(mn, __shfl_xor_sync(kFull, mn, d));
-  if (lane == 0 && mn != 0xFFFFFFFFu) atomicMin(min_left, mn);
-}
-
-// One sub-level: a warp per frontier vertex.  The decrement-while-above-k is a
-// compare-and-swap loop; each failed swap means the degree dropped, so the
-// loop ends after at most (degree - k) tries.
-__global__ void __launch_bounds__(256) k_kcore_peel(const uint32_t* __restrict__ off,
-                                                    const uint32_t* __restrict__ nbr,
-                                                    const uint32_t* __restrict__ frontier, uint32_t count,
-                                                    uint32_t k, uint32_t* __restrict__ deg,
-                                                    uint32_t* __restrict__ alive, uint32_t* __restrict__ core,
-                                                    uint32_t* __restrict__ next, uint32_t* __restrict__ next_count) {
-  const uint32_t lane = lane_id();
-  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t i = warp; i < count; i += nwarps) {
-    const uint32_t u = frontier[i];
-    if (lane == 0) core[u] = k;
-    const uint32_t b = __ldg(off + u), e = __ldg(off + u + 1);
-    for (uint32_t s0 = b; s0 < e; s0 += 32) {
-      const uint32_t s = s0 + lane;
-      bool push = false;
-      uint32_t v = 0;
-      if (s < e) {
-        v = __ldg(nbr + s);
-        uint32_t x = *(volatile uint32_t*)(deg + v);
-        while (x > k) {
-          const uint32_t old = atomicCAS(deg + v, x, x - 1);
-          if (old == x) {
-            push = x == k + 1 && atomicExch(alive + v, 0u) == 1u;
-            break;
-          }
-          x = old;
-        }
-      }
-      const unsigned bal = __ballot_sync(kFull, push);
-      if (bal) {
-        uint32_t at = 0;
-        if (lane == 0) at = atomicAdd(next_count, (uint32_t)__popc(bal));
-        at = __shfl_sync(kFull, at, 0);
-        if (push) next[at + __popc(bal & ((1u << lane) - 1))] = v;
-      }
-    }
-  }
-}
-
-// ---------------------------------------------------------------------------
-// The k-core level loop on the device: one wave kernel runs either the scan of
-// level k (live vertices of degree <= k join the frontier, the smallest degree
-// left is recorded) or one sub-level (a warp per frontier vertex, as
-// k_kcore_peel); the last block of each wave advances the state (the next
-// sub-level, the next level, or a jump past empty levels to the smallest degree
-// left) and sets the CUDA-graph loop condition.  Bounded by a wave count and
-// the device clock, like the PKT peel.
 struct KcState {
   uint32_t phase;        // 0 scan, 1 sub-level, 2 done
   uint32_t k;
-  uint32_t count;        // frontier size of the sub-level to run
-  uint32_t next_count;   // wave accumulator: frontier being built
   uint32_t min_left;     // wave accumulator (scan): smallest degree above k
   uint32_t sel;          // queue holding the frontier
   uint32_t levels, subs, kmax;
   uint32_t blocks_done;
   uint32_t err;
   uint32_t pad;
+  unsigned long long curr;       // frontier of the sub-level to run: vertices << 32 | row entries
+  unsigned long long next;       // wave accumulator: frontier being built
   unsigned long long remaining;  // live vertices
   unsigned long long waves_run, max_waves, t_start, timeout_ns;
 };
@@ -2589,8 +2517,8 @@ struct KcState {
 __global__ void k_kcore_start(KcState* st, unsigned long long max_waves, unsigned long long timeout_ns) {
   st->phase = st->remaining ? 0u : 2u;
   st->k = 1;
-  st->count = 0;
-  st->next_count = 0;
+  st->curr = 0;
+  st->next = 0;
   st->min_left = 0xFFFFFFFFu;
   st->sel = 0;
   st->max_waves = max_waves;
@@ -2598,119 +2526,171 @@ __global__ void k_kcore_start(KcState* st, unsigned long long max_waves, unsigne
   st->t_start = globaltimer();
 }
 
-__global__ void __launch_bounds__(256) k_kcore_wave(const uint32_t* __restrict__ off,
-                                                    const uint32_t* __restrict__ nbr, uint32_t n,
-                                                    uint32_t* __restrict__ deg, uint32_t* __restrict__ alive,
-                                                    uint32_t* __restrict__ core, uint32_t* __restrict__ q0,
-                                                    uint32_t* __restrict__ q1, KcState* st,
-                                                    cudaGraphConditionalHandle handle, int use_handle) {
-  const uint32_t phase = st->phase, k = st->k, sel = st->sel, count = st->count;
+struct KcArgs {
+  const uint32_t* off;
+  const uint32_t* nbr;
+  uint32_t n;
+  uint32_t* deg;
+  uint32_t* alive;
+  uint32_t* core;
+  unsigned long long* q0;  // queue entries: first row entry in the frontier << 32 | vertex
+  unsigned long long* q1;
+  KcState* st;
+  cudaGraphConditionalHandle handle;
+  int use_handle;
+};
+
+// The lanes that `take` put their vertex v (core k) into the frontier being built.
+__device__ __forceinline__ void kc_push(const KcArgs& a, unsigned long long* next, bool take, uint32_t v, uint32_t k) {
+  const unsigned bal = __ballot_sync(kFull, take);
+  if (!bal) return;
+  uint32_t len = 0;
+  if (take) {
+    a.alive[v] = 0;
+    a.core[v] = k;
+    len = __ldg(a.off + v + 1) - __ldg(a.off + v);
+  }
+  uint32_t incl = len;  // a frontier's entries stay below the slot count, 2^32
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t o = __shfl_up_sync(kFull, incl, d);
+    if (lane_id() >= (uint32_t)d) incl += o;
+  }
+  unsigned long long old = 0;
+  if (lane_id() == 31) old = atomicAdd(&a.st->next, ((unsigned long long)__popc(bal) << 32) | incl);
+  old = __shfl_sync(kFull, old, 31);
+  if (take)
+    next[(uint32_t)(old >> 32) + __popc(bal & ((1u << lane_id()) - 1))] =
+        ((unsigned long long)((uint32_t)old + incl - len) << 32) | v;
+}
+
+struct KcStart {
+  const unsigned long long* q;
+  __device__ __forceinline__ unsigned long long operator()(uint32_t x) const { return q[x] >> 32; }
+};
+
+// One wave's share of warp `warp` of `nwarps`.
+__device__ __forceinline__ void kc_work(const KcArgs& a, uint32_t phase, uint32_t k, uint32_t sel,
+                                        unsigned long long curr, uint32_t warp, uint32_t nwarps) {
   const uint32_t lane = lane_id();
   if (phase == 0) {
-    uint32_t* frontier = sel ? q1 : q0;
+    unsigned long long* frontier = sel ? a.q1 : a.q0;
     uint32_t mn = 0xFFFFFFFFu;
-    for (uint32_t b = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; b < n; b += gridDim.x * blockDim.x) {
-      const uint32_t u = b + lane;
+    for (unsigned long long b = 32ull * warp; b < a.n; b += 32ull * nwarps) {
+      const uint32_t u = (uint32_t)b + lane;
       bool take = false;
-      if (u < n && alive[u]) {
-        const uint32_t d = deg[u];
-        if (d <= k) {
-          take = true;
-          alive[u] = 0;
-        } else {
-          mn = min(mn, d);
-        }
+      if (b + lane < a.n && a.alive[u]) {
+        const uint32_t d = a.deg[u];
+        take = d <= k;
+        if (!take) mn = min(mn, d);
       }
-      const unsigned bal = __ballot_sync(kFull, take);
-      if (bal) {
-        uint32_t at = 0;
-        if (lane == 0) at = atomicAdd(&st->next_count, (uint32_t)__popc(bal));
-        at = __shfl_sync(kFull, at, 0);
-        if (take) frontier[at + __popc(bal & ((1u << lane) - 1))] = u;
-      }
+      kc_push(a, frontier, take, u, k);
     }
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) mn = min(mn, __shfl_xor_sync(kFull, mn, d));
-    if (lane == 0 && mn != 0xFFFFFFFFu) atomicMin(&st->min_left, mn);
+    mn = __reduce_min_sync(kFull, mn);
+    if (lane == 0 && mn != 0xFFFFFFFFu) atomicMin(&a.st->min_left, mn);
   } else if (phase == 1) {
-    const uint32_t* frontier = sel ? q1 : q0;
-    uint32_t* next = sel ? q0 : q1;
-    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t i = warp; i < count; i += nwarps) {
-      const uint32_t u = frontier[i];
-      if (lane == 0) core[u] = k;
-      const uint32_t b = __ldg(off + u), e = __ldg(off + u + 1);
-      for (uint32_t s0 = b; s0 < e; s0 += 32) {
-        const uint32_t s = s0 + lane;
-        bool push = false;
-        uint32_t v = 0;
-        if (s < e) {
-          v = __ldg(nbr + s);
-          uint32_t x = *(volatile uint32_t*)(deg + v);
-          while (x > k) {
-            const uint32_t old = atomicCAS(deg + v, x, x - 1);
-            if (old == x) {
-              push = x == k + 1 && atomicExch(alive + v, 0u) == 1u;
-              break;
-            }
-            x = old;
-          }
-        }
-        const unsigned bal = __ballot_sync(kFull, push);
-        if (bal) {
-          uint32_t at = 0;
-          if (lane == 0) at = atomicAdd(&st->next_count, (uint32_t)__popc(bal));
-          at = __shfl_sync(kFull, at, 0);
-          if (push) next[at + __popc(bal & ((1u << lane) - 1))] = v;
-        }
+    const unsigned long long* q = sel ? a.q1 : a.q0;
+    unsigned long long* next = sel ? a.q0 : a.q1;
+    const uint32_t count = (uint32_t)(curr >> 32), total = (uint32_t)curr;
+    // one chunk per warp, 32 consecutive entries per step
+    const unsigned long long ch = max(((total + nwarps - 1ull) / nwarps + 31) & ~31ull, 32ull);
+    if (warp * ch >= total || count == 0) return;
+    const uint32_t kend = (uint32_t)min((warp + 1) * ch, (unsigned long long)total);
+    uint32_t i = warp_last_le(KcStart{q}, 0, count - 1, warp * ch);
+    for (uint32_t j0 = (uint32_t)(warp * ch); j0 < kend; j0 += 32) {
+      // each lane's entry among the 32 from i on (every row has an entry)
+      const unsigned long long qv = i + lane < count ? q[i + lane] : ~0ull;
+      const uint32_t start = (uint32_t)(qv >> 32), j = j0 + lane;
+      uint32_t t = 0;
+#pragma unroll
+      for (int d = 16; d > 0; d >>= 1)
+        if (__shfl_sync(kFull, start, t + d) <= j) t += d;
+      const uint32_t u = __shfl_sync(kFull, (uint32_t)qv, t), at = __shfl_sync(kFull, start, t);
+      i += __shfl_sync(kFull, t, min(31u, kend - 1 - j0));
+      bool push = false;
+      uint32_t v = 0;
+      if (j < kend) {
+        v = __ldg(a.nbr + __ldg(a.off + u) + (j - at));
+        // a degree at or below k belongs to a peeled vertex or one of this
+        // level's: it is left alone.  Of the decrements that race past k + 1 one
+        // sees it, and the vertex is no longer live for the others.
+        if (*(volatile uint32_t*)(a.deg + v) > k) push = atomicSub(a.deg + v, 1u) == k + 1;
       }
+      kc_push(a, next, push, v, k);
     }
   }
+}
+
+// After a wave: the next one, or the end.  One thread.
+__device__ __forceinline__ bool kc_plan(KcState* st) {
+  const uint32_t phase = st->phase, k = st->k;
+  bool done = phase == 2;
+  if (done) return true;
+  const unsigned long long next = __ldcg(&st->next);
+  if (phase == 0) {
+    if (next) {
+      st->curr = next;
+      st->phase = 1;
+      st->levels += 1;
+      st->kmax = k;
+    } else {
+      const uint32_t ml = __ldcg(&st->min_left);
+      if (ml == 0xFFFFFFFFu) { st->err |= kErrInternal; done = true; }  // live vertices, none found
+      else st->k = max(k + 1, ml);
+    }
+  } else {
+    st->remaining -= min(st->remaining, st->curr >> 32);
+    st->subs += 1;
+    st->curr = next;
+    if (next) {
+      st->sel ^= 1u;
+    } else {
+      st->k = k + 1;
+      st->phase = 0;
+    }
+  }
+  st->next = 0;
+  st->min_left = 0xFFFFFFFFu;
+  st->waves_run += 1;
+  if (st->remaining == 0 && st->phase == 0) done = true;
+  if (st->waves_run > st->max_waves) { st->err |= kErrWaves; done = true; }
+  if (globaltimer() - st->t_start > st->timeout_ns) { st->err |= kErrTimeout; done = true; }
+  if (done) st->phase = 2;
+  return done;
+}
+
+__global__ void __launch_bounds__(256) k_kcore_wave(KcArgs a) {
+  kc_work(a, a.st->phase, a.st->k, a.st->sel, a.st->curr, (blockIdx.x * blockDim.x + threadIdx.x) >> 5,
+          (gridDim.x * blockDim.x) >> 5);
   // the last block to finish plans the next wave
   __shared__ uint32_t s_last;
   __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) s_last = atomicAdd(&st->blocks_done, 1u) == gridDim.x - 1;
+  if (threadIdx.x == 0) s_last = atomicAdd(&a.st->blocks_done, 1u) == gridDim.x - 1;
   __syncthreads();
   if (!s_last || threadIdx.x != 0) return;
   __threadfence();
-  st->blocks_done = 0;
-  uint32_t done = phase == 2;
-  if (!done) {
-    const uint32_t found = *(volatile uint32_t*)&st->next_count;
-    if (phase == 0) {
-      if (found) {
-        st->count = found;
-        st->phase = 1;
-        st->levels += 1;
-        st->kmax = k;
-      } else {
-        const uint32_t ml = *(volatile uint32_t*)&st->min_left;
-        if (ml == 0xFFFFFFFFu) { st->err |= kErrInternal; done = 1; }  // live vertices, none found
-        else st->k = max(k + 1, ml);
-      }
-    } else {
-      st->remaining -= min(st->remaining, (unsigned long long)count);
-      st->subs += 1;
-      if (found) {
-        st->count = found;
-        st->sel = sel ^ 1u;
-      } else {
-        st->count = 0;
-        st->k = k + 1;
-        st->phase = 0;
-      }
-    }
-    st->next_count = 0;
-    st->min_left = 0xFFFFFFFFu;
-    st->waves_run += 1;
-    if (st->remaining == 0 && st->phase == 0) done = 1;
-    if (st->waves_run > st->max_waves) { st->err |= kErrWaves; done = 1; }
-    if (globaltimer() - st->t_start > st->timeout_ns) { st->err |= kErrTimeout; done = 1; }
-    if (done) st->phase = 2;
+  a.st->blocks_done = 0;
+  const bool done = kc_plan(a.st);
+  if (a.use_handle) cudaGraphSetConditional(a.handle, done ? 0u : 1u);
+}
+
+// Small waves in one cluster (see k_wave_tail): sub-levels of at most `max_work`
+// row entries, and scans of graphs of at most that many vertices.
+__global__ void __launch_bounds__(kTailThreads, 1) k_kcore_tail(KcArgs a, uint32_t max_work) {
+  for (;;) {
+    const uint32_t phase = __ldcg(&a.st->phase), k = __ldcg(&a.st->k), sel = __ldcg(&a.st->sel);
+    const unsigned long long curr = __ldcg(&a.st->curr);
+    if (phase == 2 || (phase == 0 ? a.n : (uint32_t)curr) > max_work) break;
+    kc_work(a, phase, k, sel, curr, (threadIdx.x >> 5) * gridDim.x + blockIdx.x, (kTailThreads / 32) * gridDim.x);
+    __syncwarp();
+    cluster_barrier();
+    if (blockIdx.x == 0 && threadIdx.x == 0) kc_plan(a.st);
+    __syncwarp();
+    cluster_barrier();
   }
-  if (use_handle) cudaGraphSetConditional(handle, done ? 0u : 1u);
+  if (blockIdx.x == 0 && threadIdx.x == 0 && a.use_handle)
+    cudaGraphSetConditional(a.handle, __ldcg(&a.st->phase) == 2 ? 0u : 1u);
 }
 
 template <typename OutT>

@@ -270,6 +270,12 @@ struct PeelGraph {
   std::vector<size_t> key;
 };
 
+void drop_graph(PeelGraph& g) {
+  if (g.exec) cudaGraphExecDestroy(g.exec);
+  if (g.graph) cudaGraphDestroy(g.graph);
+  g = PeelGraph{};
+}
+
 struct Engine {
   int device = 0;
   int sm_count = 148;
@@ -282,6 +288,7 @@ struct Engine {
   cudaEvent_t tev[8] = {};
   void* pinned_small = nullptr;  // 4 KB for scalar read-backs
   PeelGraph peel;
+  PeelGraph kcore;            // the k-core level loop
   int wave_blocks = 0;        // k_wave<false> grid (resident blocks per SM x SMs)
   int wave_blocks_multi = 0;  // k_wave<true> grid (multigraphs)
   int tail_blocks = 0;        // k_wave_tail: blocks of its cluster (0: the device takes none)
@@ -298,6 +305,7 @@ struct Engine {
 // (16 to 48 thousand elements 13 us either way; R-MAT-12 3.83 / 3.61 / 3.49 ms at
 // a bound of 16, 32 and 48 thousand, R-MAT-19 and 22 within noise).
 constexpr unsigned long long kTailMaxWork = 49152;
+constexpr uint32_t kKcoreTailWork = 16384;  // the same for a k-core wave (R-MAT-20 7.53 / 7.58 / 7.91 / 8.52 ms at 16, 48, 128 thousand, 0)
 
 constexpr unsigned long long kTraceRecords = 1ull << 20;
 
@@ -306,8 +314,8 @@ std::map<int, Engine*> g_engines;
 
 // The small waves' cluster: one of 16 blocks, else of 8 (the portable size), on
 // the current device; 0 when neither can be resident.
-template <bool kMulti>
-cudaError_t launch_tail(int blocks, const WaveArgs& wa, cudaStream_t s) {
+template <class Kernel, class Args, class Bound>
+cudaError_t launch_cluster(Kernel kernel, int blocks, const Args& args, Bound bound, cudaStream_t s) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(blocks);
   cfg.blockDim = dim3(kTailThreads);
@@ -318,27 +326,30 @@ cudaError_t launch_tail(int blocks, const WaveArgs& wa, cudaStream_t s) {
   at.val.clusterDim.y = at.val.clusterDim.z = 1;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k_wave_tail<kMulti>, wa, kTailMaxWork);
+  return cudaLaunchKernelEx(&cfg, kernel, args, bound);
+}
+
+template <class Kernel>
+bool cluster_fits(Kernel kernel, int blocks) {
+  int clusters = 0;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(kTailThreads);
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = blocks;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+         cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters > 0;
 }
 
 int tail_cluster() {
-  for (int blocks : {16, 8}) {
-    int clusters = 0;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(blocks);
-    cfg.blockDim = dim3(kTailThreads);
-    cudaLaunchAttribute at = {};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = blocks;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    if (cudaFuncSetAttribute(k_wave_tail<false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-        cudaFuncSetAttribute(k_wave_tail<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-        cudaOccupancyMaxActiveClusters(&clusters, k_wave_tail<true>, &cfg) == cudaSuccess && clusters > 0 &&
-        cudaOccupancyMaxActiveClusters(&clusters, k_wave_tail<false>, &cfg) == cudaSuccess && clusters > 0)
+  for (int blocks : {16, 8})
+    if (cluster_fits(k_wave_tail<true>, blocks) && cluster_fits(k_wave_tail<false>, blocks) &&
+        cluster_fits(k_kcore_tail, blocks))
       return blocks;
-  }
   cudaGetLastError();
   return 0;
 }
@@ -386,11 +397,7 @@ int get_engine(int device, Engine** out) {
 
 int ensure_ws(Engine& E, size_t bytes, bool slack = true) {
   if (E.ws_cap >= bytes) return SPARX_OK;
-  if (E.peel.exec) {
-    cudaGraphExecDestroy(E.peel.exec);
-    cudaGraphDestroy(E.peel.graph);
-    E.peel = PeelGraph{};
-  }
+  drop_graph(E.peel);
   if (E.ws) { CU(cudaStreamSynchronize(E.stream)); CU(cudaFree(E.ws)); E.ws = nullptr; E.ws_cap = 0; }
   size_t cap = align_up(slack ? bytes + bytes / 8 : bytes, 1 << 21);
   cudaError_t e = cudaMalloc(&E.ws, cap);
@@ -741,11 +748,7 @@ int build_peel_graph(Engine& E, const UnionJob& J, const PeelArrays& arr) {
   const size_t* words = reinterpret_cast<const size_t*>(&arr);
   key.insert(key.end(), words, words + sizeof(PeelArrays) / sizeof(size_t));
   if (E.peel.exec && E.peel.key == key) return SPARX_OK;
-  if (E.peel.exec) {
-    cudaGraphExecDestroy(E.peel.exec);
-    cudaGraphDestroy(E.peel.graph);
-    E.peel = PeelGraph{};
-  }
+  drop_graph(E.peel);
   cudaGraph_t g;
   CU(cudaGraphCreate(&g, 0));
   cudaGraphConditionalHandle h;
@@ -773,7 +776,7 @@ int build_peel_graph(Engine& E, const UnionJob& J, const PeelArrays& arr) {
   // nothing, and the condition is read once per iteration
   for (int i = 0; i < kWavesPerIteration; ++i) {
     if (E.tail_blocks && i % kWavesPerTail == 0)
-      CU(arr.mu ? launch_tail<true>(E.tail_blocks, wa, E.capture) : launch_tail<false>(E.tail_blocks, wa, E.capture));
+      CU(launch_cluster(arr.mu ? k_wave_tail<true> : k_wave_tail<false>, E.tail_blocks, wa, kTailMaxWork, E.capture));
     if (arr.mu) k_wave<true><<<E.wave_blocks_multi, kWaveThreads, 0, E.capture>>>(wa);
     else k_wave<false><<<E.wave_blocks, kWaveThreads, 0, E.capture>>>(wa);
   }
@@ -1400,8 +1403,8 @@ Layout make_kcore_layout(uint64_t N, uint64_t W, size_t out_bytes) {
   L.dplus = take(4 * N);  // degree
   L.act0 = take(4 * N);   // live flag
   L.opos = take(4 * N);   // core
-  L.q0 = take(4 * N);     // frontier
-  L.q1 = take(4 * N);     // next frontier
+  L.q0 = take(8 * N);     // frontier
+  L.q1 = take(8 * N);     // next frontier
   L.out = take(out_bytes);
   L.stage0 = take(kStageBytes);
   L.stage1 = take(kStageBytes);
@@ -1411,10 +1414,41 @@ Layout make_kcore_layout(uint64_t N, uint64_t W, size_t out_bytes) {
   return L;
 }
 
-// Level loop of the k-core peel (liu_et_al.rs:295-420) on the device: a CUDA
-// graph whose WHILE node runs k_kcore_wave four times per iteration (the last
-// block of each wave plans the next and sets the condition), or host-launched
-// waves with SPARX_LOOP_HOST.
+// The k-core level loop's CUDA graph: a WHILE node whose body runs k_kcore_wave
+// four times, with the small waves' cluster before the first and the third.  Kept
+// for the next call with the same workspace arrays (building it took 0.4 ms).
+int build_kcore_graph(Engine& E, KcArgs ka, int wgrid) {
+  const std::vector<size_t> key = {(size_t)ka.off, (size_t)ka.nbr,  (size_t)ka.n,  (size_t)ka.deg,
+                                   (size_t)ka.alive, (size_t)ka.core, (size_t)ka.q0, (size_t)ka.q1, (size_t)ka.st};
+  if (E.kcore.exec && E.kcore.key == key) return SPARX_OK;
+  drop_graph(E.kcore);
+  cudaGraph_t g;
+  CU(cudaGraphCreate(&g, 0));
+  E.kcore.graph = g;  // freed with the engine, whatever fails below
+  CU(cudaGraphConditionalHandleCreate(&ka.handle, g, 1, cudaGraphCondAssignDefault));
+  ka.use_handle = 1;
+  cudaGraphNodeParams cp = {};
+  cp.type = cudaGraphNodeTypeConditional;
+  cp.conditional.handle = ka.handle;
+  cp.conditional.type = cudaGraphCondTypeWhile;
+  cp.conditional.size = 1;
+  cudaGraphNode_t node;
+  CU(cudaGraphAddNode(&node, g, nullptr, 0, &cp));
+  cudaGraph_t body = cp.conditional.phGraph_out[0];
+  CU(cudaStreamBeginCaptureToGraph(E.capture, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
+  for (int i = 0; i < 4; ++i) {
+    if (E.tail_blocks && i % 2 == 0) CU(launch_cluster(k_kcore_tail, E.tail_blocks, ka, kKcoreTailWork, E.capture));
+    k_kcore_wave<<<wgrid, 256, 0, E.capture>>>(ka);
+  }
+  cudaGraph_t captured;
+  CU(cudaStreamEndCapture(E.capture, &captured));
+  CU(cudaGraphInstantiate(&E.kcore.exec, g, 0));
+  E.kcore.key = key;
+  return SPARX_OK;
+}
+
+// Level loop of the k-core peel (liu_et_al.rs:295-420) on the device, or
+// host-launched waves with SPARX_LOOP_HOST.
 int run_kcore(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
   const Layout& L = J.L;
   const uint32_t N = (uint32_t)J.N;
@@ -1429,8 +1463,8 @@ int run_kcore(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
   uint32_t* deg = at<uint32_t>(E, L.dplus);
   uint32_t* alive = at<uint32_t>(E, L.act0);
   uint32_t* core = at<uint32_t>(E, L.opos);
-  uint32_t* qa = at<uint32_t>(E, L.q0);
-  uint32_t* qb = at<uint32_t>(E, L.q1);
+  unsigned long long* qa = at<unsigned long long>(E, L.q0);
+  unsigned long long* qb = at<unsigned long long>(E, L.q1);
   KcState* kst = at<KcState>(E, L.tiles);
   const int u8 = O.support_mode == SPARX_SUPPORT_U8;
   const int vgrid = grid_for(N, 256, E.sm_count * 16);
@@ -1441,46 +1475,17 @@ int run_kcore(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
   k_kcore_start<<<1, 1, 0, s>>>(kst, 3ull * N + 2 * J.W + 64, O.timeout_ms * 1000000ull);
   J.launches += 2;
   CU(cudaEventRecord(E.tev[4], s));
+  KcArgs ka{J.off, J.nbr, N, deg, alive, core, qa, qb, kst, cudaGraphConditionalHandle{}, 0};
   const int wgrid = E.sm_count * 8;
   if (O.loop == SPARX_LOOP_GRAPH) {
-    cudaGraph_t g;
-    CU(cudaGraphCreate(&g, 0));
-    cudaGraphConditionalHandle h;
-    CU(cudaGraphConditionalHandleCreate(&h, g, 1, cudaGraphCondAssignDefault));
-    cudaGraphNodeParams cp = {};
-    cp.type = cudaGraphNodeTypeConditional;
-    cp.conditional.handle = h;
-    cp.conditional.type = cudaGraphCondTypeWhile;
-    cp.conditional.size = 1;
-    cudaGraphNode_t node;
-    CU(cudaGraphAddNode(&node, g, nullptr, 0, &cp));
-    cudaGraph_t body = cp.conditional.phGraph_out[0];
-    CU(cudaStreamBeginCaptureToGraph(E.capture, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
-    for (int i = 0; i < 4; ++i)
-      k_kcore_wave<<<wgrid, 256, 0, E.capture>>>(J.off, J.nbr, N, deg, alive, core, qa, qb, kst, h, 1);
-    cudaGraph_t captured;
-    CU(cudaStreamEndCapture(E.capture, &captured));
-    cudaGraphExec_t ex;
-    cudaError_t ie = cudaGraphInstantiate(&ex, g, 0);
-    if (ie != cudaSuccess) {
-      cudaGraphDestroy(g);
-      set_error(std::string("k-core graph: ") + cudaGetErrorString(ie));
-      return SPARX_E_CUDA;
-    }
-    const cudaError_t le = cudaGraphLaunch(ex, s);
-    const cudaError_t se = cudaStreamSynchronize(s);
-    cudaGraphExecDestroy(ex);
-    cudaGraphDestroy(g);
-    if (le != cudaSuccess || se != cudaSuccess) {
-      set_error(std::string("k-core loop: ") + cudaGetErrorString(le != cudaSuccess ? le : se));
-      return SPARX_E_CUDA;
-    }
+    int rc = build_kcore_graph(E, ka, wgrid);
+    if (rc) return rc;
+    CU(cudaGraphLaunch(E.kcore.exec, s));
+    CU(cudaStreamSynchronize(s));
   } else {
     KcState* h = (KcState*)E.pinned_small;
     for (;;) {
-      for (int i = 0; i < 16; ++i)
-        k_kcore_wave<<<wgrid, 256, 0, s>>>(J.off, J.nbr, N, deg, alive, core, qa, qb, kst,
-                                           cudaGraphConditionalHandle{}, 0);
+      for (int i = 0; i < 16; ++i) k_kcore_wave<<<wgrid, 256, 0, s>>>(ka);
       J.launches += 16;
       CU(cudaMemcpyAsync(h, kst, sizeof(KcState), cudaMemcpyDeviceToHost, s));
       CU(cudaStreamSynchronize(s));
@@ -1955,7 +1960,8 @@ void engine_release(Engine* E) {
   if (!E) return;
   cudaSetDevice(E->device);
   if (E->stream) cudaStreamSynchronize(E->stream);
-  if (E->peel.exec) { cudaGraphExecDestroy(E->peel.exec); cudaGraphDestroy(E->peel.graph); }
+  drop_graph(E->peel);
+  drop_graph(E->kcore);
   if (E->ws) cudaFree(E->ws);
   if (E->ws2) cudaFree(E->ws2);
   if (E->ws3) cudaFree(E->ws3);
