@@ -59,7 +59,7 @@ typedef struct sparx_pkt_opts {
   uint32_t out_bits;       /* 8 (reference layout) or 32 */
   int32_t device;          /* CUDA ordinal; -1 = current device */
   uint32_t loop;           /* SPARX_LOOP_GRAPH | SPARX_LOOP_HOST */
-  uint32_t support_kernel; /* 0 = auto, 1 = balanced binary search, 2 = vertex hash */
+  uint32_t support_kernel; /* 0 = auto, 1 = balanced, 2 = vertex hash */
   uint64_t timeout_ms;     /* device budget for the peel; 0 = 600000 */
 } sparx_pkt_opts;
 
@@ -242,7 +242,8 @@ typedef struct sparx_tuning {
                                of at least this degree, >= 256, or 0 for none (1024) */
   uint32_t sample_min;      /* support: longer out-lists of at least this length (8 at least) are
                                searched through a rank index, shorter ones by binary search (64) */
-  uint32_t support_kernel;  /* 1 balanced edge form, 2 vertex form (1; 2 for keys with no
+  uint32_t support_kernel;  /* 1 edge form (balanced, or a thread per edge where every list is
+                               short), 2 vertex form (1; 2 for keys with no
                                slots in rows of degree >= 256 and a largest degree of 64..255,
                                which is what sparx_tuning_lookup reports for such a key) */
   uint32_t compact_pct;     /* peel: rebuild the working rows once live entries fill at most

@@ -79,7 +79,6 @@ struct Tuning {
 
 // Degree-distribution signature: log2 of the slot count, log2 bucket of the
 // largest degree, and the share (in eighths) of slots in rows of degree >= 256.
-// hist_cnt[b] / hist_slots[b]: vertices / slots with degree in [2^(b-1), 2^b).
 struct TuneKey {
   uint32_t log_w = 0, log_dmax = 0, skew8 = 0;
   bool operator<(const TuneKey& o) const {
@@ -87,15 +86,11 @@ struct TuneKey {
   }
 };
 
-TuneKey tune_key(const uint32_t* hist_cnt, const unsigned long long* hist_slots, uint64_t W) {
+// dmax: the largest degree; heavy: slots in rows of degree >= kHeavyRow, of `total`.
+TuneKey tune_key(uint32_t dmax, unsigned long long heavy, unsigned long long total, uint64_t W) {
   TuneKey k;
   k.log_w = W ? 63 - __builtin_clzll(W) : 0;
-  unsigned long long heavy = 0, total = 0;
-  for (int b = 1; b <= 32; ++b) {
-    if (hist_cnt[b]) k.log_dmax = (uint32_t)b;
-    total += hist_slots[b];
-    if (b >= 9) heavy += hist_slots[b];
-  }
+  k.log_dmax = dmax ? 32 - __builtin_clz(dmax) : 0;
   k.skew8 = total ? (uint32_t)std::min<unsigned long long>(7, 8 * heavy / total) : 0;
   return k;
 }
@@ -160,8 +155,9 @@ int tune_save_locked(const char* path) {
 // The tuning a launch uses: the autotuner's candidate, else the cached choice
 // for the key (the file named by SPARX_TUNE_FILE is read on first use), else
 // the key's defaults.
-Tuning resolve_tuning(const TuneKey& key) {
+Tuning resolve_tuning(const TuneKey& key, bool* tuned = nullptr) {
   Tuning t = default_tuning(key);
+  bool found = g_tune_force != nullptr;
   if (g_tune_force) {
     t = *g_tune_force;
   } else {
@@ -172,8 +168,10 @@ Tuning resolve_tuning(const TuneKey& key) {
       if (path && *path) tune_load_locked(path);
     }
     auto it = g_tune.find(key);
-    if (it != g_tune.end()) t = it->second;
+    found = it != g_tune.end();
+    if (found) t = it->second;
   }
+  if (tuned) *tuned = found;
   g_tune_last = t;
   g_tune_last_key = key;
   return t;
@@ -192,6 +190,10 @@ struct Counters {  // device scalars
   uint32_t hub_count;    // rows given the finer rank index
   uint32_t big_count;    // rows oriented by a block each
   uint32_t fin_err;      // served unions: error flags of one member's finalize
+  uint32_t dmax;         // largest degree
+  uint32_t pad;
+  unsigned long long heavy;  // slots in rows of degree >= kHeavyRow
+  unsigned long long elements;  // support (pair form): shorter-list entries
   uint32_t table_big;    // rank index, hash tables: what is listed for whole blocks
   double cc_possible;    // clustering: sum of d(d - 1)/2 over vertices
   double cc_local;       //             sum of local coefficients
@@ -207,7 +209,6 @@ struct Layout {
   size_t alive;                   // compaction: one bit per edge, set while it is unprocessed
   size_t kept, before;            // compaction: kept slots as a bitmap, and counted before each of its words
   size_t big;                     // rows longer than kWarpRow (a block each)
-  size_t hub_hist;                // the degree signature's histogram
   size_t tiles, ctl, mem, st, wpref, cnt, mem_tri, mem_maxsup, uni;
   size_t total;
 };
@@ -244,7 +245,6 @@ Layout make_layout(uint64_t N, uint64_t W, uint32_t G, bool own_nbr, size_t out_
   L.kept = take(4 * ((W + 31) / 32));
   L.before = take(4 * ((W + 31) / 32));
   L.big = take(4 * (W / kWarpRow + 1));
-  L.hub_hist = take(4 * 34 + 8 * 34);  // vertices, then slots, per log2 degree (the tuning key)
   L.vinfo = take(8ull * N);
   L.stage0 = take(kStageBytes);
   L.stage1 = take(kStageBytes);
@@ -551,6 +551,7 @@ void exclusive_scan(F f, unsigned long long count, T* out, T* tiles, T* grand, c
 // The vertex form needs a shared-memory table of 2x the largest out-degree;
 // beyond what a CTA can hold the balanced form runs instead.
 constexpr size_t kHeavySmemLimit = 160u << 10;
+constexpr uint64_t kPairEdges = 1ull << 24;  // 64 MB of oriented lists
 
 // What the balanced form needs besides the oriented lists.  The rank index of
 // the lists of at least `rank_min` entries lives in arrays the peel fills
@@ -584,6 +585,15 @@ int launch_support(int sm_count, uint32_t support_kernel, uint32_t n, uint64_t m
                                                      &cnt->hcursor, slots, max_dplus);
     *launches += 2;
     *support_elements = 0;
+    return SPARX_OK;
+  }
+  // 0: no list is longer than a thread walks
+  if (support_kernel == 0) {
+    const int g = grid_for(m, 256, sm_count * 32);
+    if (mu) k_support_pairs<true><<<g, 256, 0, s>>>(opos, ocol, osrc, (uint32_t)m, es, &cnt->tri, &cnt->elements, mu);
+    else k_support_pairs<false><<<g, 256, 0, s>>>(opos, ocol, osrc, (uint32_t)m, es, &cnt->tri, &cnt->elements, mu);
+    *launches += 1;
+    CU(cudaMemcpyAsync(support_elements, &cnt->elements, 8, cudaMemcpyDeviceToHost, s));
     return SPARX_OK;
   }
   if (X.hdr) {
@@ -906,8 +916,6 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
     if (*herr) { J.err = *herr; return status_from_flags(*herr); }
   }
   // -- orientation (Kernel B) --
-  uint32_t* hub_hist = at<uint32_t>(E, L.hub_hist);  // degree signature (tuning key)
-  unsigned long long* hub_hist_slots = reinterpret_cast<unsigned long long*>(hub_hist + 34);
   uint32_t* big = at<uint32_t>(E, L.big);
   // multigraphs: deduplicated rows, copies per slot, caller slot -> slot and
   // multiplicity per edge id (in the second workspace), filled by pass 0
@@ -917,15 +925,16 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
   uint32_t* mu = nullptr;
   Counters hc;
   uint32_t m32 = 0;
-  uint32_t hist[34] = {};
-  unsigned long long hist_slots[34] = {};
   for (int pass = 0;; ++pass) {
-    CU(cudaMemsetAsync(hub_hist, 0, 4 * 34 + 8 * 34, s));
-    k_hub_hist<<<grid_for(N, 256, E.sm_count * 4), 256, 0, s>>>(J.off, N, hub_hist, hub_hist_slots);
+    // the degree signature, and the rows the orientation gives a block each
+    if (pass > 0) {
+      CU(cudaMemsetAsync(&cnt->big_count, 0, 4, s));
+      CU(cudaMemsetAsync(&cnt->heavy, 0, 8, s));
+      CU(cudaMemsetAsync(&cnt->dmax, 0, 4, s));
+    }
+    k_degree_stats<<<grid_for(N, 256, E.sm_count * 8), 256, 0, s>>>(J.off, N, big, &cnt->big_count, &cnt->dmax,
+                                                                    &cnt->heavy);
     J.launches += 1;
-    // rows the orientation gives a block each
-    CU(cudaMemsetAsync(&cnt->big_count, 0, 4, s));
-    k_big_rows<<<grid_for(N, 256, E.sm_count * 8), 256, 0, s>>>(J.off, N, big, &cnt->big_count);
     k_orient_count<<<vgrid, 256, 0, s>>>(J.off, J.nbr, N, dplus, &cnt->self_loops, err, &cnt->max_dplus, big,
                                          &cnt->big_count);
     J.launches += 1;
@@ -937,13 +946,11 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
     CU(cudaMemcpyAsync(J.members.data(), dmem, sizeof(Member) * G, cudaMemcpyDeviceToHost, s));
     CU(cudaMemcpyAsync(&hc, cnt, sizeof(Counters), cudaMemcpyDeviceToHost, s));
     CU(cudaMemcpyAsync(&m32, opos + N, 4, cudaMemcpyDeviceToHost, s));
-    CU(cudaMemcpyAsync(hist, hub_hist, 4 * 34, cudaMemcpyDeviceToHost, s));
-    CU(cudaMemcpyAsync(hist_slots, hub_hist_slots, 8 * 34, cudaMemcpyDeviceToHost, s));
     CU(cudaStreamSynchronize(s));
     if (pass == 0) J.slot_self_loops = hc.self_loops;
     // (batched unions: the packer counted the relabelled copy in their budget)
     if (pass == 0 && hc.err == 0 && N > 1 && W > 0 && !J.support_only && !J.prep_only && !J.hook &&
-        resolve_tuning(tune_key(hist, hist_slots, W)).relabel) {
+        resolve_tuning(tune_key(hc.dmax, hc.heavy, W, W)).relabel) {
       // a sound simple graph: orient its degree-ordered copy instead (when the
       // device has no room for the copy, the caller's ids are used as they are)
       int rc = relabel_graph(E, J, N, W, big, &cnt->big_count, s);
@@ -992,7 +999,8 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
   if (2 * m + hc.self_loops != Ws) { J.err = kErrAsym; return SPARX_E_INVALID_CSR; }
   for (const Member& M : J.members)
     if (M.m > kEidMask) { set_error("a graph has >= 2^28 edges"); return SPARX_E_TOO_LARGE; }
-  const Tuning T = resolve_tuning(tune_key(hist, hist_slots, Ws));
+  bool tuned = false;
+  const Tuning T = resolve_tuning(tune_key(hc.dmax, hc.heavy, Ws, Ws), &tuned);
   J.tuning = T;
   // the support pass's rank index, in arrays that are idle until the peel
   // (4-entry lists cannot fill a word's 32 buckets: 8 at least)
@@ -1036,10 +1044,7 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
   const uint32_t rank_min = T.hash_min_degree ? std::max<uint32_t>(T.hash_min_degree / 4, 8) : kInvalid;
   uint32_t sup_hash_min = 0;
   {
-    uint32_t dmax_log = 0;  // largest degree < 2^dmax_log
-    for (uint32_t b = 1; b <= 32; ++b)
-      if (hist[b]) dmax_log = b;
-    const bool any_row = dmax_log >= 32 || (1ull << dmax_log) > std::min(rank_min, fine_min ? fine_min : kInvalid);
+    const bool any_row = hc.dmax >= std::min(rank_min, fine_min ? fine_min : kInvalid);
     bool index = any_row && !J.support_only && !J.prep_only && (!J.hook || J.hook_hash) && Ws < (1ull << 30) && Ws;
     bool sup_hash = T.sup_hash_min && m > 0 && m < (1ull << 28);
     const uint64_t Mx = std::max<uint64_t>(W / 2, 1);
@@ -1075,7 +1080,15 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
   // -- support (Kernel C) --
   CU(cudaMemsetAsync(es, 0, 8 * std::max<uint64_t>(m, 1), s));
   {
-    int rc = launch_support(E.sm_count, O.support_kernel ? O.support_kernel : T.support_kernel, N, m,
+    // Short lists take the pair form instead of the balanced one (a call's own
+    // choice of form and a tuned hash floor stand), and instead of a default
+    // vertex form while the lists fit the L2: ER n = 10^5, m = 2 M support 0.48 ->
+    // 0.20 ms, n = 10^6, m = 20 M 1.89 -> 1.85, but n = 4.2 M, m = 67 M 5.4 -> 8.4.
+    uint32_t form = O.support_kernel ? O.support_kernel : T.support_kernel;
+    if (!O.support_kernel && !sup_hash_min && hc.max_dplus <= kPairList &&
+        (form == 1 || (!tuned && m <= kPairEdges)))
+      form = 0;
+    int rc = launch_support(E.sm_count, form, N, m,
                             hc.max_dplus, opos, ocol, osrc, es, at<unsigned long long>(E, L.q0),
                             at<unsigned long long>(E, L.tiles), cnt, at<uint32_t>(E, L.act0), s, &J.launches,
                             &J.support_elements, X, mu, spool, sup_hash_min);
@@ -2900,16 +2913,16 @@ int sparx_tuning_default(sparx_tuning* t) {
 
 int sparx_tuning_signature(const uint64_t* offsets, uint64_t n_plus_1, uint32_t key[3]) {
   if (!offsets || !key || n_plus_1 < 1) return SPARX_E_ARG;
-  uint32_t cnt[34] = {};
-  unsigned long long slots[34] = {};
+  uint32_t dmax = 0;
+  unsigned long long heavy = 0, total = 0;
   for (uint64_t u = 0; u + 1 < n_plus_1; ++u) {
     const uint64_t d = offsets[u + 1] - offsets[u];
     if (!d || d > 0xFFFFFFFFull) continue;
-    const int b = 32 - __builtin_clz((uint32_t)d);
-    cnt[b]++;
-    slots[b] += d;
+    dmax = std::max(dmax, (uint32_t)d);
+    total += d;
+    if (d >= kHeavyRow) heavy += d;
   }
-  const TuneKey k = tune_key(cnt, slots, offsets[n_plus_1 - 1] - offsets[0]);
+  const TuneKey k = tune_key(dmax, heavy, total, offsets[n_plus_1 - 1] - offsets[0]);
   key[0] = k.log_w;
   key[1] = k.log_dmax;
   key[2] = k.skew8;
@@ -3412,7 +3425,7 @@ int run_noalloc(const uint64_t* d_offsets, uint64_t n_plus_1, const uint32_t* d_
 
   const int vgrid = grid_for(N, 256, sm * 32);  // row kernels: 32 vertices per warp
   uint32_t* big = (uint32_t*)P(L.big);  // big_count was cleared with the counters above
-  k_big_rows<<<grid_for(N, 256, sm * 8), 256, 0, s>>>(off, N, big, &cnt->big_count);
+  k_degree_stats<<<grid_for(N, 256, sm * 8), 256, 0, s>>>(off, N, big, &cnt->big_count, &cnt->dmax, &cnt->heavy);
   k_orient_count<<<vgrid, 256, 0, s>>>(off, d_nbr, N, dplus, &cnt->self_loops, err, &cnt->max_dplus, big,
                                        &cnt->big_count);
   exclusive_scan<uint32_t>(LoadU32{dplus}, N, opos, (uint32_t*)P(L.tiles), (uint32_t*)&cnt->grand, s);
@@ -3452,7 +3465,7 @@ int run_noalloc(const uint64_t* d_offsets, uint64_t n_plus_1, const uint32_t* d_
   {
     uint32_t launches = 0;
     unsigned long long elements = 0;
-    rc = launch_support(sm, 0, N, m, hc.max_dplus, opos, ocol, osrc, es, (unsigned long long*)P(L.q0),
+    rc = launch_support(sm, hc.max_dplus <= kPairList ? 0 : 1, N, m, hc.max_dplus, opos, ocol, osrc, es, (unsigned long long*)P(L.q0),
                         (unsigned long long*)P(L.tiles), cnt, (uint32_t*)P(L.act0), s, &launches, &elements, X);
     if (rc) return rc;
   }
