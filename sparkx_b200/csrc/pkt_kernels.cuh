@@ -1670,10 +1670,12 @@ struct QueueStart {
 // row descriptors of the staged edges are looked up at publication, all lanes
 // at once, so those dependent loads stay off the per-iteration path.
 constexpr int kPushBuf = 64;
-constexpr int kWaveThreads = 256;
-#ifndef SPARX_WAVE_MINB
-#define SPARX_WAVE_MINB 7  // resident 256-thread blocks per SM the register budget targets
-#endif
+constexpr int kWaveThreads = 128;
+// Resident blocks per SM, which sets the register budget (40): with the found
+// triangles staged the search no longer needs the last 16 warps an SM holds, and
+// spills less.  R-MAT-22 285.9 / 284.8 ms, R-MAT-19 47.0 / 48.4, R-MAT-16 15.2 / 16.4
+// at 48 / 64 warps per SM.
+constexpr int kWaveBlocksPerSm = 12;
 constexpr int kWaveWarps = kWaveThreads / 32;
 constexpr int kTailThreads = 512;  // threads per block of the small waves' cluster (1024: R-MAT-12 6% slower)
 // slots of the per-warp loop state in shared memory (k_wave)
@@ -1683,11 +1685,10 @@ enum : int { kCtxEb = 0, kCtxM, kCtxLevel, kCtxQsel, kCtxQcount, kCtxSegLen, kCt
 // place: every kept entry of a large scan goes through one counter per member
 constexpr int kKeepBuf = 256;
 // A run of at least kWaveRun elements of one frontier edge goes kWaveWays groups
-// of 32 at a time, their row entries, index words, found entries and states
-// loaded side by side: the wave waits for memory (19 long-scoreboard stall
-// cycles per issue in a large wave, DRAM at 28%), so loads in flight count most
-// (R-MAT-22's peel 277 ms with one group, 257 with two; 272 / 285 ms with two
-// groups at 6 / 5 blocks per SM instead of 8).
+// of 32 at a time, their row entries, index words and found entries loaded side
+// by side: the wave waits for memory (19 long-scoreboard stall cycles per issue in
+// a large wave, DRAM at 28%), so loads in flight count (R-MAT-22's peel 277 ms
+// with one group, 257 with two; three and four spill, 233 and 241 against 231).
 constexpr int kWaveWays = 2;
 constexpr uint32_t kWaveRun = 24;
 
@@ -2062,10 +2063,13 @@ __device__ __noinline__ void wave_scan_segment(const Union* Up, MemberState* st,
 // R-MAT-22's peel 315 -> 257 ms, its first large wave 0.87 -> 0.68 ms on R-MAT-20
 // with 0.60 -> 0.36 G instructions and 2.7 -> 1.4 GB read.  The index is rebuilt
 // with the rows at every compaction, so it shrinks with what is left.
+constexpr int kHitBuf = 64;  // found triangles staged per warp: fewer than 32, and 32 of a group
+
 template <int kWarps>
 struct WaveShared {
   uint32_t push_eid[kWarps][kPushBuf];
   uint32_t keep[kWarps][kKeepBuf];
+  uint32_t hit_e[kWarps][kHitBuf], hit_f[kWarps][kHitBuf], hit_h[kWarps][kHitBuf];
   // work counters (per warp: hits, groups of 32 elements inside one edge, groups
   // over several edges), here rather than in registers held across the loop;
   // lane 0 adds to them
@@ -2137,7 +2141,25 @@ __device__ __forceinline__ void wave_work(const WaveArgs& a, WaveShared<kWarps>&
         }
         __syncwarp();
         uint32_t i = i0;
-        uint32_t found = 0;
+        uint32_t found = 0, nhit = 0;
+        // the rule for hits [at, at + 32) of the stage, lanes in `on`
+        auto resolve = [&](uint32_t at, unsigned on) {
+          bool pf = false, ph = false;
+          uint32_t rf = 0, rh = 0;
+          if (on >> lane & 1) {
+            const uint32_t re = sh.hit_e[wib][at + lane];
+            rf = sh.hit_f[wib][at + lane];
+            rh = sh.hit_h[wib][at + lane];
+            const int2 s_f = U.es[rf], s_h = U.es[rh];
+            pkt_rule<kMulti>(U, re, rf, s_f, rh, s_h, w32[kCtxLevel], w32[kCtxW], pf, ph);
+          }
+          if (__any_sync(kFull, pf || ph)) {
+            push_edge(ps, U, a.Up, w32[kCtxEb], w32[kCtxM], a.st + w32[kCtxG], a.err, w32[kCtxQsel], pf, rf,
+                      w32[kCtxW]);
+            push_edge(ps, U, a.Up, w32[kCtxEb], w32[kCtxM], a.st + w32[kCtxG], a.err, w32[kCtxQsel], ph, rh,
+                      w32[kCtxW]);
+          }
+        };
         for (uint32_t r = 0; r < w32[kCtxSegLen];) {
           const uint32_t seg_len = w32[kCtxSegLen];
           const uint32_t qcount = w32[kCtxQcount];
@@ -2195,7 +2217,8 @@ __device__ __forceinline__ void wave_work(const WaveArgs& a, WaveShared<kWarps>&
           // rows may have been compacted since the entry's work was counted
           o_end = valid ? min(o_end, dsc.y) : 0u;
           const unsigned long long* words = U.rpool + dsc.z;
-          const uint32_t sh = rank_shift(dsc.w - dsc.z, hq.y);
+          const uint32_t shift = rank_shift(dsc.w - dsc.z, hq.y);
+          hq.y &= ~kRankFine;
           // warp-uniform trips: all lanes of a run share o_end; otherwise one trip
           const uint32_t o0 = o - lane;
           for (uint32_t og = 0; run ? o0 + og < o_end : og == 0; og += 32 * kWaveWays, o += 32 * kWaveWays) {
@@ -2206,25 +2229,26 @@ __device__ __forceinline__ void wave_work(const WaveArgs& a, WaveShared<kWarps>&
               en[j] = o + 32 * j < o_end ? __ldg(U.row + dsc.x + o + 32 * j) : ~0ull;
               h[j] = kInvalid;
             }
+            // f == kInvalid: a self-loop entry.  The frontier edge's own entry needs
+            // no check: its name is the longer row's vertex, which that row holds
+            // only as a self-loop (h == kInvalid).
             if (hq.y) {
               // the longer row's rank index: its words, then its entries, side by side
+              uint32_t bk[kWaveWays];
 #pragma unroll
               for (int j = 0; j < kWaveWays; ++j) {
                 w[j] = (uint32_t)en[j];
                 f[j] = (uint32_t)(en[j] >> 32);
-                // f == kInvalid: a self-loop entry; f == e: the frontier edge itself
-                const bool look = f[j] != kInvalid && f[j] != e;
-                en[j] = look ? __ldg(words + (rank_bucket(w[j], hq.x, hq.y, sh) >> 5)) : 0ull;
+                bk[j] = ((w[j] - hq.x) * hq.y) >> shift;
+                en[j] = f[j] != kInvalid ? __ldg(words + (bk[j] >> 5)) : 0ull;
               }
 #pragma unroll
               for (int j = 0; j < kWaveWays; ++j) {
-                const uint32_t bit = 1u << (rank_bucket(w[j], hq.x, hq.y, sh) & 31);
-                uint32_t p = (uint32_t)(en[j] >> 32) + __popc((uint32_t)en[j] & (bit - 1));
+                const uint32_t bit = 1u << (bk[j] & 31);
                 if ((uint32_t)en[j] & bit) {
+                  uint32_t p = (uint32_t)(en[j] >> 32) + __popc((uint32_t)en[j] & (bit - 1));
                   unsigned long long at = __ldg(U.row + p);
-                  if ((uint32_t)at < w[j])
-                    p = rank_later(U.row, p, dsc.w, words, rank_bucket(w[j], hq.x, hq.y, sh), sh, w[j], &at);
-                  // h == kInvalid: the long row's own vertex (a self-loop entry)
+                  if ((uint32_t)at < w[j]) p = rank_later(U.row, p, dsc.w, words, bk[j], shift, w[j], &at);
                   if (p != kInvalid && (uint32_t)at == w[j]) h[j] = (uint32_t)(at >> 32);
                 }
               }
@@ -2233,37 +2257,42 @@ __device__ __forceinline__ void wave_work(const WaveArgs& a, WaveShared<kWarps>&
               for (int j = 0; j < kWaveWays; ++j) {
                 w[j] = (uint32_t)en[j];
                 f[j] = (uint32_t)(en[j] >> 32);
-                if (f[j] != kInvalid && f[j] != e) {
+                if (f[j] != kInvalid) {
                   const uint32_t p = find_in_row(U.row, dsc.z, dsc.w, w[j]);
                   if (p != kInvalid) h[j] = (uint32_t)(__ldg(U.row + p) >> 32);
                 }
               }
             }
-            // both other edges' states are read only for a found triangle (a
-            // third of the elements on R-MAT)
-            int2 sf[kWaveWays], sh2[kWaveWays];
+            // found triangles gather in the warp's stage and are resolved 32 at a
+            // time, so that the rule runs on full warps (a third of the elements
+            // are hits on R-MAT)
 #pragma unroll
             for (int j = 0; j < kWaveWays; ++j) {
-              sf[j] = sh2[j] = make_int2(0, 0);
-              if (h[j] != kInvalid) { sf[j] = U.es[f[j]]; sh2[j] = U.es[h[j]]; }
-            }
-#pragma unroll
-            for (int j = 0; j < kWaveWays; ++j) {
-              bool pf = false, ph = false;
+              const unsigned hb = __ballot_sync(kFull, h[j] != kInvalid);
+              if (hb == 0) continue;
+              const uint32_t at = nhit + __popc(hb & ((1u << lane) - 1));
               if (h[j] != kInvalid) {
-                ++found;
-                pkt_rule<kMulti>(U, e, f[j], sf[j], h[j], sh2[j], w32[kCtxLevel], w32[kCtxW], pf, ph);
+                sh.hit_e[wib][at] = e;
+                sh.hit_f[wib][at] = f[j];
+                sh.hit_h[wib][at] = h[j];
               }
-              if (__any_sync(kFull, pf || ph)) {
-                push_edge(ps, U, a.Up, w32[kCtxEb], w32[kCtxM], a.st + w32[kCtxG], a.err, w32[kCtxQsel], pf, f[j],
-                          w32[kCtxW]);
-                push_edge(ps, U, a.Up, w32[kCtxEb], w32[kCtxM], a.st + w32[kCtxG], a.err, w32[kCtxQsel], ph, h[j],
-                          w32[kCtxW]);
+              nhit += __popc(hb);
+              found += __popc(hb);
+              if (nhit >= 32) {
+                __syncwarp();
+                nhit -= 32;
+                resolve(nhit, kFull);
+                __syncwarp();
               }
             }
           }
         }
-        found = __reduce_add_sync(kFull, found);
+        if (nhit) {
+          __syncwarp();
+          resolve(0, nhit == 32 ? kFull : (1u << nhit) - 1);
+          nhit = 0;
+          __syncwarp();
+        }
         if (lane == 0) sh.cnt[0][wib] += found;
         // entries belong to this member: publish before moving on
         push_flush(ps, a.Up, w32[kCtxEb], w32[kCtxM], a.st + w32[kCtxG], a.err, w32[kCtxQsel]);
@@ -2297,7 +2326,7 @@ __device__ __forceinline__ void flush_counts(const WaveArgs& a, const WaveShared
 }
 
 template <bool kMulti>
-__global__ void __launch_bounds__(kWaveThreads, SPARX_WAVE_MINB) k_wave(WaveArgs a) {
+__global__ void __launch_bounds__(kWaveThreads, kWaveBlocksPerSm) k_wave(WaveArgs a) {
   __shared__ WaveShared<kWaveWarps> sh;
   const uint32_t lane = lane_id();
   if (lane < 3) sh.cnt[lane][threadIdx.x >> 5] = 0;
@@ -2329,7 +2358,7 @@ __global__ void __launch_bounds__(kWaveThreads, SPARX_WAVE_MINB) k_wave(WaveArgs
 // while the planned one has at most `max_work` elements, its blocks meeting at
 // the cluster's hardware barrier instead of at a kernel boundary, and block 0
 // planning between two of them.  A wave of 100 elements takes 7 us here, 13 to 14
-// as a kernel of 1,184 blocks (launch gap 3, block start 1, ticket 2); what is
+// as a kernel over the whole chip (launch gap 3, block start 1, ticket 2); what is
 // left is its chain of dependent round trips to L2.  The barrier's release and
 // acquire order the waves' memory; everything a wave reads through the read-only
 // path (rows, index, edges) does not change between compactions.  Every block
