@@ -1987,6 +1987,10 @@ __device__ __forceinline__ void plan_wave(const Member* __restrict__ mem, Member
 // entry j of the segment is kept (support above the level), queued for this
 // level, or dropped (processed).  Not inlined: its staging state stays out of
 // the frontier loop's register budget.  Publishes its pushes before returning.
+// Four groups of 32 entries at a time: what bounds a scan is its instructions and
+// the two dependent loads per entry (R-MAT-22's scans 33 -> 26 ms, its largest 168
+// -> 132 us for 19 M entries; two groups 29 ms, a stage of 384 entries 28).
+constexpr int kScanWays = 4;
 __device__ __noinline__ void wave_scan_segment(const Union* Up, MemberState* st, uint32_t eb, uint32_t m,
                                                uint32_t phase, uint32_t level, uint32_t act_sel, uint32_t q_sel,
                                                uint32_t W, uint32_t a0, uint32_t seg_len, uint32_t* keepbuf,
@@ -1996,41 +2000,49 @@ __device__ __noinline__ void wave_scan_segment(const Union* Up, MemberState* st,
   PushStage ps{push_eid, 0};
   const uint32_t* act = act_sel ? U.act1 : U.act0;
   uint32_t* act_out = act_sel ? U.act0 : U.act1;
+  const bool first = phase == kPhaseScan0;
   uint32_t nkeep = 0, nzero = 0, mn = 0xFFFFFFFFu;
-  for (uint32_t r = 0; r < seg_len; r += 32) {
-    const bool valid = r + lane < seg_len;
-    bool keep = false, zero = false, queue = false;
-    uint32_t le = 0, e = 0;
-    if (valid) {
-      le = act[eb + a0 + r + lane];
-      e = eb + le;
-      const int2 st_e = U.es[e];
-      const int32_t s = st_e.x;
-      if (phase == kPhaseScan0) {
-        if (s == 0) { U.es[e].y = 0; zero = true; }
-        else { keep = true; mn = min(mn, (uint32_t)s); }
-      } else if ((uint32_t)st_e.y == kTagActive) {  // processed edges leave the active list
-        if (s <= (int32_t)level) queue = true;
-        else { keep = true; mn = min(mn, (uint32_t)s); }
-      }
+  act += eb + a0;
+  for (uint32_t r = 0; r < seg_len; r += 32 * kScanWays) {
+    // kScanWays groups of 32 entries: their ids, then their states, side by side
+    uint32_t le[kScanWays];
+    int2 se[kScanWays];
+#pragma unroll
+    for (int j = 0; j < kScanWays; ++j) le[j] = r + 32 * j + lane < seg_len ? act[r + 32 * j + lane] : kInvalid;
+#pragma unroll
+    for (int j = 0; j < kScanWays; ++j) se[j] = le[j] != kInvalid ? U.es[eb + le[j]] : make_int2(0, 0);
+    if (nkeep + 32 * kScanWays > kKeepBuf) {
+      __syncwarp();
+      uint32_t old = 0;
+      if (lane == 0) old = atomicAdd(&st->kept, nkeep);
+      old = __shfl_sync(kFull, old, 0);
+      for (uint32_t t = lane; t < nkeep; t += 32) act_out[eb + old + t] = keepbuf[t];
+      nkeep = 0;
+      __syncwarp();
     }
-    push_edge(ps, U, Up, eb, m, st, err, q_sel, queue, e, W);
-    const unsigned kb_bal = __ballot_sync(kFull, keep);
-    if (kb_bal) {
-      const uint32_t kc = __popc(kb_bal);
-      if (nkeep + kc > kKeepBuf) {
-        __syncwarp();
-        uint32_t old = 0;
-        if (lane == 0) old = atomicAdd(&st->kept, nkeep);
-        old = __shfl_sync(kFull, old, 0);
-        for (uint32_t t = lane; t < nkeep; t += 32) act_out[eb + old + t] = keepbuf[t];
-        nkeep = 0;
-        __syncwarp();
+    bool queue[kScanWays], any = false;
+#pragma unroll
+    for (int j = 0; j < kScanWays; ++j) {
+      const int32_t s = se[j].x;
+      // processed edges leave the active list (the first scan: those without support)
+      const bool live = le[j] != kInvalid && (first ? s != 0 : (uint32_t)se[j].y == kTagActive);
+      queue[j] = live && !first && s <= (int32_t)level;
+      const bool keep = live && !queue[j];
+      if (keep) mn = min(mn, (uint32_t)s);
+      if (first && le[j] != kInvalid && !live) {
+        U.es[eb + le[j]].y = 0;
+        ++nzero;
       }
-      if (keep) keepbuf[nkeep + __popc(kb_bal & ((1u << lane) - 1))] = le;
-      nkeep += kc;
+      any |= queue[j];
+      const unsigned kb = __ballot_sync(kFull, keep);
+      if (keep) keepbuf[nkeep + __popc(kb & ((1u << lane) - 1))] = le[j];
+      nkeep += __popc(kb);
     }
-    nzero += __popc(__ballot_sync(kFull, zero));
+    if (__any_sync(kFull, any)) {
+#pragma unroll
+      for (int j = 0; j < kScanWays; ++j)
+        push_edge(ps, U, Up, eb, m, st, err, q_sel, queue[j], eb + le[j], W);
+    }
   }
   __syncwarp();
   if (nkeep) {
@@ -2039,6 +2051,7 @@ __device__ __noinline__ void wave_scan_segment(const Union* Up, MemberState* st,
     old = __shfl_sync(kFull, old, 0);
     for (uint32_t t = lane; t < nkeep; t += 32) act_out[eb + old + t] = keepbuf[t];
   }
+  nzero = __reduce_add_sync(kFull, nzero);
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) mn = min(mn, __shfl_xor_sync(kFull, mn, d));
   if (lane == 0) {
