@@ -653,9 +653,40 @@ def mtx_to_csr(data: bytes, device: int = -1):
     L = lib()
     o = PktOptions(device=device).c()
     n, w = ctypes.c_uint64(), ctypes.c_uint64()
-    _check(L.sparx_mtx_to_csr(data, len(data), None, 0, None, 0, ctypes.byref(n), ctypes.byref(w), ctypes.byref(o)))
-    off = np.empty(n.value + 1, dtype=np.uint64)
-    nbr = np.empty(max(w.value, 1), dtype=np.uint64)
-    _check(L.sparx_mtx_to_csr(data, len(data), off.ctypes.data, off.shape[0], nbr.ctypes.data, nbr.shape[0],
-                              ctypes.byref(n), ctypes.byref(w), ctypes.byref(o)))
+
+    def call(off, nbr):
+        return L.sparx_mtx_to_csr(data, len(data), off.ctypes.data if off is not None else None,
+                                  off.shape[0] if off is not None else 0,
+                                  nbr.ctypes.data if nbr is not None else None,
+                                  nbr.shape[0] if nbr is not None else 0, ctypes.byref(n), ctypes.byref(w),
+                                  ctypes.byref(o))
+
+    # the size line's entries, mirrored, bound the result of a well-formed text: one
+    # call parses it.  A text with more entries than it declares is parsed again.
+    rows, entries = _mtx_declared(data)
+    off = np.empty(rows + 1, dtype=np.uint64)
+    nbr = np.empty(max(2 * entries, 1), dtype=np.uint64)
+    rc = call(off, nbr) if entries else E_ARG
+    if rc == E_ARG:
+        _check(call(None, None))
+        off = np.empty(n.value + 1, dtype=np.uint64)
+        nbr = np.empty(max(w.value, 1), dtype=np.uint64)
+        rc = call(off, nbr)
+    _check(rc)
     return off, nbr[: w.value]
+
+
+def _mtx_declared(data: bytes) -> tuple[int, int]:
+    """Rows and entries of the size line, (0, 0) where there is none to trust (more entries than the
+    text has room for, or offsets past a gigabyte; the parser judges the text itself)."""
+    at = data.find(b"\n") + 1
+    while 0 < at < len(data):
+        end = data.find(b"\n", at)
+        line = data[at:end if end >= 0 else len(data)].split()
+        if line and not line[0].startswith(b"%"):
+            size = [int(t) for t in line[:3] if t.isdigit()]
+            if len(size) == 3 and size[0] == size[1] and 4 * size[2] <= len(data) + 4 and size[0] <= 1 << 27:
+                return size[0], size[2]
+            return 0, 0
+        at = end + 1 if end >= 0 else 0
+    return 0, 0
