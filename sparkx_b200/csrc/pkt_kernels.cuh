@@ -363,6 +363,37 @@ __global__ void k_narrow_offsets(const unsigned long long* __restrict__ src, uin
 }
 
 
+// A device-resident CSR in one launch: offsets narrowed and checked as by
+// k_narrow_offsets (first 0, last `width`), ids checked as by k_range_ids.
+__global__ void k_check_csr(const unsigned long long* __restrict__ src, uint32_t* __restrict__ off, uint32_t n,
+                            const uint32_t* __restrict__ ids, unsigned long long width, uint32_t* __restrict__ err) {
+  const unsigned long long t = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
+  bool bad = t == 0 && (__ldg(src) != 0 || __ldg(src + n) != width), range = false;
+#pragma unroll 4
+  for (unsigned long long i = t; i < n; i += stride) {
+    const unsigned long long x = __ldg(src + i);
+    bad |= __ldg(src + i + 1) < x;
+    off[i] = (uint32_t)x;
+  }
+  if (t == 0) off[n] = (uint32_t)width;  // as checked above
+  // ids four at a time where the caller's array allows it
+  const unsigned long long quads = ((uintptr_t)ids & 15) == 0 ? width / 4 : 0;
+  const uint4* id4 = reinterpret_cast<const uint4*>(ids);
+#pragma unroll 4
+  for (unsigned long long i = t; i < quads; i += stride) {
+    const uint4 v = __ldg(id4 + i);
+    range |= v.x >= n || v.y >= n || v.z >= n || v.w >= n;
+  }
+  for (unsigned long long i = 4 * quads + t; i < width; i += stride) range |= __ldg(ids + i) >= n;
+  if (bad) atomicOr(err, kErrOffsets);
+  if (range) atomicOr(err, kErrRange);
+}
+
+// The input checks' verdict: kernels behind them that follow offsets or ids do
+// nothing on a flagged input (the host reads the flags once, with the counts).
+__device__ __forceinline__ bool bad_input(const uint32_t* err) { return __ldcg(err) & (kErrOffsets | kErrRange); }
+
 // ---------------------------------------------------------------------------
 // Exclusive scan across the block (all threads call it); `total` is the
 // block sum.  smem_warp holds one value per warp.
@@ -412,7 +443,9 @@ constexpr uint32_t kHeavyRow = 256;
 __global__ void __launch_bounds__(256) k_degree_stats(const uint32_t* __restrict__ off, uint32_t n,
                                                       uint32_t* __restrict__ list, uint32_t* __restrict__ count,
                                                       uint32_t* __restrict__ dmax,
-                                                      unsigned long long* __restrict__ heavy) {
+                                                      unsigned long long* __restrict__ heavy,
+                                                      const uint32_t* err) {
+  if (bad_input(err)) return;
   uint32_t mx = 0;
   unsigned long long hv = 0;
   for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < n; u += gridDim.x * blockDim.x) {
@@ -452,6 +485,8 @@ __global__ void __launch_bounds__(256) k_orient_count(const uint32_t* __restrict
                                                       uint32_t* __restrict__ max_dplus,
                                                       const uint32_t* __restrict__ big_list,
                                                       const uint32_t* __restrict__ big_count) {
+  // (this kernel itself raises kErrRange only where the checks before it did)
+  if (bad_input(err)) return;
   const uint32_t lane = lane_id();
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -1557,6 +1592,29 @@ __global__ void k_peel_init(const Member* __restrict__ mem, MemberState* __restr
     ctl->el_scan = carry;
     ctl->t_start = globaltimer();
   }
+}
+
+// A single graph's peel state in one launch: the union, its member and the loop
+// control (by value), the member's sums cleared, its first wave the level-0 scan.
+__global__ void k_peel_begin(Union U, Union* dU, Member M, Member* mem, Control c, Control* ctl, MemberState* st,
+                             unsigned long long* wpref, unsigned long long* mem_tri, uint32_t* mem_maxsup) {
+  *dU = U;
+  *mem = M;
+  *mem_tri = 0;
+  *mem_maxsup = 0;
+  MemberState s{};
+  s.phase = M.m ? kPhaseScan0 : kPhaseDone;
+  s.act_count = M.m;
+  s.min_kept = 0xFFFFFFFFu;
+  *st = s;
+  wpref[0] = 0;
+  wpref[1] = M.m;
+  c.total_work = M.m;
+  c.wave = 1;
+  c.done = M.m == 0;
+  c.el_scan = M.m;
+  c.t_start = globaltimer();
+  *ctl = c;
 }
 
 struct WaveArgs {

@@ -202,7 +202,7 @@ struct Counters {  // device scalars
   uint32_t dmax;         // largest degree
   uint32_t pad;
   unsigned long long heavy;  // slots in rows of degree >= kHeavyRow
-  unsigned long long elements;  // support (pair form): shorter-list entries
+  unsigned long long elements;  // support: shorter-list entries (not counted by the vertex form)
   uint32_t table_big;    // rank index, hash tables: what is listed for whole blocks
   double cc_possible;    // clustering: sum of d(d - 1)/2 over vertices
   double cc_local;       //             sum of local coefficients
@@ -623,7 +623,7 @@ struct SupportIndex {
 int launch_support(int sm_count, uint32_t support_kernel, uint32_t n, uint64_t m, uint32_t max_dplus,
                    const uint32_t* opos, const uint32_t* ocol, const uint32_t* osrc, int2* es,
                    unsigned long long* spref, unsigned long long* tiles, Counters* cnt, uint32_t* heavy_list,
-                   cudaStream_t s, uint32_t* launches, unsigned long long* support_elements, const SupportIndex& X,
+                   cudaStream_t s, uint32_t* launches, const SupportIndex& X,
                    const uint32_t* mu = nullptr, const unsigned long long* hpool = nullptr, uint32_t hash_min = 0) {
   if (m == 0) return SPARX_OK;
   uint32_t slots = 8;
@@ -639,7 +639,6 @@ int launch_support(int sm_count, uint32_t support_kernel, uint32_t n, uint64_t m
     k_support_heavy<<<sm_count * 4, 256, hsmem, s>>>(opos, ocol, es, &cnt->tri, heavy_list, &cnt->heavy_count,
                                                      &cnt->hcursor, slots, max_dplus);
     *launches += 2;
-    *support_elements = 0;
     return SPARX_OK;
   }
   // 0: no list is longer than a thread walks
@@ -648,7 +647,6 @@ int launch_support(int sm_count, uint32_t support_kernel, uint32_t n, uint64_t m
     if (mu) k_support_pairs<true><<<g, 256, 0, s>>>(opos, ocol, osrc, (uint32_t)m, es, &cnt->tri, &cnt->elements, mu);
     else k_support_pairs<false><<<g, 256, 0, s>>>(opos, ocol, osrc, (uint32_t)m, es, &cnt->tri, &cnt->elements, mu);
     *launches += 1;
-    CU(cudaMemcpyAsync(support_elements, &cnt->elements, 8, cudaMemcpyDeviceToHost, s));
     return SPARX_OK;
   }
   if (X.hdr) {
@@ -673,7 +671,7 @@ int launch_support(int sm_count, uint32_t support_kernel, uint32_t n, uint64_t m
     if (mu) go(k_support_balanced<true, false>); else go(k_support_balanced<false, false>);
   }
   *launches += 4;
-  CU(cudaMemcpyAsync(support_elements, spref + m, 8, cudaMemcpyDeviceToHost, s));
+  CU(cudaMemcpyAsync(&cnt->elements, spref + m, 8, cudaMemcpyDeviceToDevice, s));
   return SPARX_OK;
 }
 
@@ -961,15 +959,11 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
   Member* dmem = at<Member>(E, L.mem);
   const int vgrid = grid_for(N, 256, E.sm_count * 32);  // row kernels: 32 vertices per warp
 
+  // a single graph: its member needs no device copy before the peel, and its
+  // state is written and read back in one piece each
+  const bool solo = G == 1 && !J.hook && !J.prep_only;
+
   CU(cudaEventRecord(E.tev[1], s));
-  {
-    // offsets / ids validated by the upload must be sound before any kernel
-    // dereferences them
-    uint32_t* herr = (uint32_t*)E.pinned_small;
-    CU(cudaMemcpyAsync(herr, err, 4, cudaMemcpyDeviceToHost, s));
-    CU(cudaStreamSynchronize(s));
-    if (*herr) { J.err = *herr; return status_from_flags(*herr); }
-  }
   // -- orientation (Kernel B) --
   uint32_t* big = at<uint32_t>(E, L.big);
   // multigraphs: deduplicated rows, copies per slot, caller slot -> slot and
@@ -988,20 +982,27 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
       CU(cudaMemsetAsync(&cnt->dmax, 0, 4, s));
     }
     k_degree_stats<<<grid_for(N, 256, E.sm_count * 8), 256, 0, s>>>(J.off, N, big, &cnt->big_count, &cnt->dmax,
-                                                                    &cnt->heavy);
+                                                                    &cnt->heavy, err);
     J.launches += 1;
     k_orient_count<<<vgrid, 256, 0, s>>>(J.off, J.nbr, N, dplus, &cnt->self_loops, err, &cnt->max_dplus, big,
                                          &cnt->big_count);
     J.launches += 1;
     exclusive_scan<uint32_t>(LoadU32{dplus}, N, opos, at<uint32_t>(E, L.tiles), (uint32_t*)&cnt->grand, s);
     J.launches += 4;
-    CU(cudaMemcpyAsync(dmem, J.members.data(), sizeof(Member) * G, cudaMemcpyHostToDevice, s));
-    k_member_edges<<<grid_for(G, 256, 1024), 256, 0, s>>>(dmem, G, opos);
-    J.launches += 1;
-    CU(cudaMemcpyAsync(J.members.data(), dmem, sizeof(Member) * G, cudaMemcpyDeviceToHost, s));
-    CU(cudaMemcpyAsync(&hc, cnt, sizeof(Counters), cudaMemcpyDeviceToHost, s));
-    CU(cudaMemcpyAsync(&m32, opos + N, 4, cudaMemcpyDeviceToHost, s));
+    if (!solo) {
+      CU(cudaMemcpyAsync(dmem, J.members.data(), sizeof(Member) * G, cudaMemcpyHostToDevice, s));
+      k_member_edges<<<grid_for(G, 256, 1024), 256, 0, s>>>(dmem, G, opos);
+      J.launches += 1;
+      CU(cudaMemcpyAsync(J.members.data(), dmem, sizeof(Member) * G, cudaMemcpyDeviceToHost, s));
+    }
+    CU(cudaMemcpyAsync(E.pinned_small, cnt, sizeof(Counters), cudaMemcpyDeviceToHost, s));
     CU(cudaStreamSynchronize(s));
+    hc = *(const Counters*)E.pinned_small;
+    m32 = (uint32_t)hc.grand;  // the scan's total: oriented edges
+    if (solo) {
+      J.members[0].eb = 0;
+      J.members[0].m = m32;
+    }
     if (pass == 0) J.slot_self_loops = hc.self_loops;
     // (batched unions: the packer counted the relabelled copy in their budget)
     if (pass == 0 && hc.err == 0 && N > 1 && W > 0 && !J.support_only && !J.prep_only && !J.hook &&
@@ -1145,8 +1146,7 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
       form = 0;
     int rc = launch_support(E.sm_count, form, N, m,
                             hc.max_dplus, opos, ocol, osrc, es, at<unsigned long long>(E, L.q0),
-                            at<unsigned long long>(E, L.tiles), cnt, at<uint32_t>(E, L.act0), s, &J.launches,
-                            &J.support_elements, X, mu, spool, sup_hash_min);
+                            at<unsigned long long>(E, L.tiles), cnt, at<uint32_t>(E, L.act0), s, &J.launches, X, mu, spool, sup_hash_min);
     if (rc) return rc;
   }
   CU(cudaEventRecord(E.tev[3], s));
@@ -1207,9 +1207,6 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
     U.m = (uint32_t)m;
     U.width = (uint32_t)W;
     U.G = G;
-    CU(cudaMemcpyAsync(at<Union>(E, L.uni), &U, sizeof(Union), cudaMemcpyHostToDevice, s));
-    CU(cudaMemsetAsync(at<unsigned long long>(E, L.mem_tri), 0, 8ull * G, s));
-    CU(cudaMemsetAsync(at<uint32_t>(E, L.mem_maxsup), 0, 4ull * G, s));
     Control c0{};
     c0.G = G;
     c0.max_waves = 3ull * m + 64;  // each frontier wave processes >= 1 edge; <= 2 scans per level
@@ -1229,14 +1226,24 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
       c0.trace = E.trace;
       c0.trace_cap = kTraceRecords;
     }
-    CU(cudaMemcpyAsync(at<Control>(E, L.ctl), &c0, sizeof(Control), cudaMemcpyHostToDevice, s));
+    if (solo) {
+      k_peel_begin<<<1, 1, 0, s>>>(U, at<Union>(E, L.uni), J.members[0], dmem, c0, at<Control>(E, L.ctl),
+                                   at<MemberState>(E, L.st), at<unsigned long long>(E, L.wpref),
+                                   at<unsigned long long>(E, L.mem_tri), at<uint32_t>(E, L.mem_maxsup));
+    } else {
+      CU(cudaMemcpyAsync(at<Union>(E, L.uni), &U, sizeof(Union), cudaMemcpyHostToDevice, s));
+      CU(cudaMemsetAsync(at<unsigned long long>(E, L.mem_tri), 0, 8ull * G, s));
+      CU(cudaMemsetAsync(at<uint32_t>(E, L.mem_maxsup), 0, 4ull * G, s));
+      CU(cudaMemcpyAsync(at<Control>(E, L.ctl), &c0, sizeof(Control), cudaMemcpyHostToDevice, s));
+    }
     if (m > 0)
       k_peel_setup<<<grid_for(m, 256, E.sm_count * 8), 256, 0, s>>>(at<Union>(E, L.uni), dmem,
                                                                      O.support_mode == SPARX_SUPPORT_U8,
                                                                      at<unsigned long long>(E, L.mem_tri),
                                                                      at<uint32_t>(E, L.mem_maxsup), mu, err);
-    k_peel_init<<<1, 1024, 0, s>>>(dmem, at<MemberState>(E, L.st), at<Control>(E, L.ctl),
-                                   at<unsigned long long>(E, L.wpref), G);
+    if (!solo)
+      k_peel_init<<<1, 1024, 0, s>>>(dmem, at<MemberState>(E, L.st), at<Control>(E, L.ctl),
+                                     at<unsigned long long>(E, L.wpref), G);
     J.launches += m > 0 ? 2 : 1;
     CU(cudaEventRecord(E.tev[4], s));
     WaveArgs wa;
@@ -1365,14 +1372,30 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
   J.states.resize(G);
   J.mem_tri.resize(G);
   J.mem_maxsup.resize(G);
-  if (!J.support_only) {
+  static_assert(7 * 256 + sizeof(Control) <= 4096, "a single graph's state fits the pinned page");
+  if (solo) {
+    // the arrays from the control to the member's largest support lie side by side
+    CU(cudaMemcpyAsync(E.pinned_small, E.ws + L.ctl, L.mem_maxsup + 4 - L.ctl, cudaMemcpyDeviceToHost, s));
+    CU(cudaStreamSynchronize(s));
+    const char* h = (const char*)E.pinned_small - L.ctl;
+    hc = *(const Counters*)(h + L.cnt);
+    if (!J.support_only) {
+      J.states[0] = *(const MemberState*)(h + L.st);
+      J.mem_tri[0] = *(const unsigned long long*)(h + L.mem_tri);
+      J.mem_maxsup[0] = *(const uint32_t*)(h + L.mem_maxsup);
+      J.ctl = *(const Control*)(h + L.ctl);
+    }
+  } else if (!J.support_only) {
     CU(cudaMemcpyAsync(J.states.data(), at<MemberState>(E, L.st), sizeof(MemberState) * G, cudaMemcpyDeviceToHost, s));
     CU(cudaMemcpyAsync(J.mem_tri.data(), at<unsigned long long>(E, L.mem_tri), 8ull * G, cudaMemcpyDeviceToHost, s));
     CU(cudaMemcpyAsync(J.mem_maxsup.data(), at<uint32_t>(E, L.mem_maxsup), 4ull * G, cudaMemcpyDeviceToHost, s));
     CU(cudaMemcpyAsync(&J.ctl, at<Control>(E, L.ctl), sizeof(Control), cudaMemcpyDeviceToHost, s));
   }
-  CU(cudaMemcpyAsync(&hc, cnt, sizeof(Counters), cudaMemcpyDeviceToHost, s));
-  CU(cudaStreamSynchronize(s));
+  if (!solo) {
+    CU(cudaMemcpyAsync(&hc, cnt, sizeof(Counters), cudaMemcpyDeviceToHost, s));
+    CU(cudaStreamSynchronize(s));
+  }
+  J.support_elements = hc.elements;
   J.tri = hc.tri;
   J.hubs = hc.hub_count;
   J.kmax = hc.kmax;
@@ -3311,12 +3334,9 @@ int sparx_pkt_run_device(const uint64_t* d_offsets, uint64_t n_plus_1, const uin
   auto t0 = std::chrono::steady_clock::now();
   CU(cudaMemsetAsync(cnt, 0, sizeof(Counters), s));
   CU(cudaEventRecord(E.tev[0], s));
-  k_narrow_offsets<<<grid_for(n_plus_1, 256, E.sm_count * 16), 256, 0, s>>>(
-      (const unsigned long long*)d_offsets, J.off, (uint32_t)n_plus_1, 0u, 0ll, (long long)width, &cnt->err);
-  if (width)
-    k_range_ids<<<grid_for(width, 256, E.sm_count * 16), 256, 0, s>>>(d_neighbours, nullptr, width, (uint32_t)n, 0u,
-                                                                       &cnt->err);
-  J.launches += width ? 2 : 1;
+  k_check_csr<<<grid_for(std::max(n_plus_1, width), 256, E.sm_count * 16), 256, 0, s>>>(
+      (const unsigned long long*)d_offsets, J.off, (uint32_t)n, d_neighbours, width, &cnt->err);
+  J.launches += 1;
   rc = run_union(E, J, O, s);
   fill_stats(J, 0, stats);
   if (rc) return rc;
@@ -3479,7 +3499,7 @@ int run_noalloc(const uint64_t* d_offsets, uint64_t n_plus_1, const uint32_t* d_
 
   const int vgrid = grid_for(N, 256, sm * 32);  // row kernels: 32 vertices per warp
   uint32_t* big = (uint32_t*)P(L.big);  // big_count was cleared with the counters above
-  k_degree_stats<<<grid_for(N, 256, sm * 8), 256, 0, s>>>(off, N, big, &cnt->big_count, &cnt->dmax, &cnt->heavy);
+  k_degree_stats<<<grid_for(N, 256, sm * 8), 256, 0, s>>>(off, N, big, &cnt->big_count, &cnt->dmax, &cnt->heavy, err);
   k_orient_count<<<vgrid, 256, 0, s>>>(off, d_nbr, N, dplus, &cnt->self_loops, err, &cnt->max_dplus, big,
                                        &cnt->big_count);
   exclusive_scan<uint32_t>(LoadU32{dplus}, N, opos, (uint32_t*)P(L.tiles), (uint32_t*)&cnt->grand, s);
@@ -3518,9 +3538,8 @@ int run_noalloc(const uint64_t* d_offsets, uint64_t n_plus_1, const uint32_t* d_
   CU(cudaMemsetAsync(es, 0, 8 * std::max<uint64_t>(m, 1), s));
   {
     uint32_t launches = 0;
-    unsigned long long elements = 0;
     rc = launch_support(sm, hc.max_dplus <= kPairList ? 0 : 1, N, m, hc.max_dplus, opos, ocol, osrc, es, (unsigned long long*)P(L.q0),
-                        (unsigned long long*)P(L.tiles), cnt, (uint32_t*)P(L.act0), s, &launches, &elements, X);
+                        (unsigned long long*)P(L.tiles), cnt, (uint32_t*)P(L.act0), s, &launches, X);
     if (rc) return rc;
   }
 
