@@ -31,6 +31,7 @@
 //   vinfo[n] (u64)              per vertex: the header of its row's rank index
 #pragma once
 
+#include <cstddef>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -2152,10 +2153,31 @@ struct WaveShared {
   uint32_t w32[kWarps][8];            // kCtxEb .. kCtxW
 };
 
-// This warp's share of wave W (warp `warp` of `nwarps`).
-template <bool kMulti, int kWarps>
+// What a small wave's warps need of member 0, read in the same round of loads as
+// the control: a single graph's wave then starts one L2 round trip earlier (a wave
+// over the whole chip loses more to the registers this holds: R-MAT-19 2% slower).
+struct WaveHead {
+  uint4 s;                  // phase, level, act_sel, q_sel
+  unsigned long long curr;
+  Member M;
+};
+__device__ __forceinline__ WaveHead wave_head(const WaveArgs& a) {
+  const uint4* st = reinterpret_cast<const uint4*>(a.st);
+  WaveHead h;
+  h.s = __ldcg(st);
+  h.curr = __ldcg(reinterpret_cast<const unsigned long long*>(st + 2));
+  h.M = a.mem[0];
+  return h;
+}
+static_assert(offsetof(MemberState, phase) == 0 && offsetof(MemberState, q_sel) == 12 &&
+                  offsetof(MemberState, curr) == 32, "wave_head reads MemberState as uint4 words");
+
+// This warp's share of wave W (warp `warp` of `nwarps`).  kTail (small waves): a
+// warp's queue window brings its entries' row descriptors along, 24 bytes more per
+// entry for a round trip less.
+template <bool kMulti, bool kTail, int kWarps>
 __device__ __forceinline__ void wave_work(const WaveArgs& a, WaveShared<kWarps>& sh, unsigned long long total,
-                                          uint32_t W, uint32_t G, unsigned long long warp,
+                                          uint32_t W, uint32_t G, const WaveHead& head, unsigned long long warp,
                                           unsigned long long nwarps) {
   const uint32_t lane = lane_id();
   const uint32_t wib = threadIdx.x >> 5;
@@ -2184,11 +2206,13 @@ __device__ __forceinline__ void wave_work(const WaveArgs& a, WaveShared<kWarps>&
         if (lane == 0) atomicOr(a.err, kErrInternal);
         break;
       }
-      const Member M = a.mem[g];
       MemberState* st = a.st + g;
-      const uint32_t phase = st->phase, level = st->level, act_sel = st->act_sel, q_sel = st->q_sel;
+      const bool ready = kTail && G == 1;  // the head brought it
+      const Member M = ready ? head.M : a.mem[g];
+      const uint32_t phase = ready ? head.s.x : st->phase, level = ready ? head.s.y : st->level,
+                     act_sel = ready ? head.s.z : st->act_sel, q_sel = ready ? head.s.w : st->q_sel;
       if (phase == kPhaseProc) {
-        const uint32_t qcount0 = (uint32_t)(st->curr >> kWorkBits);
+        const uint32_t qcount0 = (uint32_t)((ready ? head.curr : st->curr) >> kWorkBits);
         if (qcount0 == 0) {
           if (lane == 0) atomicOr(a.err, kErrInternal);
           k = seg_end;
@@ -2245,6 +2269,12 @@ __device__ __forceinline__ void wave_work(const WaveArgs& a, WaveShared<kWarps>&
           const unsigned long long jr = w64[kCtxJb] + r;
           const unsigned long long qv =
               (i + lane < qcount) ? ((w32[kCtxQsel] ? U.q1 : U.q0) + w32[kCtxEb])[i + lane] : ~0ull;
+          uint4 wd = make_uint4(0, 0, 0, 0);
+          uint2 wh = make_uint2(0, 0);
+          if (kTail && i + lane < qcount) {
+            wd = ((w32[kCtxQsel] ? U.qd1 : U.qd0) + w32[kCtxEb])[i + lane];
+            if (U.qh0) wh = ((w32[kCtxQsel] ? U.qh1 : U.qh0) + w32[kCtxEb])[i + lane];
+          }
           const int32_t dq = (int32_t)max((long long)(jr - (qv >> kEidBits)), (long long)INT32_MIN);
           // elements of entry i from jr on (an end past the queue is 2^31)
           const uint32_t rem = min(seg_len - r, 0u - (uint32_t)__shfl_sync(kFull, dq, 1));
@@ -2254,6 +2284,7 @@ __device__ __forceinline__ void wave_work(const WaveArgs& a, WaveShared<kWarps>&
           uint2 hq = make_uint2(0, 0);
           uint32_t o_end;       // the lane's elements o, o + 32, ... below o_end
           const bool run = (int32_t)rem >= (int32_t)kWaveRun;
+          const uint32_t i_win = i;
           uint32_t x = i;
           if (run) {
             // the rest of entry i: one edge, the same rows for the whole warp
@@ -2281,7 +2312,12 @@ __device__ __forceinline__ void wave_work(const WaveArgs& a, WaveShared<kWarps>&
             r += 32;
             if (lane == 0) sh.cnt[2][wib]++;
           }
-          if (valid) {
+          if (kTail) {
+            const int src = (int)(x - i_win);
+            dsc = make_uint4(__shfl_sync(kFull, wd.x, src), __shfl_sync(kFull, wd.y, src),
+                             __shfl_sync(kFull, wd.z, src), __shfl_sync(kFull, wd.w, src));
+            hq = make_uint2(__shfl_sync(kFull, wh.x, src), __shfl_sync(kFull, wh.y, src));
+          } else if (valid) {
             dsc = ((w32[kCtxQsel] ? U.qd1 : U.qd0) + w32[kCtxEb])[x];
             if (U.qh0) hq = ((w32[kCtxQsel] ? U.qh1 : U.qh0) + w32[kCtxEb])[x];
           }
@@ -2404,7 +2440,7 @@ __global__ void __launch_bounds__(kWaveThreads, kWaveBlocksPerSm) k_wave(WaveArg
   __syncwarp();
   // a stopped loop (host-launched waves run on until the host looks) does no
   // work, but its blocks still hand over to the planner
-  wave_work<kMulti>(a, sh, a.ctl->done ? 0ull : a.ctl->total_work, a.ctl->wave, a.ctl->G,
+  wave_work<kMulti, false>(a, sh, a.ctl->done ? 0ull : a.ctl->total_work, a.ctl->wave, a.ctl->G, WaveHead{},
                     ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5,
                     ((unsigned long long)gridDim.x * blockDim.x) >> 5);
   __syncthreads();
@@ -2450,8 +2486,9 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_wave_tail(WaveArgs a, unsig
     const unsigned long long total = __ldcg(&a.ctl->total_work);
     const uint32_t W = __ldcg(&a.ctl->wave);
     const uint32_t G = __ldcg(&a.ctl->G);
+    const WaveHead head = wave_head(a);
     if (__ldcg(&a.ctl->done) || total > max_work) break;
-    wave_work<kMulti>(a, sh, total, W, G, wib * gridDim.x + blockIdx.x, (kTailThreads / 32) * gridDim.x);
+    wave_work<kMulti, true>(a, sh, total, W, G, head, wib * gridDim.x + blockIdx.x, (kTailThreads / 32) * gridDim.x);
     __syncwarp();
     cluster_barrier();
     if (blockIdx.x == 0) plan_wave(a.mem, a.st, a.ctl, a.wpref, a.err, a.handle, 0, s_plan, G, false);
