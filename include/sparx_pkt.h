@@ -239,7 +239,7 @@ typedef struct sparx_tuning {
   uint32_t struct_size;     /* sizeof(sparx_tuning) */
   uint32_t merge_ratio;     /* 1..1024; kept with the key, no effect: rows are no longer merged (8) */
   uint32_t hub_min_degree;  /* hub maps (a rank index with twice the buckets) for the rows of vertices
-                               of at least this degree, >= 256, or 0 for none (1024) */
+                               of at least this degree, >= 256, or 0 for none (0) */
   uint32_t sample_min;      /* support: longer out-lists of at least this length (8 at least) are
                                searched through a rank index, shorter ones by binary search (64) */
   uint32_t support_kernel;  /* 1 edge form (balanced, or a thread per edge where every list is
@@ -247,7 +247,7 @@ typedef struct sparx_tuning {
                                slots in rows of degree >= 256 and a largest degree of 64..255,
                                which is what sparx_tuning_lookup reports for such a key) */
   uint32_t compact_pct;     /* peel: rebuild the working rows once live entries fill at most
-                               this percentage of them (85) */
+                               this percentage of them (76) */
   uint32_t hash_min_degree; /* peel: rows of at least a quarter of this many entries (>= 8; 8 at least)
                                are searched through a rank index instead of by binary search; 0 = hub
                                rows only (128).  Skipped, with the same results, when its workspace

@@ -24,7 +24,7 @@
 //                               segment [eb_g, eb_g + m_g) for member g
 //   working CSR (off, row)      the peel's view: row0 at first, then rebuilt
 //                               without processed edges whenever the live
-//                               edges fill at most 85% of it (two ping-pong
+//                               edges fill at most 76% of it (two ping-pong
 //                               buffers)
 //   rank index (u64)            per row of the working CSR: where its names lie
 //                               (see rank_find); rebuilt with the rows
@@ -1924,10 +1924,10 @@ __device__ __forceinline__ uint32_t plan_commit(Control* ctl, uint32_t* __restri
   if (e) { done = 1; reason = kExitError; }
   if (waves > max_waves) { atomicOr(err, kErrWaves); done = 1; reason = kExitError; }
   if (globaltimer() - t_start > timeout) { atomicOr(err, kErrTimeout); done = 1; reason = kExitError; }
-  // live edges fill at most compact_pct % of the working rows (85 unless
+  // live edges fill at most compact_pct % of the working rows (76 unless
   // tuned): stop so the host can compact them (a compaction is a few passes
-  // over the rows, which the shorter rows repay at this fill; 78% and 90%
-  // measured slower on R-MAT-22)
+  // over the rows, which the shorter rows repay at this fill: R-MAT-22 276.4 ms,
+  // 85% 281.4, 70% 281.9, 90% 283.5)
   // ... once the waves since the last one have searched at least a kCompactPay-th
   // as many elements as it would move: a graph whose peel ends in a few small
   // waves (de Bruijn: 305 elements, 49 M slots, 0.6 of its 5.2 ms) never pays it

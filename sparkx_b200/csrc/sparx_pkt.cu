@@ -77,10 +77,10 @@ int status_from_flags(uint32_t f) {
 // defaults otherwise).  None of them changes a result, only the time.
 struct Tuning {
   uint32_t merge_ratio = 8;        // read and kept, no effect (rows are no longer merged)
-  uint32_t hub_min_degree = 1024;  // hub maps (the finer rank index) for vertices of at least this degree (0: none)
+  uint32_t hub_min_degree = 0;     // hub maps (the finer rank index) for vertices of at least this degree (0: none)
   uint32_t sample_min = 64;        // support: longer out-lists from this length are searched through a rank index
   uint32_t support_kernel = 1;     // 1 balanced edge form, 2 vertex form
-  uint32_t compact_pct = 85;       // rebuild the peel's rows when live entries fill <= this % of them
+  uint32_t compact_pct = 76;       // rebuild the peel's rows when live entries fill <= this % of them
   uint32_t hash_min_degree = 128;  // rows of a quarter of this many entries have a rank index (0: hubs only)
   uint32_t sup_hash_min = 0;       // support: out-lists of at least this length are probed in a hash table (0: none)
   uint32_t relabel = 0;            // rebuild the CSR on degree-ordered vertex ids first (0/1)
@@ -104,9 +104,14 @@ TuneKey tune_key(uint32_t dmax, unsigned long long heavy, unsigned long long tot
   return k;
 }
 
-// The knobs a key gets without a cached choice: the defaults, with the vertex
-// form of the support pass for unskewed graphs whose largest degree is 64..255
-// (no slots in rows of degree >= 256).  Measured on one B200 with both forms:
+// The knobs a key gets without a cached choice.  No finer index for hub rows and
+// rebuilds at 76%: against hub rows from degree 1024 and 85%, R-MAT-19 46.7 ->
+// 45.8 ms, R-MAT-22 281.5 -> 277 (the finer words' footprint costs more than the
+// absent names they stop: R-MAT-23 582 -> 573; 28 rebuilds -> 17), the batched
+// mix's peel 130.5 -> 127.6; 70% is 0.4 ms better at R-MAT-19 and 2 worse at
+// R-MAT-22, 90% is 3% slower at both.  Unskewed graphs whose largest degree is
+// 64..255 (no slots in rows of degree >= 256) get the vertex form of the support
+// pass.  Measured on one B200 with both forms:
 // ER n = 4.2 M, m = 67 M support 5.4 vs 7.8 ms, mix members of that class
 // 0.86-1.56 vs 1.09-2.56 ms; smaller largest degrees (de Bruijn graphs, sparse
 // ER) and skewed graphs (R-MAT) are faster with the edge form.
@@ -114,10 +119,10 @@ Tuning default_tuning(const TuneKey& k) {
   Tuning t;
   if (k.skew8 == 0 && k.log_dmax >= 7 && k.log_dmax <= 8) t.support_kernel = 2;
   // large skewed graphs (2^26 slots or more, a quarter of them or more in rows
-  // of degree >= 256) run on the degree-bucket relabelled CSR: R-MAT-22 / 23 /
-  // 24 437 -> 409, 963 -> 883, 2179 -> 1962 ms; below 2^26 slots the state
-  // fits the cache well enough that the relabelling costs more than it saves
-  // (R-MAT-16 .. 21 and R-MAT-22 with edge factor 8: 4-25% slower)
+  // of degree >= 256) run on the degree-bucket relabelled CSR: R-MAT-22 / 23
+  // 322 -> 277, 685 -> 573 ms, R-MAT-22 with edge factor 8 106 -> 103; below
+  // 2^26 slots it is a matter of the density (R-MAT-21 with edge factor 5 / 8 /
+  // 12 35.8 -> 39.4, 59.2 -> 59.3, 106.6 -> 102.6; R-MAT-17 .. 19 up to 11% slower)
   if (k.skew8 >= 2 && k.log_w >= 26) t.relabel = 1;
   return t;
 }
@@ -3134,10 +3139,10 @@ int autotune_core(RunF run, uint32_t repeats, Tuning* best_out, TuneKey* key_out
   for (uint32_t sh : {16u, 64u}) { Tuning t = cur; t.sup_hash_min = sh; c1.push_back(t); }
   if ((rc = try_group(c1, true))) return rc;
   std::vector<Tuning> c2;
-  for (uint32_t h : {0u, 512u, 4096u}) { Tuning t = cur; t.hub_min_degree = h; c2.push_back(t); }
+  for (uint32_t h : {512u, 1024u, 4096u}) { Tuning t = cur; t.hub_min_degree = h; c2.push_back(t); }
   if ((rc = try_group(c2, false))) return rc;
   std::vector<Tuning> c3;
-  for (uint32_t cp : {75u, 95u}) { Tuning t = cur; t.compact_pct = cp; c3.push_back(t); }
+  for (uint32_t cp : {65u, 88u}) { Tuning t = cur; t.compact_pct = cp; c3.push_back(t); }
   if ((rc = try_group(c3, false))) return rc;
   {
     // the relabelling changes the support pass and the peel (and costs a pass

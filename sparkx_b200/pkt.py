@@ -543,10 +543,10 @@ def run_pkt_device_noalloc(d_offsets: int, n_plus_1: int, d_neighbours: int, wid
 class PktTuning:
     """The engine's performance knobs (``sparx_tuning``); none changes a result."""
     merge_ratio: int = 8
-    hub_min_degree: int = 1024
+    hub_min_degree: int = 0
     sample_min: int = 64
     support_kernel: int = 1
-    compact_pct: int = 85
+    compact_pct: int = 76
     hash_min_degree: int = 128
     sup_hash_min: int = 0
     relabel: int = 0
