@@ -4,12 +4,11 @@
 // slot s maps to the new slot rmap[s].  Rows are sorted by id, and within a
 // degree bucket the new ids keep the old order, so each new row is the old
 // row stably partitioned by its neighbours' buckets: no sort of the slots is
-// needed.  On R-MAT-22 the same engine ran the bucket-ordered copy of the
-// graph 32 ms faster than the original (support 86.5 -> 80.6 ms, peel 340.6
-// -> 315.1 ms): edges of similar-degree vertices sit together, so the peel's
-// random state and row reads fall on far fewer lines.  Below 2^26 slots it
-// costs more than it saves (R-MAT-20 and 21: peel 5-6 ms slower), so the
-// tuning turns it on only for large skewed graphs.
+// needed.  Edges of similar-degree vertices sit together, so the peel's random
+// state and row reads fall on far fewer lines, and the copy is oriented by id
+// alone, which shortens the support pass's searches: R-MAT-22 (orientation +
+// support + peel) 6.3 + 50.8 + 249.9 -> 9.0 + 31.1 + 215.6 ms, R-MAT-21 with edge
+// factor 12 2.0 + 14.2 + 87.7 -> 4.4 + 8.8 + 82.4.
 //   k_vertex_keys       ((member << 5 | bucket) << 32 | id) per vertex, for the
 //                       radix passes (one for a single graph)
 //   k_vertex_order      new id and new degree per vertex

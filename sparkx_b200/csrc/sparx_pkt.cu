@@ -625,7 +625,7 @@ struct SupportIndex {
   uint32_t rank_min = Tuning{}.sample_min;
 };
 
-int launch_support(int sm_count, uint32_t support_kernel, uint32_t n, uint64_t m, uint32_t max_dplus,
+int launch_support(int sm_count, uint32_t support_kernel, bool by_id, uint32_t n, uint64_t m, uint32_t max_dplus,
                    const uint32_t* opos, const uint32_t* ocol, const uint32_t* osrc, int2* es,
                    unsigned long long* spref, unsigned long long* tiles, Counters* cnt, uint32_t* heavy_list,
                    cudaStream_t s, uint32_t* launches, const SupportIndex& X,
@@ -663,7 +663,8 @@ int launch_support(int sm_count, uint32_t support_kernel, uint32_t n, uint64_t m
                                                                &cnt->table_big);
     *launches += 2;
   }
-  exclusive_scan<unsigned long long>(SupportWork{opos, osrc, ocol}, m, spref, tiles, &cnt->grand, s);
+  if (by_id) exclusive_scan<unsigned long long>(SupportWork<true>{opos, osrc, ocol}, m, spref, tiles, &cnt->grand, s);
+  else exclusive_scan<unsigned long long>(SupportWork<false>{opos, osrc, ocol}, m, spref, tiles, &cnt->grand, s);
   const int g = sm_count * kSupBlocks;
   const uint32_t mm = (uint32_t)m;
   auto go = [&](auto kernel) {
@@ -671,9 +672,13 @@ int launch_support(int sm_count, uint32_t support_kernel, uint32_t n, uint64_t m
                              hpool, hash_min);
   };
   if (hpool && hash_min) {
-    if (mu) go(k_support_balanced<true, true>); else go(k_support_balanced<false, true>);
+    if (mu) go(k_support_balanced<true, true, false>);
+    else if (by_id) go(k_support_balanced<false, true, true>);
+    else go(k_support_balanced<false, true, false>);
   } else {
-    if (mu) go(k_support_balanced<true, false>); else go(k_support_balanced<false, false>);
+    if (mu) go(k_support_balanced<true, false, false>);
+    else if (by_id) go(k_support_balanced<false, false, true>);
+    else go(k_support_balanced<false, false, false>);
   }
   *launches += 4;
   CU(cudaMemcpyAsync(&cnt->elements, spref + m, 8, cudaMemcpyDeviceToDevice, s));
@@ -979,6 +984,11 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
   uint32_t* mu = nullptr;
   Counters hc;
   uint32_t m32 = 0;
+  // the relabelled copy's ids ascend with the degree's power of two: oriented by
+  // id alone its lists are no longer than by degree to speak of (R-MAT-19: 525
+  // entries at most against 506), and the support pass searches 0.62 of the
+  // elements (SupportWork)
+  bool by_id = false;
   for (int pass = 0;; ++pass) {
     // the degree signature, and the rows the orientation gives a block each
     if (pass > 0) {
@@ -989,8 +999,12 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
     k_degree_stats<<<grid_for(N, 256, E.sm_count * 8), 256, 0, s>>>(J.off, N, big, &cnt->big_count, &cnt->dmax,
                                                                     &cnt->heavy, err);
     J.launches += 1;
-    k_orient_count<<<vgrid, 256, 0, s>>>(J.off, J.nbr, N, dplus, &cnt->self_loops, err, &cnt->max_dplus, big,
-                                         &cnt->big_count);
+    if (by_id)
+      k_orient_count_by_id<<<grid_for(N, 256, E.sm_count * 16), 256, 0, s>>>(J.off, J.nbr, N, dplus, &cnt->self_loops,
+                                                                             &cnt->max_dplus);
+    else
+      k_orient_count<<<vgrid, 256, 0, s>>>(J.off, J.nbr, N, dplus, &cnt->self_loops, err, &cnt->max_dplus, big,
+                                           &cnt->big_count);
     J.launches += 1;
     exclusive_scan<uint32_t>(LoadU32{dplus}, N, opos, at<uint32_t>(E, L.tiles), (uint32_t*)&cnt->grand, s);
     J.launches += 4;
@@ -1018,6 +1032,7 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
       if (rc == SPARX_E_OOM) break;
       if (rc) return rc;
       smap = const_cast<uint32_t*>(J.smap);
+      by_id = true;
       // the next pass counts them again
       CU(cudaMemsetAsync(&cnt->self_loops, 0, 8, s));
       CU(cudaMemsetAsync(&cnt->max_dplus, 0, 4, s));
@@ -1076,8 +1091,9 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
   }
   {
     uint32_t* owner = at<uint32_t>(E, L.q0);  // in-slot owners; the q buffers are idle until the peel
-    k_orient_fill<<<vgrid, 256, 0, s>>>(J.off, J.nbr, N, opos, ocol, osrc, row0, owner, big, &cnt->big_count,
-                                        const_cast<uint32_t*>(X.hdr ? X.oname : nullptr));
+    const auto fill = by_id ? k_orient_fill<true> : k_orient_fill<false>;
+    fill<<<vgrid, 256, 0, s>>>(J.off, J.nbr, N, opos, ocol, osrc, row0, owner, big, &cnt->big_count,
+                               const_cast<uint32_t*>(X.hdr ? X.oname : nullptr));
     k_orient_reverse<<<grid_for(Ws, 256, E.sm_count * 16), 256, 0, s>>>(J.nbr, owner, Ws, opos, ocol, row0, err);
     if (J.multi) {
       // multiplicity per edge id from its out-slot; the in-slot must agree
@@ -1149,7 +1165,7 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
     if (!O.support_kernel && !sup_hash_min && hc.max_dplus <= kPairList &&
         (form == 1 || (!tuned && m <= kPairEdges)))
       form = 0;
-    int rc = launch_support(E.sm_count, form, N, m,
+    int rc = launch_support(E.sm_count, form, by_id, N, m,
                             hc.max_dplus, opos, ocol, osrc, es, at<unsigned long long>(E, L.q0),
                             at<unsigned long long>(E, L.tiles), cnt, at<uint32_t>(E, L.act0), s, &J.launches, X, mu, spool, sup_hash_min);
     if (rc) return rc;
@@ -3535,7 +3551,7 @@ int run_noalloc(const uint64_t* d_offsets, uint64_t n_plus_1, const uint32_t* d_
     X.pool = (unsigned long long*)P(L.qd0);
     X.chunks = (uint2*)P(L.act0);
   }
-  k_orient_fill<<<vgrid, 256, 0, s>>>(off, d_nbr, N, opos, ocol, osrc, row0, (uint32_t*)P(L.q0), big,
+  k_orient_fill<false><<<vgrid, 256, 0, s>>>(off, d_nbr, N, opos, ocol, osrc, row0, (uint32_t*)P(L.q0), big,
                                       &cnt->big_count, const_cast<uint32_t*>(X.hdr ? X.oname : nullptr));
   k_orient_reverse<<<grid_for(width, 256, sm * 16), 256, 0, s>>>(d_nbr, (uint32_t*)P(L.q0), width, opos, ocol,
                                                                 row0, err);
@@ -3543,7 +3559,7 @@ int run_noalloc(const uint64_t* d_offsets, uint64_t n_plus_1, const uint32_t* d_
   CU(cudaMemsetAsync(es, 0, 8 * std::max<uint64_t>(m, 1), s));
   {
     uint32_t launches = 0;
-    rc = launch_support(sm, hc.max_dplus <= kPairList ? 0 : 1, N, m, hc.max_dplus, opos, ocol, osrc, es, (unsigned long long*)P(L.q0),
+    rc = launch_support(sm, hc.max_dplus <= kPairList ? 0 : 1, false, N, m, hc.max_dplus, opos, ocol, osrc, es, (unsigned long long*)P(L.q0),
                         (unsigned long long*)P(L.tiles), cnt, (uint32_t*)P(L.act0), s, &launches, X);
     if (rc) return rc;
   }
