@@ -259,7 +259,9 @@ typedef struct sparx_tuning {
                                in (floor(log2 degree), id) order (a union's members each within their own
                                id range) before the decomposition, for locality;
                                results are returned in the caller's slot order (0; 1 for keys of
-                               2^26 slots or more with a quarter of them in rows of degree >= 256) */
+                               2^26 slots or more with a quarter of them in rows of degree >= 256.
+                               Keys without an entry are also run with 1 from 2^23 slots with half of
+                               them in such rows: sparx_tuning_last reports what a launch used) */
 } sparx_tuning;
 
 int sparx_tuning_default(sparx_tuning* t);

@@ -119,10 +119,9 @@ Tuning default_tuning(const TuneKey& k) {
   Tuning t;
   if (k.skew8 == 0 && k.log_dmax >= 7 && k.log_dmax <= 8) t.support_kernel = 2;
   // large skewed graphs (2^26 slots or more, a quarter of them or more in rows
-  // of degree >= 256) run on the degree-bucket relabelled CSR: R-MAT-22 / 23
-  // 322 -> 277, 685 -> 573 ms, R-MAT-22 with edge factor 8 106 -> 103; below
-  // 2^26 slots it is a matter of the density (R-MAT-21 with edge factor 5 / 8 /
-  // 12 35.8 -> 39.4, 59.2 -> 59.3, 106.6 -> 102.6; R-MAT-17 .. 19 up to 11% slower)
+  // of degree >= 256) run on the degree-bucket relabelled CSR: R-MAT-22 with edge
+  // factor 15 / 8 309 -> 258, 105.0 -> 96.5 ms; smaller ones where resolve_tuning
+  // says so
   if (k.skew8 >= 2 && k.log_w >= 26) t.relabel = 1;
   return t;
 }
@@ -185,6 +184,13 @@ Tuning resolve_tuning(const TuneKey& key, bool* tuned = nullptr) {
     found = it != g_tune.end();
     if (found) t = it->second;
   }
+  // Without a choice for the key, half the slots in rows of degree >= 256 are
+  // enough from 2^23 slots on: R-MAT-21 (edge factor 12 / 8) 104.7 -> 96.6, 58.6 ->
+  // 55.6 ms, R-MAT-20 (15 / 12) 79.8 -> 75.7, 59.4 -> 57.2, R-MAT-19 (15) 47.2 ->
+  // 46.1; with three eighths it is 2-3% slower (R-MAT-21 / 20 / 19 with edge
+  // factor 5 / 8 / 12 34.9 -> 36.1, 36.6 -> 37.3, 35.8 -> 36.5), and below 2^22
+  // slots as well (R-MAT-17 20.1 -> 20.7).
+  if (!found && key.skew8 >= 4 && key.log_w >= 23) t.relabel = 1;
   if (tuned) *tuned = found;
   g_tune_last = t;
   g_tune_last_key = key;
