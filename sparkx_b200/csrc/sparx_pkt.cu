@@ -2767,8 +2767,8 @@ int mtx_to_csr(const char* text, uint64_t len, uint64_t* offsets_out, uint64_t o
   const int pgrid = grid_for(lines, 256, E.sm_count * 16);
   if (lines) {
     k_mtx_fill_lines<<<grid_for(chunks, 256, E.sm_count * 16), 256, 0, s>>>(body, blen, cpref, starts);
-    k_mtx_parse<false><<<pgrid, 256, 0, s>>>(body, blen, starts, lines, H.n, H.symmetric, count, nullptr, nullptr,
-                                             derr, dcnt + 1);
+    k_mtx_parse<<<pgrid, 256, 0, s>>>(body, blen, starts, lines, H.n, H.symmetric, count,
+                                      at<unsigned long long>(E, o_kb), derr, dcnt + 1);
   }
   uint32_t herr = 0;
   unsigned long long bad = 0, edges = 0;
@@ -2802,15 +2802,12 @@ int mtx_to_csr(const char* text, uint64_t len, uint64_t* offsets_out, uint64_t o
   uint32_t* deg = at<uint32_t>(E, o_deg);
   unsigned long long* doff = at<unsigned long long>(E, o_off);
   unsigned long long* dnbr = at<unsigned long long>(E, o_nbr);
-  if (lines)
-    k_mtx_parse<true><<<pgrid, 256, 0, s>>>(body, blen, starts, lines, H.n, H.symmetric, nullptr, atp, ka, derr,
-                                            dcnt + 1);
-  // sort by (row, column): the low 32 bits (columns), then the high (rows),
-  // only the bits that vertex ids < n use
+  // keys row << bits | column with only the bits that vertex ids < n use, sorted
+  // a digit at a time across both parts
   const int bits = H.n > 1 ? 64 - __builtin_clzll(H.n - 1) : 1;
+  if (lines) k_mtx_emit<<<pgrid, 256, 0, s>>>(count, kb, atp, lines, bits, ka);
   std::vector<int> shifts;
-  for (int b = 0; b < bits; b += 8) shifts.push_back(b);
-  for (int b = 0; b < bits; b += 8) shifts.push_back(32 + b);
+  for (int b = 0; b < 2 * bits; b += 8) shifts.push_back(b);
   const uint32_t blocks = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(rblocks, (edges + 4095) / 4096));
   unsigned long long *src = ka, *dst = kb;
   if (edges > 1) {
@@ -2822,9 +2819,8 @@ int mtx_to_csr(const char* text, uint64_t len, uint64_t* offsets_out, uint64_t o
     }
   }
   CU(cudaMemsetAsync(deg, 0, 4 * (H.n + 1), s));
-  if (edges) k_mtx_rows<<<grid_for(edges, 256, E.sm_count * 16), 256, 0, s>>>(src, edges, deg);
+  if (edges) k_mtx_rows<<<grid_for(edges, 256, E.sm_count * 16), 256, 0, s>>>(src, edges, bits, deg, dnbr);
   exclusive_scan<unsigned long long>(LoadCount{deg}, H.n, doff, tiles, dcnt, s);
-  if (edges) k_mtx_columns<<<grid_for(edges, 256, E.sm_count * 16), 256, 0, s>>>(src, edges, dnbr);
   if (H.n == 0) CU(cudaMemsetAsync(doff, 0, 8, s));
   rc = download(E, offsets_out, doff, 8 * (H.n + 1), s);
   if (rc) return rc;
