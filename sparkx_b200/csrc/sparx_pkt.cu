@@ -1186,7 +1186,7 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
   }
   if (J.support_only && J.clustering) {
     k_clustering<<<vgrid, 256, 0, s>>>(J.off, row0, es, N, O.support_mode == SPARX_SUPPORT_U8, (double*)J.out,
-                                       &cnt->cc_possible, &cnt->cc_local, &cnt->cc_slots, mult2);
+                                       &cnt->cc_possible, &cnt->cc_local, &cnt->cc_slots, mult2, big, &cnt->big_count);
     J.launches += 1;
     CU(cudaEventRecord(E.tev[4], s));
     CU(cudaEventRecord(E.tev[5], s));
