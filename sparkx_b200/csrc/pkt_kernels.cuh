@@ -475,6 +475,12 @@ __global__ void __launch_bounds__(256) k_degree_stats(const uint32_t* __restrict
   }
 }
 
+// Entries of a row read side by side by a lane (or a warp): what bounds the two
+// passes over the rows is the latency of an entry and then its vertex's offsets.
+// One / two / four: R-MAT-19 (with its degree-ordered copy) 1.78 / 1.50 / 1.35 ms of
+// orientation, R-MAT-17 285 / 230 / 225 us, ER n = 10^5, m = 10^6 121 / 118 / 117.
+constexpr int kOrientWays = 4;
+
 // Kernel B1: per-row validation + oriented out-degree.
 //   rows strictly ascending (equal -> multigraph), counts self-loops, and
 //   dplus[u] = #{v in N(u): v != u, rank(u) < rank(v)}.
@@ -500,16 +506,25 @@ __global__ void __launch_bounds__(256) k_orient_count(const uint32_t* __restrict
     uint32_t cnt = 0;
     if (u < n && e - b <= kLaneRow) {
       uint32_t prev = 0;
-      for (uint32_t s = b; s < e; ++s) {
-        const uint32_t v = __ldg(nbr + s);
-        if (s > b && prev < n) {  // the pair (prev, v), judged as the warp path does
-          if (v == prev) flags |= kErrMulti;
-          else if (v < prev) flags |= kErrUnsorted;
+      for (uint32_t s = b; s < e; s += kOrientWays) {
+        uint32_t vs[kOrientWays], dv[kOrientWays];
+#pragma unroll
+        for (int i = 0; i < kOrientWays; ++i) vs[i] = s + i < e ? __ldg(nbr + s + i) : kInvalid;
+#pragma unroll
+        for (int i = 0; i < kOrientWays; ++i) dv[i] = vs[i] < n ? deg_of(off, vs[i]) : 0u;
+#pragma unroll
+        for (int i = 0; i < kOrientWays; ++i) {
+          if (s + i >= e) break;
+          const uint32_t v = vs[i];
+          if (s + i > b && prev < n) {  // the pair (prev, v), judged as the warp path does
+            if (v == prev) flags |= kErrMulti;
+            else if (v < prev) flags |= kErrUnsorted;
+          }
+          prev = v;
+          if (v >= n) { flags |= kErrRange; continue; }
+          if (v == u) { selfc++; continue; }
+          cnt += rank_less(e - b, u, dv[i], v);
         }
-        prev = v;
-        if (v >= n) { flags |= kErrRange; continue; }
-        if (v == u) { selfc++; continue; }
-        cnt += rank_less(e - b, u, deg_of(off, v), v);
       }
     }
     const bool blk = u < n && e - b > kWarpRow;  // counted below, a block per row
@@ -520,16 +535,28 @@ __global__ void __launch_bounds__(256) k_orient_count(const uint32_t* __restrict
       const uint32_t bu = base + j, bb = __shfl_sync(kFull, b, j), be = __shfl_sync(kFull, e, j);
       const uint32_t du = be - bb;
       uint32_t c = 0;
-      for (uint32_t s = bb + lane; s < be; s += 32) {
-        const uint32_t v = __ldg(nbr + s);
-        if (v >= n) { flags |= kErrRange; continue; }
-        if (s + 1 < be) {
-          const uint32_t nx = __ldg(nbr + s + 1);
-          if (nx == v) flags |= kErrMulti;
-          else if (nx < v) flags |= kErrUnsorted;
+      for (uint32_t s0 = bb + lane; s0 < be; s0 += 32 * kOrientWays) {
+        uint32_t vs[kOrientWays], nx[kOrientWays], dv[kOrientWays];
+#pragma unroll
+        for (int i = 0; i < kOrientWays; ++i) {
+          const uint32_t s = s0 + 32 * i;
+          vs[i] = s < be ? __ldg(nbr + s) : kInvalid;
+          nx[i] = s < be && s + 1 < be ? __ldg(nbr + s + 1) : kInvalid;
         }
-        if (v == bu) { selfc++; continue; }
-        c += rank_less(du, bu, deg_of(off, v), v);
+#pragma unroll
+        for (int i = 0; i < kOrientWays; ++i) dv[i] = vs[i] < n ? deg_of(off, vs[i]) : 0u;
+#pragma unroll
+        for (int i = 0; i < kOrientWays; ++i) {
+          const uint32_t s = s0 + 32 * i, v = vs[i];
+          if (s >= be) break;
+          if (v >= n) { flags |= kErrRange; continue; }
+          if (s + 1 < be) {
+            if (nx[i] == v) flags |= kErrMulti;
+            else if (nx[i] < v) flags |= kErrUnsorted;
+          }
+          if (v == bu) { selfc++; continue; }
+          c += rank_less(du, bu, dv[i], v);
+        }
       }
 #pragma unroll
       for (int d = 16; d > 0; d >>= 1) c += __shfl_xor_sync(kFull, c, d);
@@ -638,23 +665,34 @@ __global__ void __launch_bounds__(256) k_orient_fill(const uint32_t* __restrict_
     if (u < n) { b = __ldg(off + u); e = __ldg(off + u + 1); }
     if (u < n && e - b <= kLaneRow) {
       uint32_t p = __ldg(opos + u);
-      for (uint32_t s = b; s < e; ++s) {
-        const uint32_t v = __ldg(nbr + s);
-        uint32_t own = kInvalid;
-        const uint32_t name = v < n ? __ldg(off + v) : 0u;
-        if (v == u || v >= n) {
-          row0[s] = make_pair(name, kInvalid);
-        } else if (kById ? u < v : rank_less(e - b, u, __ldg(off + v + 1) - name, v)) {
-          ocol[p] = v;
-          osrc[p] = u;
-          if (oname) oname[p] = name;
-          row0[s] = make_pair(name, p);
-          ++p;
-        } else {
-          own = u;
-          pair_name(row0, s) = name;
+      for (uint32_t s0 = b; s0 < e; s0 += kOrientWays) {
+        uint32_t vs[kOrientWays], names[kOrientWays], ends[kOrientWays];
+#pragma unroll
+        for (int i = 0; i < kOrientWays; ++i) vs[i] = s0 + i < e ? __ldg(nbr + s0 + i) : kInvalid;
+#pragma unroll
+        for (int i = 0; i < kOrientWays; ++i) {
+          names[i] = vs[i] < n ? __ldg(off + vs[i]) : 0u;
+          ends[i] = !kById && vs[i] < n ? __ldg(off + vs[i] + 1) : 0u;
         }
-        owner[s] = own;
+#pragma unroll
+        for (int i = 0; i < kOrientWays; ++i) {
+          const uint32_t s = s0 + i, v = vs[i], name = names[i];
+          if (s >= e) break;
+          uint32_t own = kInvalid;
+          if (v == u || v >= n) {
+            row0[s] = make_pair(name, kInvalid);
+          } else if (kById ? u < v : rank_less(e - b, u, ends[i] - name, v)) {
+            ocol[p] = v;
+            osrc[p] = u;
+            if (oname) oname[p] = name;
+            row0[s] = make_pair(name, p);
+            ++p;
+          } else {
+            own = u;
+            pair_name(row0, s) = name;
+          }
+          owner[s] = own;
+        }
       }
     }
     unsigned big = __ballot_sync(kFull, u < n && e - b > kLaneRow && e - b <= kWarpRow);
@@ -664,28 +702,39 @@ __global__ void __launch_bounds__(256) k_orient_fill(const uint32_t* __restrict_
       const uint32_t bu = base0 + j, bb = __shfl_sync(kFull, b, j), be = __shfl_sync(kFull, e, j);
       const uint32_t du = be - bb;
       uint32_t p0 = __ldg(opos + bu);
-      for (uint32_t s0 = bb; s0 < be; s0 += 32) {
-        const uint32_t s = s0 + lane;
-        bool out = false;
-        uint32_t v = 0, name = 0;
-        if (s < be) {
-          v = __ldg(nbr + s);
-          uint32_t own = kInvalid;
-          if (v < n) name = __ldg(off + v);
-          if (v == bu || v >= n) row0[s] = make_pair(name, kInvalid);
-          else if (kById ? bu < v : rank_less(du, bu, __ldg(off + v + 1) - name, v)) out = true;
-          else { own = bu; pair_name(row0, s) = name; }
-          owner[s] = own;
+      for (uint32_t s0 = bb; s0 < be; s0 += 32 * kOrientWays) {
+        uint32_t vs[kOrientWays], names[kOrientWays], ends[kOrientWays];
+#pragma unroll
+        for (int i = 0; i < kOrientWays; ++i) {
+          const uint32_t s = s0 + 32 * i + lane;
+          vs[i] = s < be ? __ldg(nbr + s) : kInvalid;
         }
-        const unsigned bal = __ballot_sync(kFull, out);
-        if (out) {
-          const uint32_t p = p0 + __popc(bal & ((1u << lane) - 1));
-          ocol[p] = v;
-          osrc[p] = bu;
-          if (oname) oname[p] = name;
-          row0[s] = make_pair(name, p);
+#pragma unroll
+        for (int i = 0; i < kOrientWays; ++i) {
+          names[i] = vs[i] < n ? __ldg(off + vs[i]) : 0u;
+          ends[i] = !kById && vs[i] < n ? __ldg(off + vs[i] + 1) : 0u;
         }
-        p0 += __popc(bal);
+#pragma unroll
+        for (int i = 0; i < kOrientWays; ++i) {
+          const uint32_t s = s0 + 32 * i + lane, v = vs[i], name = names[i];
+          bool out = false;
+          if (s < be) {
+            uint32_t own = kInvalid;
+            if (v == bu || v >= n) row0[s] = make_pair(name, kInvalid);
+            else if (kById ? bu < v : rank_less(du, bu, ends[i] - name, v)) out = true;
+            else { own = bu; pair_name(row0, s) = name; }
+            owner[s] = own;
+          }
+          const unsigned bal = __ballot_sync(kFull, out);
+          if (out) {
+            const uint32_t p = p0 + __popc(bal & ((1u << lane) - 1));
+            ocol[p] = v;
+            osrc[p] = bu;
+            if (oname) oname[p] = name;
+            row0[s] = make_pair(name, p);
+          }
+          p0 += __popc(bal);
+        }
       }
     }
   }
