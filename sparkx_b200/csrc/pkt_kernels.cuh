@@ -314,20 +314,8 @@ __device__ __forceinline__ unsigned long long warp_incl_scan(unsigned long long 
 }
 
 // ---------------------------------------------------------------------------
-// Kernel A: narrowing (u64 ids -> u32) with range check.  Grid-stride.
-__global__ void k_narrow_ids(const unsigned long long* __restrict__ src, uint32_t* __restrict__ dst,
-                             unsigned long long count, unsigned long long n_limit, uint32_t base,
-                             uint32_t* __restrict__ err) {
-  unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
-  bool bad = false;
-  for (; i < count; i += stride) {
-    unsigned long long x = src[i];
-    bad |= x >= n_limit;
-    dst[i] = (uint32_t)x + base;
-  }
-  if (bad) atomicOr(err, kErrRange);
-}
+// Kernel A: ids and offsets in, checked (u64 ids are narrowed by the host as it
+// fills the staging buffers).
 
 // u32 ids: range check, optionally copying with a base shift (dst may be null)
 __global__ void k_range_ids(const uint32_t* __restrict__ ids, uint32_t* __restrict__ dst,

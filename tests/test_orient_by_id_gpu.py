@@ -64,3 +64,16 @@ def test_union():
             P.tuning_clear()
         for w, (got, _, status) in zip(want, res):
             assert status == 0 and np.array_equal(got, w), s
+
+
+@pytest.mark.parametrize("d", [31, 32, 33, 127, 128, 129, 257, 2047, 2048, 2049, 3073, 20_000])
+def test_row_lengths_of_the_copy(d):
+    """Two hubs with rows of d (a warp's, a block's, parts of both) over a ring of mixed degrees."""
+    ring = np.arange(d)
+    edges = [(d, i) for i in range(d)] + [(d + 1, i) for i in range(0, d, 2)] + [(int(i), int((i + 1) % d)) for i in ring]
+    edges += [(int(i), int((i + k) % d)) for i in ring[::7] for k in range(2, 9)]
+    edges += [(u, v) for u in range(d + 2, d + 14) for v in range(d + 2, u)] + [(d, d + 1)]
+    g = gen.from_edges(d + 14, [(u, v) for u, v in edges if u != v])
+    want, st0 = _run(g, relabel=0)
+    got, st = _run(g, relabel=1)
+    assert np.array_equal(got, want) and st.triangles == st0.triangles
