@@ -77,3 +77,14 @@ def test_row_lengths_of_the_copy(d):
     want, st0 = _run(g, relabel=0)
     got, st = _run(g, relabel=1)
     assert np.array_equal(got, want) and st.triangles == st0.triangles
+
+
+@pytest.mark.parametrize("scale,ef,relabels", [(17, 16, 0), (19, 6, 0), (19, 18, 1)])
+def test_rule_for_keys_without_an_entry(scale, ef, relabels):
+    g = gen.rmat(scale, ef, seed=11)
+    P.tuning_clear()
+    got, st = P.run_pkt(g.offsets, g.neighbours, O32)
+    used, key = P.tuning_last()
+    assert used.relabel == relabels == int(key[0] >= 23 and key[2] >= 4)
+    want, st0 = _run(g, relabel=1 - relabels)
+    assert np.array_equal(got, want) and st.triangles == st0.triangles
