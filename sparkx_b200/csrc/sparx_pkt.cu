@@ -1,7 +1,8 @@
 // Host side of the B200 PKT k-truss engine: C ABI (include/sparx_pkt.h),
 // device workspace, pinned-staging upload, kernel sequencing and the
 // device-resident peel loop (a CUDA graph with a conditional WHILE node whose
-// body is four wave kernels; the last block of each wave plans the next).
+// body is wave kernels, the last block of each planning the next, and a cluster
+// that runs the small waves).
 #include <algorithm>
 #include <cctype>
 #include <atomic>
