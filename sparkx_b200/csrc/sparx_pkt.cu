@@ -3545,10 +3545,10 @@ int run_noalloc(const uint64_t* d_offsets, uint64_t n_plus_1, const uint32_t* d_
     return SPARX_E_TOO_LARGE;
   }
   // the support pass's rank index, in arrays that are idle until the peel (the
-  // headers where one per vertex fits: no more vertices than slots)
+  // headers, 8 bytes a vertex, where they fit a queue's descriptors, 16 a pair of slots)
   SupportIndex X;
   X.oname = ocol;
-  if (hc.max_dplus >= X.rank_min && N <= width) {
+  if (hc.max_dplus >= X.rank_min && N <= 2 * (width / 2)) {
     X.oname = (uint32_t*)P(L.act1);
     X.hdr = (unsigned long long*)P(L.qd1);
     X.pool = (unsigned long long*)P(L.qd0);
