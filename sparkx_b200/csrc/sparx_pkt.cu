@@ -902,10 +902,11 @@ SortedBufs radix_sort(int sm_count, unsigned long long* ka, unsigned long long* 
 // become the new rows, J.smap the caller slot -> new slot map the finalize
 // reads through.  `big` / `big_count`:
 // the rows longer than kWarpRow (listed by the orientation pass).  Everything
-// lives in the second workspace.
+// lives in the second workspace: `used` of its bytes, SPARX_E_OOM where they are
+// more than `room` or than the device has (the graph is left as it was).
 static_assert(kRelabelWarpRow == kWarpRow, "the relabel's block rows are the orientation's big-row list");
 int relabel_graph(Engine& E, UnionJob& J, uint32_t N, uint64_t W, const uint32_t* big, const uint32_t* big_count,
-                  cudaStream_t s) {
+                  uint64_t room, uint64_t* used, cudaStream_t s) {
   const uint32_t blocks_max = (uint32_t)E.sm_count * 4;
   const uint64_t scan_items = std::max<uint64_t>(256ull * blocks_max + 1, N + 1ull);
   size_t p = 0;
@@ -919,8 +920,10 @@ int relabel_graph(Engine& E, UnionJob& J, uint32_t N, uint64_t W, const uint32_t
                o_hist = take(4ull * 256 * blocks_max), o_hstart = take(4ull * (256 * blocks_max + 1)),
                o_tiles = take(4 * (scan_items / kScanTile + 4)), o_grand = take(4),
                o_mvb = take(4ull * J.members.size());
+  if (p > room) return SPARX_E_OOM;
   int rc = ensure_ws2(E, p);
   if (rc) return rc;
+  *used = p;
   char* b = E.ws2;
   uint32_t* off_r = (uint32_t*)(b + o_off);
   uint32_t* nbr_r = (uint32_t*)(b + o_nbr);
@@ -989,6 +992,7 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
   uint32_t* mult2 = nullptr;
   uint32_t* smap = nullptr;
   uint32_t* mu = nullptr;
+  uint64_t ws2_used = 0;                // bytes of the second workspace this launch holds
   Counters hc;
   uint32_t m32 = 0;
   // the relabelled copy's ids ascend with the degree's power of two: oriented by
@@ -1030,12 +1034,14 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
       J.members[0].m = m32;
     }
     if (pass == 0) J.slot_self_loops = hc.self_loops;
-    // (batched unions: the packer counted the relabelled copy in their budget)
     if (pass == 0 && hc.err == 0 && N > 1 && W > 0 && !J.support_only && !J.prep_only && !J.hook &&
         resolve_tuning(tune_key(hc.dmax, hc.heavy, W, W)).relabel) {
       // a sound simple graph: orient its degree-ordered copy instead (when the
-      // device has no room for the copy, the caller's ids are used as they are)
-      int rc = relabel_graph(E, J, N, W, big, &cnt->big_count, s);
+      // launch's budget or the device has no room for the copy, the caller's ids
+      // are used as they are; the packer of batched unions counts the copy, but
+      // not for a graph that fits its budget only alone)
+      const uint64_t room = !J.budget ? ~0ull : J.budget - std::min<uint64_t>(J.budget, L.total);
+      int rc = relabel_graph(E, J, N, W, big, &cnt->big_count, room, &ws2_used, s);
       if (rc == SPARX_E_OOM) break;
       if (rc) return rc;
       smap = const_cast<uint32_t*>(J.smap);
@@ -1054,6 +1060,7 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
                  o_smap = o_mult + align_up(4 * W), o_mu = o_smap + align_up(4 * W), total = o_mu + align_up(4 * Mx);
     int rc = ensure_ws2(E, total);
     if (rc) return rc;
+    ws2_used = total;
     uint32_t* off2 = (uint32_t*)(E.ws2 + o_off);
     uint32_t* nbr2 = (uint32_t*)(E.ws2 + o_nbr);
     mult2 = (uint32_t*)(E.ws2 + o_mult);
@@ -1137,7 +1144,7 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
     // long rows' chunks, and lists with tables past a warp's shared slice (more
     // than kTableSmem / 2 entries: fewer of them)
     const size_t big_b = align_up(sizeof(uint2) * rank_chunks_max(W));
-    if ((index || sup_hash) && ((J.budget && L.total + pool_b + 2 * qh_b + spool_b + big_b > J.budget) ||
+    if ((index || sup_hash) && ((J.budget && L.total + ws2_used + pool_b + 2 * qh_b + spool_b + big_b > J.budget) ||
                                 ensure_ws3(E, pool_b + 2 * qh_b + spool_b + big_b) != SPARX_OK)) {
       index = sup_hash = false;
       pool_b = qh_b = spool_b = 0;
