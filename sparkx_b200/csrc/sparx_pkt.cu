@@ -22,11 +22,11 @@
 #include <vector>
 
 #include <omp.h>
-#include <sys/mman.h>
 
 #include "../../include/sparx_pkt.h"
 #include "pkt_kernels.cuh"
 #include "mtx_kernels.cuh"
+#include "prefault.h"
 #include "relabel_kernels.cuh"
 
 using namespace sparx;
@@ -535,36 +535,6 @@ int upload_ids(Engine& E, const void* host, int bits, uint64_t count, uint32_t* 
   }
   return SPARX_OK;
 }
-
-// The pages of large result buffers, made present while the device computes: a
-// fresh buffer's page faults otherwise fall into its download (125 MB of supports:
-// 4.9 -> 3.1 ms).  Contents are left alone; a kernel without MADV_POPULATE_WRITE
-// faults as before.
-class Prefault {
- public:
-  void add(void* p, size_t bytes) {
-    const uintptr_t page = 4096, b = ((uintptr_t)p + page - 1) & ~(page - 1), e = ((uintptr_t)p + bytes) & ~(page - 1);
-    for (uintptr_t at = b; at < e; at += kPart) parts.push_back({at, std::min<size_t>(kPart, e - at)});
-  }
-  void start() {
-    if (parts.size() * kPart < kLeast) return;
-    for (int i = 0; i < kThreads; ++i)
-      threads.emplace_back([this] {
-        for (size_t k; (k = next++) < parts.size();)
-          madvise((void*)parts[k].first, parts[k].second, MADV_POPULATE_WRITE);
-      });
-  }
-  ~Prefault() {
-    for (auto& t : threads) t.join();
-  }
-
- private:
-  static constexpr int kThreads = 4;
-  static constexpr size_t kPart = 4ull << 20, kLeast = 16ull << 20;
-  std::vector<std::pair<uintptr_t, size_t>> parts;
-  std::atomic<size_t> next{0};
-  std::vector<std::thread> threads;
-};
 
 // Pieces through the ring: fetch(c, buffer) issues piece c's copy to the host,
 // take(c, buffer) empties it; half of the ring is on its way while another piece
@@ -1725,12 +1695,10 @@ int run_host(const uint64_t* offsets, uint64_t n_plus_1, const void* nbrs, int b
   // one narrowing kernel per offsets chunk (the ids are narrowed by the host)
   const uint64_t off_chunk = piece_bytes(n_plus_1 * 8) / 8;
   J.launches += (uint32_t)((n_plus_1 + off_chunk - 1) / off_chunk);
-  {
-    Prefault ready;
-    ready.add(out_host, out_bytes);
-    ready.start();
-    rc = kcore ? run_kcore(E, J, O, s) : run_union(E, J, O, s);
-  }
+  Prefault ready;  // until the call ends: the download follows it through the buffer
+  ready.add(out_host, out_bytes);
+  ready.start();
+  rc = kcore ? run_kcore(E, J, O, s) : run_union(E, J, O, s);
   if (rc) {
     fill_stats(J, 0, stats);
     return rc;
@@ -1921,12 +1889,10 @@ int run_batch_union(Engine& E, std::vector<HostMember>& hm, const Opts& O, int* 
   CU(cudaEventRecord(E.tev[0], s));
   rc = upload_union(E, hm, J.members, N, Wt, J.off, (uint32_t*)J.nbr, s);
   if (rc) { fail_all(rc); return rc; }
-  {
-    Prefault ready;
-    for (const HostMember& h : hm) ready.add(h.out, (O.out_bits / 8) * h.w);
-    ready.start();
-    rc = run_union(E, J, O, s);
-  }
+  Prefault ready;
+  for (const HostMember& h : hm) ready.add(h.out, (O.out_bits / 8) * h.w);
+  ready.start();
+  rc = run_union(E, J, O, s);
   if (rc == SPARX_E_INVALID_CSR || rc == SPARX_E_MULTIGRAPH || rc == SPARX_E_OVERFLOW_U8 ||
       rc == SPARX_E_TOO_LARGE) {
     if (G == 1) {
