@@ -684,7 +684,7 @@ def _mtx_declared(data: bytes) -> tuple[int, int]:
         end = data.find(b"\n", at)
         line = data[at:end if end >= 0 else len(data)].split()
         if line and not line[0].startswith(b"%"):
-            size = [int(t) for t in line[:3] if t.isdigit()]
+            size = [int(t) for t in line[:3] if t.isdigit() and len(t) <= 20]  # a u64 has 20 digits at most
             if len(size) == 3 and size[0] == size[1] and 4 * size[2] <= len(data) + 4 and size[0] <= 1 << 27:
                 return size[0], size[2]
             return 0, 0
