@@ -231,10 +231,14 @@ struct Layout {
   size_t kept, before;            // compaction: kept slots as a bitmap, and counted before each of its words
   size_t big;                     // rows longer than kWarpRow (a block each)
   size_t tiles, ctl, mem, st, wpref, cnt, mem_tri, mem_maxsup, uni;
+  // the peel's rank index, where it is part of the layout (`indexed`: served
+  // unions; other launches take it from the third workspace, see run_union)
+  bool indexed;
+  size_t rpool, qh0, qh1, chunks;
   size_t total;
 };
 
-Layout make_layout(uint64_t N, uint64_t W, uint32_t G, bool own_nbr, size_t out_bytes) {
+Layout make_layout(uint64_t N, uint64_t W, uint32_t G, bool own_nbr, size_t out_bytes, bool indexed = false) {
   Layout L{};
   size_t p = 0;
   auto take = [&](size_t bytes) {
@@ -279,6 +283,13 @@ Layout make_layout(uint64_t N, uint64_t W, uint32_t G, bool own_nbr, size_t out_
   L.mem_tri = take(8ull * G);
   L.mem_maxsup = take(4ull * G);
   L.uni = take(sizeof(Union));
+  L.indexed = indexed;
+  if (indexed) {
+    L.rpool = take(8 * W);
+    L.qh0 = take(8 * M);
+    L.qh1 = take(8 * M);
+    L.chunks = take(sizeof(uint2) * rank_chunks_max(W));
+  }
   L.total = p;
   return L;
 }
@@ -698,6 +709,16 @@ int read_opts(const sparx_pkt_opts* o, Opts* out) {
   return SPARX_OK;
 }
 
+// The peel's rank index of the working rows: where it lies and which rows have it.
+struct RowIndex {
+  unsigned long long* pool = nullptr;  // nullptr: no index
+  uint2* qh0 = nullptr;                // per queue entry: its longer row's header
+  uint2* qh1 = nullptr;
+  uint2* chunks = nullptr;
+  uint32_t rank_min = kInvalid;        // rows of at least this many entries
+  uint32_t fine_min = 0;               // the finer index for rows of vertices of at least this degree (0: none)
+};
+
 // A prepared launch: members laid out in one union, CSR already on device.
 struct UnionJob;
 struct Engine;
@@ -711,6 +732,7 @@ struct PeelCtx {
   uint64_t Ws;                    // slots in the union
   uint32_t N, G;
   uint64_t waves_run = 0;         // waves the union's loop has run so far
+  RowIndex index;
   bool resume = false;            // the hook added members or some are still running
 };
 // Served unions: called at every stop of the peel loop (a member finished,
@@ -728,7 +750,6 @@ struct UnionJob {
   bool prep_only = false;        // stop after the support pass (members about to join a served union)
   const uint32_t* smap = nullptr;  // multigraphs: caller slot -> deduplicated slot (device)
   uint64_t budget = 0;             // device bytes the launch may hold (batched and served unions); 0: no bound
-  bool hook_hash = false;          // served union that takes no joins: rank index allowed
   uint64_t prep_m = 0, prep_Ws = 0;  // prep_only: edges and slots prepared
   std::vector<Member> members;  // vb, n, sb, w set; eb, m filled by the pipeline
   Layout L{};
@@ -761,6 +782,20 @@ struct UnionJob {
 
 template <class T>
 T* at(Engine& E, size_t off) { return reinterpret_cast<T*>(E.ws + off); }
+
+// The index of the rows of vertices [v0, v0 + count): `roff` / `rows` the working
+// rows, `off0` the rows as they were at first.
+int index_rows(Engine& E, const Layout& L, const RowIndex& X, const uint32_t* off0, const uint32_t* roff,
+               const unsigned long long* rows, uint32_t v0, uint32_t count, uint32_t* fine_count, cudaStream_t s) {
+  unsigned long long* hdr = at<unsigned long long>(E, L.vinfo) + v0;
+  uint32_t* listed = &at<Counters>(E, L.cnt)->table_big;
+  CU(cudaMemsetAsync(listed, 0, 4, s));
+  k_rank_index<unsigned long long><<<grid_for(count, 256, E.sm_count * 16), 256, 0, s>>>(
+      roff + v0, count, X.rank_min, rows, X.pool, hdr, X.chunks, listed, off0 + v0, X.fine_min, fine_count);
+  k_rank_index_chunks<unsigned long long><<<E.sm_count * 8, 256, 0, s>>>(roff + v0, rows, X.pool, hdr, X.chunks,
+                                                                         listed);
+  return SPARX_OK;
+}
 
 PeelArrays peel_arrays(const Union& U) {
   PeelArrays a{};
@@ -1091,22 +1126,25 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
     }
   }
   J.launches += 2;
-  // the peel's rank index of the working rows (in a served union only when it
-  // takes no joins, since joining rows would have none) and, as a tuned option,
+  // the peel's rank index of the working rows (a served union has it in its
+  // layout, with room for the rows that join) and, as a tuned option,
   // hash tables of the support pass's out-lists.  Both are optional: when their
   // workspace does not fit the launch's budget or cannot be allocated, the
   // launch runs without them (same results).
-  unsigned long long* rpool = nullptr;
+  RowIndex RI;
+  RI.fine_min = T.hub_min_degree ? std::max<uint32_t>(T.hub_min_degree, kHubFloor) : 0;
+  RI.rank_min = T.hash_min_degree ? std::max<uint32_t>(T.hash_min_degree / 4, 8) : kInvalid;
   unsigned long long* spool = nullptr;
-  uint2* qh0 = nullptr;
-  uint2* qh1 = nullptr;
-  uint2* index_chunks = nullptr;
-  const uint32_t fine_min = T.hub_min_degree ? std::max<uint32_t>(T.hub_min_degree, kHubFloor) : 0;
-  const uint32_t rank_min = T.hash_min_degree ? std::max<uint32_t>(T.hash_min_degree / 4, 8) : kInvalid;
   uint32_t sup_hash_min = 0;
+  const uint32_t index_floor = std::min(RI.rank_min, RI.fine_min ? RI.fine_min : kInvalid);  // rows below have none
+  if (L.indexed && index_floor != kInvalid) {
+    RI.pool = at<unsigned long long>(E, L.rpool);
+    RI.qh0 = at<uint2>(E, L.qh0);
+    RI.qh1 = at<uint2>(E, L.qh1);
+    RI.chunks = at<uint2>(E, L.chunks);
+  }
   {
-    const bool any_row = hc.dmax >= std::min(rank_min, fine_min ? fine_min : kInvalid);
-    bool index = any_row && !J.support_only && !J.prep_only && (!J.hook || J.hook_hash) && Ws < (1ull << 30) && Ws;
+    bool index = hc.dmax >= index_floor && !J.support_only && !J.prep_only && !J.hook && Ws < (1ull << 30) && Ws;
     bool sup_hash = T.sup_hash_min && m > 0 && m < (1ull << 28);
     const uint64_t Mx = std::max<uint64_t>(W / 2, 1);
     size_t pool_b = index ? align_up(8ull * Ws) : 0, qh_b = index ? align_up(8ull * Mx) : 0;
@@ -1121,10 +1159,10 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
     }
     uint32_t* big_list = (uint32_t*)(E.ws3 + pool_b + 2 * qh_b + spool_b);
     if (index) {
-      rpool = (unsigned long long*)E.ws3;
-      qh0 = (uint2*)(E.ws3 + pool_b);
-      qh1 = (uint2*)(E.ws3 + pool_b + qh_b);
-      index_chunks = (uint2*)big_list;
+      RI.pool = (unsigned long long*)E.ws3;
+      RI.qh0 = (uint2*)(E.ws3 + pool_b);
+      RI.qh1 = (uint2*)(E.ws3 + pool_b + qh_b);
+      RI.chunks = (uint2*)big_list;
     }
     if (sup_hash) {
       spool = (unsigned long long*)(E.ws3 + pool_b + 2 * qh_b);
@@ -1189,24 +1227,15 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
     U.q[1] = at<unsigned long long>(E, L.q1);
     U.qd[0] = at<uint4>(E, L.qd0);
     U.qd[1] = at<uint4>(E, L.qd1);
-    U.rpool = rpool;
-    U.qh[0] = qh0;
-    U.qh[1] = qh1;
+    U.rpool = RI.pool;
+    U.qh[0] = RI.qh0;
+    U.qh[1] = RI.qh1;
     U.vinfo = nullptr;
-    auto index_rows = [&](const uint32_t* roff, const unsigned long long* rows, uint32_t* fine_count) -> int {
-      unsigned long long* vinfo = at<unsigned long long>(E, L.vinfo);
-      CU(cudaMemsetAsync(&cnt->table_big, 0, 4, s));
-      k_rank_index<unsigned long long><<<grid_for(N, 256, E.sm_count * 16), 256, 0, s>>>(
-          roff, N, rank_min, rows, rpool, vinfo, index_chunks, &cnt->table_big, J.off, fine_min, fine_count);
-      k_rank_index_chunks<unsigned long long><<<E.sm_count * 8, 256, 0, s>>>(roff, rows, rpool, vinfo, index_chunks,
-                                                                             &cnt->table_big);
-      J.launches += 2;
-      return SPARX_OK;
-    };
-    if (rpool) {
+    if (RI.pool) {
       U.vinfo = at<unsigned long long>(E, L.vinfo);
-      const int rc = index_rows(J.off, row0, &cnt->hub_count);
+      const int rc = index_rows(E, L, RI, J.off, J.off, row0, 0, N, &cnt->hub_count, s);
       if (rc) return rc;
+      J.launches += 2;
     }
     U.n = N;
     U.m = (uint32_t)m;
@@ -1282,6 +1311,7 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
       ctx.N = pN;
       ctx.G = pG;
       ctx.waves_run = hctl->waves_run;
+      ctx.index = RI;
       int rc = J.hook->at_stop(E, J, ctx, reason, s);
       if (rc) return rc;
       U = ctx.U;
@@ -1338,9 +1368,10 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
       k_compact_offsets<<<grid_for(pN + 1ull, 256, E.sm_count * 16), 256, 0, s>>>(cur_off, pN, slots, kept, before,
                                                                                   (uint32_t*)&cnt->grand, off2);
       k_compact_commit<<<1, 1, 0, s>>>(at<Union>(E, L.uni), off2, row2, off2 + pN, wa.ctl);
-      if (rpool) {
-        const int rc = index_rows(off2, row2, nullptr);
+      if (RI.pool) {
+        const int rc = index_rows(E, L, RI, J.off, off2, row2, 0, pN, nullptr, s);
         if (rc) return rc;
+        J.launches += 2;
       }
       const uint32_t per = std::max<uint32_t>(1, (uint32_t)(E.sm_count * 8) / std::max<uint32_t>(pG, 1));
       k_refresh_desc<<<pG * per, 256, 0, s>>>(wa.Up, dmem, wa.st, pG, per);
@@ -2103,8 +2134,8 @@ void server_finish(sparx_server* S, ServerReq* r, int status) {
 
 uint64_t prep_budget(uint64_t lane_budget) { return lane_budget / 5; }
 
-bool layout_fits(uint64_t N, uint64_t W, uint32_t G, size_t esz, uint64_t budget) {
-  return N < 0xFFFFFFFFull && W < 0xFFFFFFFFull && make_layout(N, W, G, true, esz * W).total <= budget;
+bool layout_fits(uint64_t N, uint64_t W, uint32_t G, size_t esz, uint64_t budget, bool indexed = false) {
+  return N < 0xFFFFFFFFull && W < 0xFFFFFFFFull && make_layout(N, W, G, true, esz * W, indexed).total <= budget;
 }
 
 // The lane's hook: delivers members as they finish and joins waiting requests.
@@ -2327,6 +2358,10 @@ struct LaneHook : ServeHook {
       k_shift_u32<<<gridM, 256, 0, s>>>(at<uint32_t>(E, L.osrc) + m0, at<uint32_t>(*P, PJ.L.osrc), mp, N0);
       CU(cudaMemcpyAsync(at<int2>(E, L.es) + m0, at<int2>(*P, PJ.L.es), 8 * mp, cudaMemcpyDeviceToDevice, s));
     }
+    if (ctx.index.pool && Np) {
+      const int irc = index_rows(E, L, ctx.index, off, ctx.cur_off, ctx.cur_row, N0, (uint32_t)Np, nullptr, s);
+      if (irc) return irc;
+    }
     Counters* cnt = at<Counters>(E, L.cnt);
     std::vector<Member> nm;
     for (const Member& M : PJ.members)
@@ -2461,6 +2496,8 @@ void server_worker(sparx_server* S, int lane) {
           ++it;
           continue;
         }
+        // a union grows only while its rank index fits as well
+        if (!batch.empty() && !layout_fits(N2, W2, kServeMaxMembers, esz, main_budget, true)) { ++it; continue; }
         if (batch.empty()) fresh = r->fresh_only;
         it = S->queue.erase(it);
         r->running = true;
@@ -2510,14 +2547,16 @@ void server_worker(sparx_server* S, int lane) {
     }
     for (const HostMember& h : hm) hook.max_member_w = std::max<uint64_t>(hook.max_member_w, h.w);
     // a union holding a member past kJoinMaxMemberSlots never takes joins: it
-    // gets no room for them, and its rows are final, so the rank index
-    // (built once, before the peel) are safe for it within the lane's budget
+    // gets no room for them
     const bool no_joins = hook.max_member_w > kJoinMaxMemberSlots;
+    // the rank index, where the lane's budget holds it with the union (what joins
+    // later gets its own part of it, see join_group)
+    const bool indexed = layout_fits(N, W, kServeMaxMembers, esz, main_budget, true);
     // room: the largest extra (slots e, vertices e / 2) the lane's budget holds
     uint64_t extra = 0;
     for (uint64_t step = 1ull << 40; step && !no_joins; step >>= 1) {
       const uint64_t e2 = extra + step;
-      if (W + e2 < (1ull << 31) && layout_fits(N + e2 / 2, W + e2, kServeMaxMembers, esz, main_budget))
+      if (W + e2 < (1ull << 31) && layout_fits(N + e2 / 2, W + e2, kServeMaxMembers, esz, main_budget, indexed))
         extra = e2;
     }
     hook.N_cap = N + extra / 2;
@@ -2526,10 +2565,9 @@ void server_worker(sparx_server* S, int lane) {
     J.N = N;
     J.W = W;
     J.hook = &hook;
-    J.hook_hash = no_joins;
     J.budget = main_budget;
     S->unions += 1;
-    J.L = make_layout(hook.N_cap, hook.W_cap, kServeMaxMembers, true, esz * hook.W_cap);
+    J.L = make_layout(hook.N_cap, hook.W_cap, kServeMaxMembers, true, esz * hook.W_cap, indexed);
     int rc = ensure_ws(E, J.L.total, false);
     if (!rc) {
       cudaStream_t s = E.stream;
@@ -2542,8 +2580,8 @@ void server_worker(sparx_server* S, int lane) {
       if (!rc) rc = run_union(E, J, S->O, s);
     }
     if (E.ws3) {
-      // the rank index of a union without join room leaves with it, so the
-      // lane holds no more than its share while its next union runs
+      // a union's support tables leave with it, so the lane holds no more than
+      // its share while its next union runs
       cudaStreamSynchronize(E.stream);
       cudaFree(E.ws3);
       E.ws3 = nullptr;
