@@ -2429,8 +2429,9 @@ struct LaneHook : ServeHook {
 };
 
 // Requests that could not join (an input defect or a multigraph): the batch
-// path, which attributes a device error to the member that caused it.
-void run_fresh(sparx_server* S, Engine& E, std::vector<ServerReq*>& batch) {
+// path, which attributes a device error to the member that caused it; what is
+// optional there is taken only within the lane's budget.
+void run_fresh(sparx_server* S, Engine& E, std::vector<ServerReq*>& batch, uint64_t budget) {
   std::vector<HostMember> hm;
   std::vector<size_t> which;
   std::vector<int> status(batch.size(), SPARX_OK);
@@ -2447,7 +2448,7 @@ void run_fresh(sparx_server* S, Engine& E, std::vector<ServerReq*>& batch) {
   std::vector<int> st2(hm.size(), SPARX_OK);
   std::vector<sparx_pkt_stats> stats(hm.size());
   int first_fail = SPARX_OK;
-  if (!hm.empty()) run_batch_union(E, hm, S->O, st2.data(), stats.data(), &first_fail);
+  if (!hm.empty()) run_batch_union(E, hm, S->O, st2.data(), stats.data(), &first_fail, budget);
   {
     std::lock_guard<std::mutex> lk(S->mu);
     for (size_t k = 0; k < which.size(); ++k) {
@@ -2513,7 +2514,7 @@ void server_worker(sparx_server* S, int lane) {
       }
     }
     if (fresh) {
-      run_fresh(S, E, batch);
+      run_fresh(S, E, batch, main_budget);
       continue;
     }
     // a served union: the batch, with room for requests that join while it runs
@@ -2595,7 +2596,7 @@ void server_worker(sparx_server* S, int lane) {
         if (!hook.delivered[g]) rest.push_back(hook.reqs[g]);
       cudaStreamSynchronize(E.stream);
       cudaGetLastError();
-      if (!rest.empty()) run_fresh(S, E, rest);
+      if (!rest.empty()) run_fresh(S, E, rest, main_budget);
     }
     {
       std::lock_guard<std::mutex> lk(S->mu);
