@@ -232,7 +232,8 @@ struct Layout {
   size_t big;                     // rows longer than kWarpRow (a block each)
   size_t tiles, ctl, mem, st, wpref, cnt, mem_tri, mem_maxsup, uni;
   // the peel's rank index, where it is part of the layout (`indexed`: served
-  // unions; other launches take it from the third workspace, see run_union)
+  // unions and the allocation-free entry point; other launches take it from the
+  // third workspace, see run_union)
   bool indexed;
   size_t rpool, qh0, qh1, chunks;
   size_t total;
@@ -784,16 +785,15 @@ template <class T>
 T* at(Engine& E, size_t off) { return reinterpret_cast<T*>(E.ws + off); }
 
 // The index of the rows of vertices [v0, v0 + count): `roff` / `rows` the working
-// rows, `off0` the rows as they were at first.
-int index_rows(Engine& E, const Layout& L, const RowIndex& X, const uint32_t* off0, const uint32_t* roff,
-               const unsigned long long* rows, uint32_t v0, uint32_t count, uint32_t* fine_count, cudaStream_t s) {
-  unsigned long long* hdr = at<unsigned long long>(E, L.vinfo) + v0;
-  uint32_t* listed = &at<Counters>(E, L.cnt)->table_big;
+// rows, `off0` the rows as they were at first, `hdr` the vertices' headers.
+int index_rows(int sm_count, const RowIndex& X, unsigned long long* hdr, uint32_t* listed, const uint32_t* off0,
+               const uint32_t* roff, const unsigned long long* rows, uint32_t v0, uint32_t count,
+               uint32_t* fine_count, cudaStream_t s) {
   CU(cudaMemsetAsync(listed, 0, 4, s));
-  k_rank_index<unsigned long long><<<grid_for(count, 256, E.sm_count * 16), 256, 0, s>>>(
-      roff + v0, count, X.rank_min, rows, X.pool, hdr, X.chunks, listed, off0 + v0, X.fine_min, fine_count);
-  k_rank_index_chunks<unsigned long long><<<E.sm_count * 8, 256, 0, s>>>(roff + v0, rows, X.pool, hdr, X.chunks,
-                                                                         listed);
+  k_rank_index<unsigned long long><<<grid_for(count, 256, sm_count * 16), 256, 0, s>>>(
+      roff + v0, count, X.rank_min, rows, X.pool, hdr + v0, X.chunks, listed, off0 + v0, X.fine_min, fine_count);
+  k_rank_index_chunks<unsigned long long><<<sm_count * 8, 256, 0, s>>>(roff + v0, rows, X.pool, hdr + v0, X.chunks,
+                                                                       listed);
   return SPARX_OK;
 }
 
@@ -1233,7 +1233,8 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
     U.vinfo = nullptr;
     if (RI.pool) {
       U.vinfo = at<unsigned long long>(E, L.vinfo);
-      const int rc = index_rows(E, L, RI, J.off, J.off, row0, 0, N, &cnt->hub_count, s);
+      const int rc = index_rows(E.sm_count, RI, at<unsigned long long>(E, L.vinfo), &cnt->table_big, J.off, J.off, row0,
+                                0, N, &cnt->hub_count, s);
       if (rc) return rc;
       J.launches += 2;
     }
@@ -1369,7 +1370,8 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
                                                                                   (uint32_t*)&cnt->grand, off2);
       k_compact_commit<<<1, 1, 0, s>>>(at<Union>(E, L.uni), off2, row2, off2 + pN, wa.ctl);
       if (RI.pool) {
-        const int rc = index_rows(E, L, RI, J.off, off2, row2, 0, pN, nullptr, s);
+        const int rc = index_rows(E.sm_count, RI, at<unsigned long long>(E, L.vinfo), &cnt->table_big, J.off, off2, row2,
+                                  0, pN, nullptr, s);
         if (rc) return rc;
         J.launches += 2;
       }
@@ -2358,11 +2360,12 @@ struct LaneHook : ServeHook {
       k_shift_u32<<<gridM, 256, 0, s>>>(at<uint32_t>(E, L.osrc) + m0, at<uint32_t>(*P, PJ.L.osrc), mp, N0);
       CU(cudaMemcpyAsync(at<int2>(E, L.es) + m0, at<int2>(*P, PJ.L.es), 8 * mp, cudaMemcpyDeviceToDevice, s));
     }
+    Counters* cnt = at<Counters>(E, L.cnt);
     if (ctx.index.pool && Np) {
-      const int irc = index_rows(E, L, ctx.index, off, ctx.cur_off, ctx.cur_row, N0, (uint32_t)Np, nullptr, s);
+      const int irc = index_rows(E.sm_count, ctx.index, at<unsigned long long>(E, L.vinfo), &cnt->table_big, off,
+                                 ctx.cur_off, ctx.cur_row, N0, (uint32_t)Np, nullptr, s);
       if (irc) return irc;
     }
-    Counters* cnt = at<Counters>(E, L.cnt);
     std::vector<Member> nm;
     for (const Member& M : PJ.members)
       nm.push_back(Member{M.vb + N0, M.n, M.sb + (uint32_t)W0, M.w, M.eb + (uint32_t)m0, M.m});
@@ -3446,8 +3449,9 @@ struct DrainOnExit {
   }
 };
 
-// The same arrays as the engine's workspace, minus staging and output.
-Layout make_noalloc_layout(uint64_t N, uint64_t W) {
+// The same arrays as the engine's workspace, minus staging and output; `indexed`:
+// with the peel's rank index.
+Layout make_noalloc_layout(uint64_t N, uint64_t W, bool indexed) {
   Layout L{};
   size_t p = 0;
   auto take = [&](size_t bytes) {
@@ -3480,6 +3484,14 @@ Layout make_noalloc_layout(uint64_t N, uint64_t W) {
   L.mem_tri = take(8);
   L.mem_maxsup = take(4);
   L.uni = take(sizeof(Union));
+  L.indexed = indexed;
+  if (indexed) {
+    L.vinfo = take(8 * N);
+    L.rpool = take(8 * W);
+    L.qh0 = take(8 * M);
+    L.qh1 = take(8 * M);
+    L.chunks = take(sizeof(uint2) * rank_chunks_max(W));
+  }
   L.total = p;
   return L;
 }
@@ -3496,7 +3508,9 @@ int run_noalloc(const uint64_t* d_offsets, uint64_t n_plus_1, const uint32_t* d_
   rc = noalloc_scratch(device, &base);
   if (rc) return rc;
   const uint64_t n = n_plus_1 - 1;
-  const Layout L = make_noalloc_layout(n, width);
+  // with the rank index where the scratch holds it (about 1.1 M slots), else without
+  Layout L = make_noalloc_layout(n, width, true);
+  if (L.total > kNoAllocScratchBytes) L = make_noalloc_layout(n, width, false);
   if (L.total > kNoAllocScratchBytes) {
     set_error("graph needs " + std::to_string(L.total) + " bytes of scratch; the allocation-free entry point has " +
               std::to_string(kNoAllocScratchBytes) + " (about 1.4 M CSR slots); use sparx_pkt_run_device");
@@ -3579,7 +3593,7 @@ int run_noalloc(const uint64_t* d_offsets, uint64_t n_plus_1, const uint32_t* d_
     if (rc) return rc;
   }
 
-  Union U{};  // no rank index in the fixed scratch
+  Union U{};
   U.off = off;
   U.row = row0;
   U.opos = opos;
@@ -3592,6 +3606,22 @@ int run_noalloc(const uint64_t* d_offsets, uint64_t n_plus_1, const uint32_t* d_
   U.q[1] = (unsigned long long*)P(L.q1);
   U.qd[0] = (uint4*)P(L.qd0);
   U.qd[1] = (uint4*)P(L.qd1);
+  RowIndex RI;
+  RI.rank_min = std::max<uint32_t>(Tuning{}.hash_min_degree / 4, 8);
+  // Only where an eighth of the slots are in rows of degree >= 256: R-MAT-12 / 14 / 16
+  // (edge factor 9) 5.35 -> 4.59, 12.3 -> 10.2, 15.5 -> 12.3 ms, K_1000 6.8 -> 6.3, but
+  // building it costs what shorter rows gain (ER n = 20,000, m = 500,000 0.51 -> 0.55, a
+  // ring of rows of 64 0.89 -> 0.99)
+  if (L.indexed && 8 * hc.heavy >= width) {
+    RI.pool = (unsigned long long*)P(L.rpool);
+    RI.chunks = (uint2*)P(L.chunks);
+    U.rpool = RI.pool;
+    U.qh[0] = (uint2*)P(L.qh0);
+    U.qh[1] = (uint2*)P(L.qh1);
+    U.vinfo = (const unsigned long long*)P(L.vinfo);
+    rc = index_rows(sm, RI, (unsigned long long*)P(L.vinfo), &cnt->table_big, off, off, row0, 0, N, nullptr, s);
+    if (rc) return rc;
+  }
   U.n = N;
   U.m = (uint32_t)m;
   U.width = (uint32_t)width;
