@@ -1452,7 +1452,7 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
       std::fclose(f);
     }
   }
-  // each WHILE-loop iteration is one wave kernel (its last block plans)
+  // the device loop counts by its waves, whatever launches they shared
   if (!J.support_only && O.loop == SPARX_LOOP_GRAPH)
     J.launches += (uint32_t)std::max<unsigned long long>(J.ctl.waves_run, 1);
   J.err = hc.err;
