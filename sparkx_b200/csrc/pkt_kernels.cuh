@@ -245,13 +245,12 @@ __device__ __forceinline__ uint32_t find_in_row(const unsigned long long* __rest
   return (lo < end && (uint32_t)__ldg(row + lo) == w) ? lo : kInvalid;
 }
 
-// Warp-cooperative searches over a non-decreasing key(x).  Each step gathers
-// 32 evenly spaced keys with one load per lane and keeps the stretch between
-// the two samples that bracket the target, so a span of n entries costs
-// ceil(log32 n) + 1 dependent gathers instead of log2 n dependent loads.  All
-// lanes must call them with the same arguments.
-
-// largest x in [lo, hi] with key(x) <= t; requires key(lo) <= t
+// Warp-cooperative search over a non-decreasing key(x): the largest x in [lo, hi]
+// with key(x) <= t, given key(lo) <= t.  Each step gathers 32 evenly spaced keys
+// with one load per lane and keeps the stretch between the two samples that
+// bracket the target, so a span of n entries costs ceil(log32 n) + 1 dependent
+// gathers instead of log2 n dependent loads.  All lanes must call it with the
+// same arguments.
 template <class KeyF>
 __device__ __forceinline__ uint32_t warp_last_le(const KeyF& key, uint32_t lo, uint32_t hi,
                                                  unsigned long long t) {
@@ -270,37 +269,9 @@ __device__ __forceinline__ uint32_t warp_last_le(const KeyF& key, uint32_t lo, u
   return lo + 31 - __clz(b);
 }
 
-// first x in [lo, hi) with key(x) >= t, or hi
-template <class KeyF>
-__device__ __forceinline__ uint32_t warp_lower_bound(const KeyF& key, uint32_t lo, uint32_t hi,
-                                                     unsigned long long t) {
-  const uint32_t lane = lane_id();
-  while (hi - lo > 32) {
-    const uint32_t step = (hi - lo + 31) / 32;
-    const unsigned long long s = (unsigned long long)lo + (unsigned long long)lane * step;
-    const bool lt = s < hi && key((uint32_t)s) < t;
-    const uint32_t b = __ballot_sync(kFull, lt);
-    if (b == 0) return lo;
-    const uint32_t tl = 31 - __clz(b);
-    // key(lo + tl*step) < t <= key(lo + (tl+1)*step) (or past hi)
-    const uint32_t nlo = lo + tl * step + 1;
-    hi = min(hi, lo + (tl + 1) * step);
-    lo = nlo;
-  }
-  const bool lt = lo + lane < hi && key(lo + lane) < t;
-  return lo + __popc(__ballot_sync(kFull, lt));
-}
-
 struct PrefKey {
   const unsigned long long* p;
   __device__ __forceinline__ unsigned long long operator()(uint32_t x) const { return p[x]; }
-};
-
-struct RowIdKey {
-  const unsigned long long* row;
-  __device__ __forceinline__ unsigned long long operator()(uint32_t x) const {
-    return (uint32_t)__ldg(row + x);
-  }
 };
 
 __device__ __forceinline__ unsigned long long warp_incl_scan(unsigned long long v) {
@@ -1060,11 +1031,6 @@ __global__ void __launch_bounds__(256) k_rank_index_chunks(const uint32_t* __res
 // triangle (a, b, c), credited on e, (a -> c) and (b -> c).  Work elements are
 // spread evenly over warps through the exclusive prefix `spref`; a warp owns a
 // contiguous chunk and walks it 32 elements at a time.
-struct PrefStart {
-  const unsigned long long* p;
-  __device__ __forceinline__ unsigned long long operator()(uint32_t x) const { return p[x]; }
-};
-
 template <class StartF>
 __device__ __forceinline__ uint32_t window_find(const StartF& start, uint32_t i, uint32_t count,
                                                 unsigned long long j, bool valid);
@@ -1139,7 +1105,7 @@ __global__ void __launch_bounds__(256, kSupBlocks) k_support_balanced(
   const unsigned long long nwarps = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
   unsigned long long ch = total / (nwarps * 4);
   ch = min(max((ch + 31) & ~31ull, 32ull), 4096ull);
-  const PrefStart ps{spref};
+  const PrefKey ps{spref};
   unsigned long long found_total = 0;
   for (unsigned long long c0 = warp * ch; c0 < total; c0 += nwarps * ch) {
     const unsigned long long kend = min(c0 + ch, total);

@@ -504,8 +504,7 @@ inline int grid_for(unsigned long long items, int threads, int cap_blocks) {
 // the pinned buffer (so 4 bytes per slot cross PCIe, not 8), and the chunk goes
 // straight to its place in HBM.  A bad id sets kErrRange in *d_err's host twin.
 int upload_ids(Engine& E, const void* host, int bits, uint64_t count, uint32_t* dst, uint64_t n_limit,
-               uint32_t base, cudaStream_t s, char* stage[2], uint32_t* d_err) {
-  (void)stage;
+               uint32_t base, cudaStream_t s, uint32_t* d_err) {
   const uint64_t chunk = piece_bytes(count * 4) / 4;
   bool bad = false;
   for (uint64_t c = 0, at = 0; at < count; ++c, at += chunk) {
@@ -1723,7 +1722,7 @@ int run_host(const uint64_t* offsets, uint64_t n_plus_1, const void* nbrs, int b
     }
   }
   if (bad_host) { set_error("offsets: first must be 0, last must equal width, non-decreasing"); return SPARX_E_INVALID_CSR; }
-  rc = upload_ids(E, nbrs, bits, width, (uint32_t*)J.nbr, n, 0, s, stage, &cnt->err);
+  rc = upload_ids(E, nbrs, bits, width, (uint32_t*)J.nbr, n, 0, s, &cnt->err);
   if (rc) return rc;
   // one narrowing kernel per offsets chunk (the ids are narrowed by the host)
   const uint64_t off_chunk = piece_bytes(n_plus_1 * 8) / 8;
