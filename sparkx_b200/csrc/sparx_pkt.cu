@@ -1032,6 +1032,11 @@ int run_union(Engine& E, UnionJob& J, const Opts& O, cudaStream_t s) {
     CU(cudaMemcpyAsync(E.pinned_small, cnt, sizeof(Counters), cudaMemcpyDeviceToHost, s));
     CU(cudaStreamSynchronize(s));
     hc = *(const Counters*)E.pinned_small;
+    if (hc.err & (kErrOffsets | kErrRange)) {  // refused input: no row was read, nothing counted
+      for (Member& M : J.members) M.eb = M.m = 0;
+      J.err = hc.err;
+      return status_from_flags(hc.err);
+    }
     m32 = (uint32_t)hc.grand;  // the scan's total: oriented edges
     if (solo) {
       J.members[0].eb = 0;
