@@ -2839,7 +2839,8 @@ __device__ __forceinline__ void kc_work(const KcArgs& a, uint32_t phase, uint32_
     const uint32_t kend = (uint32_t)min((warp + 1) * ch, (unsigned long long)total);
     uint32_t i = warp_last_le(KcStart{q}, 0, count - 1, warp * ch);
     for (uint32_t j0 = (uint32_t)(warp * ch); j0 < kend; j0 += 32) {
-      // each lane's entry among the 32 from i on (every row has an entry)
+      // each lane's entry among the 32 from i on (every row has an entry, and the
+      // window's first one owns element j0: 32 elements span at most 32 of them)
       const unsigned long long qv = i + lane < count ? q[i + lane] : ~0ull;
       const uint32_t start = (uint32_t)(qv >> 32), j = j0 + lane;
       uint32_t t = 0;
@@ -2847,7 +2848,12 @@ __device__ __forceinline__ void kc_work(const KcArgs& a, uint32_t phase, uint32_
       for (int d = 16; d > 0; d >>= 1)
         if (__shfl_sync(kFull, start, t + d) <= j) t += d;
       const uint32_t u = __shfl_sync(kFull, (uint32_t)qv, t), at = __shfl_sync(kFull, start, t);
-      i += __shfl_sync(kFull, t, min(31u, kend - 1 - j0));
+      // on to the owner of j0 + 32: the last lane's entry, or the one after it where
+      // that starts there (past the window after 32 rows of one entry)
+      const uint32_t tl = __shfl_sync(kFull, t, min(31u, kend - 1 - j0));
+      const uint32_t after = tl < 31 ? __shfl_sync(kFull, start, tl + 1)
+                             : i + 32 < count ? (uint32_t)(q[i + 32] >> 32) : 0xFFFFFFFFu;
+      i += tl + (after <= j0 + 32);
       bool push = false;
       uint32_t v = 0;
       if (j < kend) {
