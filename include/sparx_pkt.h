@@ -269,7 +269,9 @@ typedef struct sparx_tuning {
 int sparx_tuning_default(sparx_tuning* t);
 /* The key of a host CSR (its offsets only). */
 int sparx_tuning_signature(const uint64_t* offsets, uint64_t n_plus_1, uint32_t key[3]);
-/* Cached knobs for a key (*found = 0: the defaults are returned). */
+/* Cached knobs for a key (*found = 0: the defaults are returned; relabel = 0 among
+ * them for keys of 2^23 to 2^26 slots, see above: a program that stores what it read
+ * here turns the relabelling off for such a key; start from sparx_tuning_last). */
 int sparx_tuning_lookup(const uint32_t key[3], sparx_tuning* out, int* found);
 int sparx_tuning_store(const uint32_t key[3], const sparx_tuning* t);
 int sparx_tuning_clear(void);
@@ -333,9 +335,10 @@ typedef struct sparx_server sparx_server;
  * its next wave, and the requests that fit join the union there (prepared on
  * the lane's second engine and placed behind the running members).  A union
  * takes no joins while it holds a graph of more than 2^26 slots or while its
- * waves average more than 60 us (newcomers then wait for a lane), and a union
- * without join room gets the rank index.  Every member's result goes back
- * as soon as its own peel ends.  A request needing
+ * waves average more than 60 us (newcomers then wait for a lane).  A union has
+ * the peel's rank index where the lane's share holds it (16 B a slot; the room for
+ * joins is sized with it), and what joins gets its part.  Every member's result
+ * goes back as soon as its own peel ends.  A request needing
  * more than any lane holds completes with SPARX_E_OOM.  Requests stay
  * addressable by ticket until sparx_server_destroy. */
 int sparx_server_create(sparx_server** out, uint64_t hbm_budget_bytes, const sparx_pkt_opts* opts);

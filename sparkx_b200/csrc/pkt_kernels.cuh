@@ -1038,13 +1038,13 @@ __device__ __forceinline__ uint32_t window_find(const StartF& start, uint32_t i,
 // What bounds it: issue slots (61% busy) and the latency of its three dependent
 // loads (element, word, entry); the credits are a tenth of it (R-MAT-20 9.1 ms
 // with them, 8.2 without).  Hence the most warps (8 blocks of 256 threads per
-// SM, 32 registers: 40.3 ms on R-MAT-22, 42.7 / 44.0 / 43.6 at 7 / 6 / 5 blocks
-// with 2 / 2 / 3 groups in flight), and a run of at least kSupRun elements of
-// one edge goes kSupWays groups of 32 at a time with its loads side by side (one
-// group 50.0 ms, two 40.3).  Against binary searches narrowed through 64 samples
-// of the longer list the rank index takes the pass from 80.0 to 40.3 ms on
-// R-MAT-22 (11.8 G elements), 15.0 to 8.5 ms on R-MAT-20; 4 to 8 buckets per entry
-// instead of 8 to 16 cost 5 ms more.
+// SM, 32 registers), and a run of at least kSupRun elements of one edge goes
+// kSupWays groups of 32 at a time with its loads side by side.  R-MAT-22 as it runs,
+// on its copy oriented by id: 7.2 G elements, 32.8 ms.  The choices were measured
+// on the copy oriented by degree (11.8 G elements): 40.3 ms; 42.7 / 44.0 / 43.6 at
+// 7 / 6 / 5 blocks with 2 / 2 / 3 groups in flight; one group 50.0; 4 to 8 buckets
+// per entry instead of 8 to 16 45; binary searches narrowed through 64 samples of
+// the longer list, which the index replaced, 80.0.  R-MAT-20 15.0 -> 8.5 ms.
 constexpr int kSupBlocks = 8;
 constexpr int kSupRun = 24;
 constexpr int kSupWays = 2;
@@ -1771,8 +1771,8 @@ constexpr int kPushBuf = 64;
 constexpr int kWaveThreads = 128;
 // Resident blocks per SM, which sets the register budget (40): with the found
 // triangles staged the search no longer needs the last 16 warps an SM holds, and
-// spills less.  R-MAT-22 285.9 / 284.8 ms, R-MAT-19 47.0 / 48.4, R-MAT-16 15.2 / 16.4
-// at 48 / 64 warps per SM.
+// spills less.  Calls at 48 / 64 warps per SM, when that was chosen: R-MAT-22
+// 285.9 / 284.8 ms, R-MAT-19 47.0 / 48.4, R-MAT-16 15.2 / 16.4.
 constexpr int kWaveBlocksPerSm = 12;
 constexpr int kWaveWarps = kWaveThreads / 32;
 constexpr int kTailThreads = 512;  // threads per block of the small waves' cluster (1024: R-MAT-12 6% slower)
@@ -1786,7 +1786,8 @@ constexpr int kKeepBuf = 256;
 // of 32 at a time, their row entries, index words and found entries loaded side
 // by side: the wave waits for memory (19 long-scoreboard stall cycles per issue in
 // a large wave, DRAM at 28%), so loads in flight count (R-MAT-22's peel 277 ms
-// with one group, 257 with two; three and four spill, 233 and 241 against 231).
+// with one group, 257 with two).  Three and four spill (233 and 241 ms against 231,
+// once the found triangles were staged).
 constexpr int kWaveWays = 2;
 constexpr uint32_t kWaveRun = 24;
 
